@@ -73,6 +73,47 @@ struct MemBodies {
   OGX_HD dv3 dpoint(int w, int i) const { return cvt<double>(point(w, i)); }
   OGX_HD const MemBodies& mem_view() const { return *this; }
 
+  // lane-local best value and its index, the runner-up's value, and (kMax) the largest
+  // |coordinate|, over the body's own points (not the padding)
+  template <bool kMax, class Team>
+  OGX_HD void scan_top(const Team& t, int w, fv3 d, float& best, int& bi, float& second, float& amax) const {
+    best = second = -INFINITY;
+    bi = 0x7fffffff;
+    amax = 0.0f;
+    const int nb = n4[w] >> 2;
+    const float* X = base[w];
+#if defined(__CUDA_ARCH__)
+#pragma unroll 2
+#endif
+    for (int q = t.lane(); q < nb; q += Team::L) {
+#if defined(__CUDA_ARCH__)
+      const float4* X4 = reinterpret_cast<const float4*>(X);
+      const float4 x = __ldg(X4 + q), y = __ldg(X4 + nb + q), z = __ldg(X4 + 2 * nb + q);
+#else
+      const float *Y = X + n4[w], *Z = X + 2 * n4[w];
+      const float4 x = make_float4_(X[4 * q], X[4 * q + 1], X[4 * q + 2], X[4 * q + 3]);
+      const float4 y = make_float4_(Y[4 * q], Y[4 * q + 1], Y[4 * q + 2], Y[4 * q + 3]);
+      const float4 z = make_float4_(Z[4 * q], Z[4 * q + 1], Z[4 * q + 2], Z[4 * q + 3]);
+#endif
+      float v[4];
+      sdot4(x, y, z, d, v);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (4 * q + c >= n[w]) v[c] = -INFINITY;
+        const bool win = v[c] > best;
+        second = win ? best : fmaxf(second, v[c]);
+        best = win ? v[c] : best;
+        bi = win ? 4 * q + c : bi;
+      }
+      if (kMax) {  // (the padding repeats a point)
+        const float ax = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
+        const float ay = fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)));
+        const float az = fmaxf(fmaxf(fabsf(z.x), fabsf(z.y)), fmaxf(fabsf(z.z), fabsf(z.w)));
+        amax = fmaxf(amax, fmaxf(ax, fmaxf(ay, az)));
+      }
+    }
+  }
+
   // lane-local best value over all points, best value over the points whose index is
   // not in ex[0..3) (the final simplex's points of this body), and max |coordinate|
   template <class Team>
@@ -122,6 +163,7 @@ struct MemBodies {
       block_best(v2, 4 * q2, best, bi);
     }
 #endif
+#pragma unroll 1
     for (; q < nb; q += Team::L) {
 #if defined(__CUDA_ARCH__)
       const float4 x = __ldg(reinterpret_cast<const float4*>(X) + q);
@@ -175,6 +217,7 @@ struct WideMemBodies : MemBodies {
         block_best(v, 4 * (q + u * Team::L), best, bi);
       }
     }
+#pragma unroll 1
     for (; q + Team::L < nb; q += 2 * Team::L) {
       const int q2 = q + Team::L;
       const float4 x = __ldg(X4 + q), y = __ldg(Y4 + q), z = __ldg(Z4 + q);
@@ -185,6 +228,7 @@ struct WideMemBodies : MemBodies {
       block_best(v, 4 * q, best, bi);
       block_best(v2, 4 * q2, best, bi);
     }
+#pragma unroll 1
     for (; q < nb; q += Team::L) {
       const float4 x = __ldg(X4 + q), y = __ldg(Y4 + q), z = __ldg(Z4 + q);
       float v[4];
@@ -251,6 +295,22 @@ struct Posed : Base {
     Base::scan(t, w, pose_dir(xf[w], d), best, bi);
     const float* m = xf[w];
     best += fmaf(m[11], d.z, fmaf(m[10], d.y, m[9] * d.x));
+  }
+  // as MemBodies::scan_top, on the posed points
+  template <bool kMax, class Team>
+  OGX_HD void scan_top(const Team& t, int w, fv3 d, float& best, int& bi, float& second, float& amax) const {
+    best = second = -INFINITY;
+    bi = 0x7fffffff;
+    amax = 0.0f;
+    for (int i = t.lane(); i < this->n[w]; i += Team::L) {
+      const fv3 p = point(w, i);
+      const float v = sdot(p, d);
+      const bool win = v > best;
+      second = win ? best : fmaxf(second, v);
+      best = win ? v : best;
+      bi = win ? i : bi;
+      if (kMax) amax = fmaxf(amax, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
+    }
   }
   // as MemBodies::scan_excl, on the posed points
   template <class Team>

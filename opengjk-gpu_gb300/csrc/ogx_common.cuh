@@ -24,10 +24,15 @@
 #define OGX_D __device__ __forceinline__
 // a rarely taken path kept out of line, so that its registers do not weigh on the loop
 // that calls it
-#define OGX_COLD __host__ __device__ __noinline__
+#define OGX_COLD inline __host__ __device__ __noinline__
+// long arithmetic used from many places (double-float division, FP64 predicates), kept out
+// of line: inlined, the kernels grew to 110-230 KB of code each and a warp spent more time
+// on instruction fetches than on anything else where few warps share a code path
+#define OGX_LEAF inline __host__ __device__ __noinline__
 #else
 #define OGX_HD inline
 #define OGX_COLD inline
+#define OGX_LEAF inline
 #endif
 
 #if !defined(__CUDACC__)
@@ -178,7 +183,7 @@ OGX_HD df operator*(df a, df b) {
   p.lo += a.hi * b.lo + a.lo * b.hi;
   return fast_two_sum(p.hi, p.lo);
 }
-OGX_HD df operator/(df a, df b) {
+OGX_LEAF df operator/(df a, df b) {
   const float q1 = a.hi / b.hi;
   df r = a - b * mk_df(q1, 0.0f);
   const float q2 = r.hi / b.hi;
@@ -187,7 +192,7 @@ OGX_HD df operator/(df a, df b) {
   return fast_two_sum(q1, q2) + mk_df(q3, 0.0f);
 }
 // square root: one Newton step from the float root (Karp and Markstein's form)
-OGX_HD df df_sqrt(df a) {
+OGX_LEAF df df_sqrt(df a) {
   if (!(a.hi > 0.0f)) return mk_df(0.0f, 0.0f);
   const float x = sqrtf(a.hi);
   const df r = a - two_prod(x, x);
@@ -222,6 +227,11 @@ OGX_HD double sc<double>(float x) { return (double)x; }
 template <>
 OGX_HD df sc<df>(float x) { return mk_df(x, 0.0f); }
 typedef vec3<df> xv3;
+// (a double-float dot product is ~130 instructions, a cross product ~210: out of line)
+OGX_LEAF df dot(xv3 a, xv3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+OGX_LEAF xv3 cross(xv3 a, xv3 b) {
+  return v3<df>(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
+}
 // exact difference of two float points as double-float components
 OGX_HD xv3 xdiff(fv3 a, fv3 b) { return v3<df>(two_sum(a.x, -b.x), two_sum(a.y, -b.y), two_sum(a.z, -b.z)); }
 
@@ -299,6 +309,22 @@ OGX_HD int popc32(uint32_t x) {
 #endif
 }
 
+OGX_HD int popc64(uint64_t x) {
+#if defined(__CUDA_ARCH__)
+  return __popcll(x);
+#else
+  return __builtin_popcountll(x);
+#endif
+}
+// position of the lowest set bit (x != 0)
+OGX_HD int lowest64(uint64_t x) {
+#if defined(__CUDA_ARCH__)
+  return __ffsll((long long)x) - 1;
+#else
+  return __builtin_ctzll(x);
+#endif
+}
+
 // EPA capacities.  With at most 64 expansions the polytope has at most 68 vertices and
 // (Euler, closed triangulated surface) 2*68-4 = 132 faces.
 constexpr int kEpaVmax = 68;
@@ -312,6 +338,7 @@ struct SerialTeam {
   static constexpr int L = 1;
   OGX_HD int lane() const { return 0; }
   OGX_HD void argmax(float&, int&) const {}
+  OGX_HD void argmax_pair(float&, int&, float&, int&) const {}
   OGX_HD void argmin(float&, int&) const {}
   OGX_HD void argmax2(float&, int&, float&) const {}
   OGX_HD void argmax_d(double&, int&) const {}
@@ -330,6 +357,17 @@ struct SerialTeam {
 };
 
 #if defined(__CUDACC__)
+// A float (not NaN) as an unsigned integer of the same order, -0 as +0, and back.  Full-warp
+// teams reduce these keys with the warp's integer reduction (redux.sync): one instruction
+// for the value and one for the lowest index that holds it, where the shuffle tree takes
+// five dependent rounds of two shuffles.
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t u = __float_as_uint(v + 0.0f);
+  return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float order_value(uint32_t k) {
+  return __uint_as_float(k ^ (~(uint32_t)((int32_t)k >> 31) | 0x80000000u));
+}
 // L consecutive lanes of a warp (L a power of two <= 32).
 template <int L_>
 struct WarpTeam {
@@ -344,6 +382,13 @@ struct WarpTeam {
   __device__ int lane() const { return ln; }
   // max value, ties to the smaller index
   __device__ void argmax(float& v, int& i) const {
+    if constexpr (L == 32) {
+      const uint32_t k = order_key(v);
+      const uint32_t m = __reduce_max_sync(0xffffffffu, k);
+      i = (int)__reduce_min_sync(0xffffffffu, k == m ? (uint32_t)i : 0xffffffffu);
+      v = order_value(m);
+      return;
+    }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
       const float v2 = __shfl_xor_sync(mask, v, o);
@@ -354,8 +399,55 @@ struct WarpTeam {
       }
     }
   }
+  // argmax of (va, ia) and of (vb, ib).  Teams of 4 to 16 lanes: after one exchange the even
+  // lanes reduce a and the odd lanes b, and a last exchange gives both to all -- two
+  // shuffles a round instead of four.
+  __device__ void argmax_pair(float& va, int& ia, float& vb, int& ib) const {
+    if constexpr (L == 1) return;
+    if constexpr (L == 2 || L == 32) {
+      argmax(va, ia);
+      argmax(vb, ib);
+      return;
+    }
+    const bool odd = ln & 1;
+    float v = odd ? vb : va;
+    int i = odd ? ib : ia;
+    const float sv = odd ? va : vb;
+    const int si = odd ? ia : ib;
+    float v2 = __shfl_xor_sync(mask, sv, 1);
+    int i2 = __shfl_xor_sync(mask, si, 1);
+    if (v2 > v || (v2 == v && i2 < i)) {
+      v = v2;
+      i = i2;
+    }
+#pragma unroll
+    for (int o = 2; o < L; o <<= 1) {
+      v2 = __shfl_xor_sync(mask, v, o);
+      i2 = __shfl_xor_sync(mask, i, o);
+      if (v2 > v || (v2 == v && i2 < i)) {
+        v = v2;
+        i = i2;
+      }
+    }
+    v2 = __shfl_xor_sync(mask, v, 1);
+    i2 = __shfl_xor_sync(mask, i, 1);
+    va = odd ? v2 : v;
+    ia = odd ? i2 : i;
+    vb = odd ? v : v2;
+    ib = odd ? i : i2;
+  }
   // FP64 max value, ties to the smaller index
   __device__ void argmax_d(double& v, int& i) const {
+    if constexpr (L == 32) {
+      // usually one lane holds the only candidate (the others' value is -infinity)
+      const uint32_t c = __ballot_sync(0xffffffffu, v > -INFINITY);
+      if (__popc(c) == 1) {
+        const int src = __ffs(c) - 1;
+        v = __shfl_sync(0xffffffffu, v, src);
+        i = __shfl_sync(0xffffffffu, i, src);
+        return;
+      }
+    }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
       const double v2 = __shfl_xor_sync(mask, v, o);
@@ -395,6 +487,13 @@ struct WarpTeam {
   }
   // min value, ties to the smaller index (index -1 means "none" and loses)
   __device__ void argmin(float& v, int& i) const {
+    if constexpr (L == 32) {
+      const uint32_t k = order_key(v);
+      const uint32_t m = __reduce_min_sync(0xffffffffu, k);
+      i = (int)__reduce_min_sync(0xffffffffu, k == m ? (uint32_t)i : 0xffffffffu);
+      v = order_value(m);
+      return;
+    }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
       const float v2 = __shfl_xor_sync(mask, v, o);
@@ -425,11 +524,13 @@ struct WarpTeam {
     return inc - x;
   }
   __device__ int imax(int x) const {
+    if constexpr (L == 32) return __reduce_max_sync(0xffffffffu, x);
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) x = max(x, __shfl_xor_sync(mask, x, o));
     return x;
   }
   __device__ float fmax_(float x) const {
+    if constexpr (L == 32) return order_value(__reduce_max_sync(0xffffffffu, order_key(x)));
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(mask, x, o));
     return x;

@@ -104,7 +104,7 @@ constexpr int kBucketCap[kBuckets] = {16, 32, 64, 128, 256, 512, 0};
 
 std::mutex g_init_mu;
 int g_init_device = -1;
-int g_grid_bin = 0, g_grid_polish = 0, g_grid_pack = 0, g_grid_refine = 0, g_grid_spill = 0;
+int g_grid_bin = 0, g_grid_polish = 0, g_grid_pack = 0, g_grid_refine = 0, g_grid_cont = 0, g_grid_spill = 0;
 uint32_t* g_subtab = nullptr;  // sub-distance decision table on the initialised device
 // per-device autotuned choices (variant index per bucket), -1 = not tuned
 int g_tuned[16][2][kBuckets];
@@ -137,11 +137,8 @@ constexpr int kDefaultEpa[kBuckets][2] = {{8, 1 + (5 << kOccShift)}, {8, 1 + (5 
                                           {8, 5 << kOccShift},     {8, 5 << kOccShift},
                                           {16, 5 << kOccShift}};
 
-// otherwise one pair per warp, fewest registers that fit
-int default_choice(const std::vector<Launch>& vs, int b, bool epa) {
-  const int* want = epa ? kDefaultEpa[b] : kDefaultGjk[b];
-  for (int i = 0; i < (int)vs.size(); ++i)
-    if (vs[i].L == want[0] && vs[i].K == want[1] && serves(vs[i], b)) return i;
+// one pair per warp, fewest registers that fit
+int warp_choice(const std::vector<Launch>& vs, int b) {
   int best = -1;
   for (int i = 0; i < (int)vs.size(); ++i) {
     if (!serves(vs[i], b) || vs[i].L != 32) continue;
@@ -153,6 +150,13 @@ int default_choice(const std::vector<Launch>& vs, int b, bool epa) {
     if (best < 0 || vs[i].K < vs[best].K) best = i;
   }
   return best;
+}
+
+int default_choice(const std::vector<Launch>& vs, int b, bool epa) {
+  const int* want = epa ? kDefaultEpa[b] : kDefaultGjk[b];
+  for (int i = 0; i < (int)vs.size(); ++i)
+    if (vs[i].L == want[0] && vs[i].K == want[1] && serves(vs[i], b)) return i;
+  return warp_choice(vs, b);
 }
 
 ogx_status init_variant(Launch* k, bool epa, int sms) {
@@ -237,6 +241,9 @@ ogx_status init_kernels(int device) {
   e = refine_occupancy(kBlock, &per_sm);
   if (e != cudaSuccess) return ogx_cuda_fail(e, "occupancy(k_refine)");
   g_grid_refine = std::max(1, per_sm) * sms;
+  e = continue_occupancy(kBlock, &per_sm);
+  if (e != cudaSuccess) return ogx_cuda_fail(e, "occupancy(k_refine_cont)");
+  g_grid_cont = std::min(2, std::max(1, per_sm)) * sms;
   {
     std::vector<uint32_t> tab(kSubTabSize);
     fill_subtab(tab.data());
@@ -476,6 +483,7 @@ extern "C" int ogx_ctx_work_counts(ogx_ctx* ctx, int32_t* counts, int cap) {
                       ctx->stream) != cudaSuccess ||
       cudaStreamSynchronize(ctx->stream) != cudaSuccess)
     return -1;
+  counts[kCntRefine] += counts[kCntRefineFull] + counts[kCntRefineBig];  // every refined pair
   return kCntSlots;
 }
 
@@ -825,7 +833,7 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   const cudaStream_t rst = st;
   if (refine) {
     ctx->mark("refine");
-    e = launch_refine(B, fit_grid(g_grid_refine, npairs, 1), fit_grid(g_grid_pack, npairs, 1), rst,
+    e = launch_refine(B, fit_grid(g_grid_refine, npairs, 1), fit_grid(g_grid_cont, npairs, 32), rst,
                       fork ? ctx->aux_r : rst, fork ? ctx->route_ev : nullptr);
     if (e == cudaSuccess && fork) {
       e = cudaEventRecord(ctx->rjoin_ev, ctx->aux_r);
@@ -833,7 +841,7 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
     }
     if (e != cudaSuccess) return ogx_cuda_fail(e, "k_refine launch");
     stage("refine", rst);
-    launches += 3;
+    launches += 2;
     if (mode != kModeGjk) {
       // the contacts the refinement found (usually none), after it on the same stream
       ctx->mark("epa_late");

@@ -56,7 +56,6 @@ struct EpaMemCert : EpaMem {
   double4 fn64[kEpaFmax];  // unit outward normal and plane distance, FP64 from exact points
 };
 OGX_HD double4* plane64_slot(EpaMemCert& M, int f) { return &M.fn64[f]; }
-
 // A small-capacity expansion that ran out of room, kept for the full-capacity pass to
 // continue from instead of starting again: the polytope and the loop state at the top of
 // the iteration that overflowed.  The full pass makes the same decisions up to there (the
@@ -159,36 +158,36 @@ OGX_HD fv3 msupport(const Team& t, const Bodies& B, fv3 d, int& ia, int& ib) {
   float ba, bb;
   B.scan(t, 0, d, ba, ia);
   B.scan(t, 1, -d, bb, ib);
-  t.argmax(ba, ia);
-  t.argmax(bb, ib);
+  t.argmax_pair(ba, ia, bb, ib);
   return B.point(0, ia) - B.point(1, ib);
 }
 
-// FP64 plane (unit normal, offset) of live face f from its exact points; w = INFINITY
-// for a degenerate face
-template <class Mem, class Bodies>
-OGX_HD double4 face_plane64(const Mem& M, const Bodies& B, int f) {
-  const int a = M.fv[f][0], b = M.fv[f][1], c = M.fv[f][2];
-  const dv3 q0 = B.dpoint(0, M.vid[a].x) - B.dpoint(1, M.vid[a].y);
-  const dv3 q1 = B.dpoint(0, M.vid[b].x) - B.dpoint(1, M.vid[b].y);
-  const dv3 q2 = B.dpoint(0, M.vid[c].x) - B.dpoint(1, M.vid[c].y);
+// FP64 plane (unit normal, offset) of the triangle q0, q1, q2; w = INFINITY when degenerate
+OGX_LEAF double4 plane64(dv3 q0, dv3 q1, dv3 q2) {
   const dv3 m = cross(q1 - q0, q2 - q0);
   const double mm = dot(m, m);
   if (!(mm > 0.0)) return make_double4_(0.0, 0.0, 0.0, (double)INFINITY);
   const double inv = 1.0 / sqrt(mm);
   return make_double4_(m.x * inv, m.y * inv, m.z * inv, dot(m, q0) * inv);
 }
+// the same of polytope vertices a, b, c, from their exact points
+template <class Mem, class Bodies>
+OGX_HD double4 face_plane64(const Mem& M, const Bodies& B, int a, int b, int c) {
+  return plane64(B.dpoint(0, M.vid[a].x) - B.dpoint(1, M.vid[a].y), B.dpoint(0, M.vid[b].x) - B.dpoint(1, M.vid[b].y),
+                 B.dpoint(0, M.vid[c].x) - B.dpoint(1, M.vid[c].y));
+}
 
 // Thin-contact check at FP32 convergence: true when exact supports along face f's FP64
 // plane improve on the face by more than tol.
 template <class Team, class Bodies, class Mem>
 OGX_HD bool thin_gain_exceeds(const Team& t, const Bodies& B, const Mem& M, int f, float tol) {
-  const double4 p = face_plane64(M, B, f);
+  const double4 p = face_plane64(M, B, M.fv[f][0], M.fv[f][1], M.fv[f][2]);
   if (!(p.w < (double)INFINITY)) return false;
   const dv3 n64 = v3<double>(p.x, p.y, p.z);
   double ha, hb;
-  exact_support(t, B, 0, n64, ha);
-  exact_support(t, B, 1, -n64, hb);
+  float ma = -1.0f, mb = -1.0f;
+  exact_support(t, B, 0, n64, ma, &ha);
+  exact_support(t, B, 1, -n64, mb, &hb);
   return ha + hb - p.w > (double)tol;
 }
 
@@ -206,24 +205,13 @@ OGX_HD float4 face_plane(const Mem& M, const Bodies& B, int a, int b, int c, boo
   float4 r;
   if (all64 || (escalate && nn < 1e-6f * s * s)) {
     // sine of the face angle below ~1e-3: FP32 normal unreliable
-    const dv3 q0 = B.dpoint(0, M.vid[a].x) - B.dpoint(1, M.vid[a].y);
-    const dv3 q1 = B.dpoint(0, M.vid[b].x) - B.dpoint(1, M.vid[b].y);
-    const dv3 q2 = B.dpoint(0, M.vid[c].x) - B.dpoint(1, M.vid[c].y);
-    const dv3 m = cross(q1 - q0, q2 - q0);
-    const double mm = dot(m, m);
     status |= OGX_S_EPA_ESCALATED;
-    if (mm > 0.0) {
-      const double inv = 1.0 / sqrt(mm);
-      r.x = (float)(m.x * inv);
-      r.y = (float)(m.y * inv);
-      r.z = (float)(m.z * inv);
-      r.w = (float)(dot(m, q0) * inv);
-      if (p64) *p64 = make_double4_(m.x * inv, m.y * inv, m.z * inv, dot(m, q0) * inv);
-    } else {
-      r.x = r.y = r.z = 0.0f;
-      r.w = INFINITY;  // degenerate: never the closest face, never visible
-      if (p64) *p64 = make_double4_(0.0, 0.0, 0.0, (double)INFINITY);
-    }
+    const double4 p = face_plane64(M, B, a, b, c);
+    if (p64) *p64 = p;
+    r.x = (float)p.x;  // degenerate: w infinite, never the closest face, never visible
+    r.y = (float)p.y;
+    r.z = (float)p.z;
+    r.w = (float)p.w;
     return r;
   }
   if (nn > 0.0f) {
@@ -298,6 +286,7 @@ template <class Mem, class Bodies>
 OGX_HD bool epa_emit(const Mem& M, const Bodies& B, int f, float tie, EpaOut& o, bool rerun_ok) {
   int a = M.fv[f][0], b = M.fv[f][1], c = M.fv[f][2];
   float l[3];
+#pragma unroll 1
   for (int hop = 0; hop < 4; ++hop) {
     a = M.fv[f][0];
     b = M.fv[f][1];
@@ -422,10 +411,12 @@ OGX_HD void epa_save(const Team& t, const Mem& M, const EpaResumeSink& sink, Epa
   slot = t.imax(slot);
   if (slot >= sink.cap) return;
   EpaResume& R = sink.buf[slot];
+#pragma unroll 1
   for (int j = t.lane(); j < nv; j += Team::L) {
     R.vp[j] = M.vp[j];
     R.vid[j] = M.vid[j];
   }
+#pragma unroll 1
   for (int f = t.lane(); f < fend; f += Team::L) {
     R.fn[f] = M.fn[f];
     for (int k = 0; k < 4; ++k) {
@@ -496,10 +487,12 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
     st = rs->st;
     scale2 = rs->scale2;
     o.status = rs->status;
+#pragma unroll 1
     for (int j = lane; j < nv; j += L) {
       M.vp[j] = rs->vp[j];
       M.vid[j] = rs->vid[j];
     }
+#pragma unroll 1
     for (int f = lane; f < fend; f += L) {
       M.fn[f] = rs->fn[f];
       for (int k = 0; k < 4; ++k) {
@@ -508,6 +501,7 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
       }
     }
     t.sync();
+#pragma unroll 1
     for (int f = lane; f < fend; f += L)
       if (M.fv[f][3] && M.fn[f].w < cbd) {
         cbd = M.fn[f].w;
@@ -546,42 +540,31 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
       }
     ++n;
   };
-  if (n == 1) {
-    int qa, qb;
-    const fv3 q = msupport(t, B, P[0], qa, qb);
-    if (!is_new(q, qa, qb)) {
-      epa_touch(B.point(0, qa), B.point(1, qb), o);
-      return;
+  bool flip = false;  // the triangle's second direction
+#pragma unroll 1
+  while (n < 4) {
+    fv3 d = P[0];
+    if (n == 2) {
+      const fv3 e = P[1] - P[0];
+      fv3 axis = v3<float>(1.0f, 0.0f, 0.0f);
+      const float el = sqrtf(dot(e, e));
+      if (el > FLT_EPSILON && fabsf(e.x) > 0.9f * el) axis = v3<float>(0.0f, 1.0f, 0.0f);
+      d = cross(e, axis);
+      if (dot(d, d) < FLT_EPSILON) d = cross(e, v3<float>(0.0f, 0.0f, 1.0f));
+    } else if (n == 3) {
+      d = cross(P[1] - P[0], P[2] - P[0]);
+      if (flip) d = -d;
     }
-    append(q, qa, qb);
-  }
-  if (n == 2) {
-    const fv3 e = P[1] - P[0];
-    fv3 axis = v3<float>(1.0f, 0.0f, 0.0f);
-    const float el = sqrtf(dot(e, e));
-    if (el > FLT_EPSILON && fabsf(e.x) > 0.9f * el) axis = v3<float>(0.0f, 1.0f, 0.0f);
-    fv3 d = cross(e, axis);
-    if (dot(d, d) < FLT_EPSILON) d = cross(e, v3<float>(0.0f, 0.0f, 1.0f));
     int qa, qb;
     const fv3 q = msupport(t, B, d, qa, qb);
-    if (!is_new(q, qa, qb)) {
+    if (is_new(q, qa, qb)) {
+      append(q, qa, qb);
+    } else if (n == 3 && !flip) {
+      flip = true;
+    } else {
       epa_touch(B.point(0, qa), B.point(1, qb), o);
       return;
     }
-    append(q, qa, qb);
-  }
-  if (n == 3) {
-    fv3 d = cross(P[1] - P[0], P[2] - P[0]);
-    int qa, qb;
-    fv3 q = msupport(t, B, d, qa, qb);
-    if (!is_new(q, qa, qb)) {
-      q = msupport(t, B, -d, qa, qb);
-      if (!is_new(q, qa, qb)) {
-        epa_touch(B.point(0, qa), B.point(1, qb), o);
-        return;
-      }
-    }
-    append(q, qa, qb);
   }
 
   // ---- tetrahedron
@@ -600,6 +583,7 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
 #pragma unroll
   for (int j = 0; j < 4; ++j) scale2 = fmaxf(scale2, dot(P[j], P[j]));
   t.sync();
+#pragma unroll 1
   for (int f = lane; f < 4; f += L) {
     const int va = f == 2 ? i1 : (f == 3 ? i2 : 0);
     const int vb = f == 0 ? i2 : (f == 1 ? i1 : (f == 2 ? i2 : 0));
@@ -627,6 +611,7 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
   bool done = false;
   bool thin = false;
   float thin_tol = 0.0f;
+  float amax0 = -1.0f, amax1 = -1.0f;  // the bodies' largest |coordinate| (certified run)
   while (it < cfg.epa_max_iter) {
     ++it;
     // closest live face
@@ -652,8 +637,8 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
       const double4 pl = *plane64_slot(M, best);
       const dv3 n64 = v3<double>(pl.x, pl.y, pl.z);
       double ha, hb;
-      qa = exact_support(t, B, 0, n64, ha);
-      qb = exact_support(t, B, 1, -n64, hb);
+      qa = exact_support(t, B, 0, n64, amax0, &ha);
+      qb = exact_support(t, B, 1, -n64, amax1, &hb);
       q = B.point(0, qa) - B.point(1, qb);
       q64 = B.dpoint(0, qa) - B.dpoint(1, qb);
       scale = sqrtf(fmaxf(scale2, dot(q, q)));
@@ -680,6 +665,7 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
       break;
     }
     bool dup = false;
+#pragma unroll 1
     for (int j = lane; j < nv; j += L) {
       const int2 id = M.vid[j];
       dup |= (id.x == qa && id.y == qb);
@@ -719,6 +705,7 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
     cbd = INFINITY;
     cbest = -1;
     int nvis = 0;
+#pragma unroll 1
     for (int f0 = 0; f0 < fend; f0 += L) {
       const int f = f0 + lane;
       bool s = false;
@@ -755,6 +742,7 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
     }
     // 2. horizon edges: edge e of a visible face whose neighbour is not visible
     int htot = 0;
+#pragma unroll 1
     for (int k0 = 0; k0 < nvis; k0 += L) {
       const int k = k0 + lane;
       bool h[3] = {false, false, false};
@@ -801,6 +789,7 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
     t.sync();
     // 3. relink the faces outside the horizon, index the horizon by its vertices, retire
     // the visible faces
+#pragma unroll 1
     for (int k = lane; k < htot; k += L) {
       const int s = k < nvis ? M.vlist[k] : fend + k - nvis;
       const int a = M.hz[k][0], b = M.hz[k][1], g2 = M.hz[k][2];
@@ -809,11 +798,13 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
       M.hstart[a] = (uint8_t)s;
       M.hend[b] = (uint8_t)s;
     }
+#pragma unroll 1
     for (int k = lane; k < nvis; k += L) M.fv[M.vlist[k]][3] = 0;
     t.sync();
     // a vertex that starts (or ends) two horizon edges means the horizon is not one
     // simple loop; keep the closest face found this step and stop
     bool bad = false;
+#pragma unroll 1
     for (int k = lane; k < htot; k += L) {
       const int s = k < nvis ? M.vlist[k] : fend + k - nvis;
       bad |= (M.hstart[M.hz[k][0]] != s) || (M.hend[M.hz[k][1]] != s);
@@ -829,6 +820,7 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
       break;
     }
     // 4. new face (a, b, p) across each horizon edge a->b
+#pragma unroll 1
     for (int k = lane; k < htot; k += L) {
       const int s = k < nvis ? M.vlist[k] : fend + k - nvis;
       const int a = M.hz[k][0], b = M.hz[k][1];

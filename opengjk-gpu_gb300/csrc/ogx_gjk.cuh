@@ -28,20 +28,6 @@
 namespace ogx {
 
 template <class T>
-struct Eps {
-  static constexpr double v = 0.0;
-};
-template <>
-struct Eps<float> {
-  static constexpr double v = FLT_EPSILON;
-};
-
-// flag set when a decision falls inside its rounding bound
-struct Unc {
-  bool hit;
-};
-
-template <class T>
 struct Vx {
   vec3<T> p;
   int k;  // slot of this vertex in the caller's simplex
@@ -53,307 +39,98 @@ struct Sx {
   Vx<T> v[4];
 };
 
-template <class T>
-OGX_HD T tabs(T x) {
-  return x < T(0) ? -x : x;
-}
+// The predicates and projections of the signed-volume step on exact points.  Each is one
+// out-of-line function, evaluated only where the decision asks for it.
 
 // (p - q) . p > 0 : the origin projects beyond p towards q (openGJK.c:219-230)
 template <class T>
-OGX_HD bool edge_keeps(vec3<T> p, vec3<T> q, Unc& u) {
+OGX_LEAF bool edge_keeps(vec3<T> p, vec3<T> q) {
   T acc = T(0);
   acc += (p.x * p.x - p.x * q.x);
   acc += (p.y * p.y - p.y * q.y);
   acc += (p.z * p.z - p.z * q.z);
-  if (Eps<T>::v != 0.0) {
-    const T perm = p.x * p.x + tabs(p.x * q.x) + p.y * p.y + tabs(p.y * q.y) + p.z * p.z +
-                   tabs(p.z * q.z);
-    if (tabs(acc) <= T(16.0 * Eps<T>::v) * perm) u.hit = true;
-  }
   return acc > T(0);
 }
 
 // origin beyond edge pq, away from r, in the plane pqr (openGJK.c:232-248)
 template <class T>
-OGX_HD bool edge_drops(vec3<T> p, vec3<T> q, vec3<T> r, Unc& u) {
+OGX_LEAF bool edge_drops(vec3<T> p, vec3<T> q, vec3<T> r) {
   const vec3<T> e1 = q - p, e2 = r - p;
   const vec3<T> nrm = cross(e1, cross(e1, e2));
-  const T val = dot(p, nrm);
-  if (Eps<T>::v != 0.0) {
-    const T b = l1(e1);
-    if (tabs(val) <= T(64.0 * Eps<T>::v) * l1(p) * b * b * l1(e2)) u.hit = true;
-  }
-  return val < T(0);
+  return dot(p, nrm) < T(0);
 }
 
-// origin on the far side of triangle (p, q, r) seen from ... (openGJK.c:250-255)
+// p . (q x r) <= 0 (openGJK.c:250-255); also the sign of the tetrahedron's volume
 template <class T>
-OGX_HD bool face_drops(vec3<T> p, vec3<T> q, vec3<T> r, Unc& u) {
-  const T val = dot(p, cross(q, r));
-  if (Eps<T>::v != 0.0) {
-    if (tabs(val) <= T(32.0 * Eps<T>::v) * l1(p) * l1(q) * l1(r)) u.hit = true;
-  }
-  return val <= T(0);
+OGX_LEAF bool face_drops(vec3<T> p, vec3<T> q, vec3<T> r) {
+  return dot(p, cross(q, r)) <= T(0);
 }
 
 template <class T>
-OGX_HD void onto_line(vec3<T> p, vec3<T> q, vec3<T>& out) {
+OGX_LEAF vec3<T> onto_line(vec3<T> p, vec3<T> q) {
   const vec3<T> d = p - q;
   const T t = dot(p, d) / dot(d, d);
-  out = p - d * t;
+  return p - d * t;
 }
 
 template <class T>
-OGX_HD void onto_plane(vec3<T> p, vec3<T> q, vec3<T> r, vec3<T>& out, Unc& u) {
+OGX_LEAF vec3<T> onto_plane(vec3<T> p, vec3<T> q, vec3<T> r) {
   const vec3<T> nrm = cross(p - q, p - r);
-  const T nn = dot(nrm, nrm);
-  if (Eps<T>::v != 0.0) {
-    const T b = T(32.0 * Eps<T>::v) * l1(p - q) * l1(p - r);
-    if (nn <= b * b) u.hit = true;
-  }
-  out = nrm * (dot(nrm, p) / nn);
+  return nrm * (dot(nrm, p) / dot(nrm, nrm));
 }
 
+// predicate `m` (one PB_* bit) of the step on s (n points, newest last), on exact points
 template <class T>
-OGX_HD void keep1(Sx<T>& s, const Vx<T>& a) {
-  s.n = 1;
-  s.v[0] = a;
-}
-template <class T>
-OGX_HD void keep2(Sx<T>& s, const Vx<T>& a, const Vx<T>& b) {
-  s.n = 2;
-  s.v[0] = a;
-  s.v[1] = b;
-}
-template <class T>
-OGX_HD void keep3(Sx<T>& s, const Vx<T>& a, const Vx<T>& b, const Vx<T>& c) {
-  s.n = 3;
-  s.v[0] = a;
-  s.v[1] = b;
-  s.v[2] = c;
+OGX_LEAF bool exact_bit(const Vx<T>* s, int n, uint32_t m) {
+  const vec3<T> q1 = s[n - 1].p;
+  if (m < PB_NEG) return edge_keeps(q1, s[m >> 1].p);  // 1, 2, 4: slots 0, 1, 2
+  if (m < (1u << PB_D)) {
+    if (m == PB_NEG) return face_drops(s[1].p - q1, s[0].p - q1, s[2].p - q1);
+    const int j = m == PB_F2 ? 1 : (m == PB_F3 ? 0 : 2), k = m == PB_F2 ? 0 : (m == PB_F3 ? 2 : 1);
+    return face_drops(q1, s[j].p, s[k].p);
+  }
+  // hff2 pairs in dpair() order: (0,1) (1,0) (0,2) (2,0) (1,2) (2,1)
+  const int d = m < (4u << PB_D) ? (m < (2u << PB_D) ? 0 : 1)
+                                 : (m < (16u << PB_D) ? (m < (8u << PB_D) ? 2 : 3) : (m < (32u << PB_D) ? 4 : 5));
+  const int lo = d < 4 ? 0 : 1, hi = d < 2 ? 1 : 2;
+  return edge_drops(q1, s[(d & 1) ? hi : lo].p, s[(d & 1) ? lo : hi].p);
 }
 
-// segment: newest vertex v[1]
+// Signed-volume step (openGJK.c:257-613) on exact points: reduces s (2 to 4 points, newest
+// last) to the vertices it needs and sets dir to its closest point to the origin.  The
+// decision is the FP32 step's, on exactly evaluated bits: `bits` are its predicates, those
+// in `known` already right (an FP32 value outside its rounding bound has the exact sign);
+// the others are evaluated when the decision comes to depend on them, each once.
 template <class T>
-OGX_HD void sub_segment(Sx<T>& s, vec3<T>& dir, Unc& u) {
-  const Vx<T> q1 = s.v[1], q2 = s.v[0];
-  if (edge_keeps(q1.p, q2.p, u)) {
-    onto_line(q1.p, q2.p, dir);
-  } else {
-    dir = q1.p;
-    keep1(s, q1);
+OGX_LEAF void subdistance(Sx<T>& s, vec3<T>& dir, const uint32_t* subtab, uint32_t bits, uint32_t known) {
+  const int n = s.n;
+  if (n < 2) return;
+  SubOut o;
+#pragma unroll 1
+  for (;;) {
+    o = step_decide(n, bits, subtab);
+    uint32_t need = o.used & ~known;
+    if (need == 0u) break;
+    need &= 0u - need;  // the lowest one first: the edge tests, then the faces, then the rest
+    known |= need;
+    bits = exact_bit(s.v, n, need) ? bits | need : bits & ~need;
   }
-}
-
-// triangle: newest vertex v[2]
-template <class T>
-OGX_HD void sub_triangle(Sx<T>& s, vec3<T>& dir, Unc& u) {
-  const Vx<T> q1 = s.v[2], q2 = s.v[1], q3 = s.v[0];
-  const bool k12 = edge_keeps(q1.p, q2.p, u);
-  const bool k13 = edge_keeps(q1.p, q3.p, u);
-  int pick = 0;  // 0 plane, 1 segment q1-q3, 2 segment q1-q2, 3 vertex q1
-  if (k12) {
-    if (!edge_drops(q1.p, q2.p, q3.p, u)) {
-      if (k13 && edge_drops(q1.p, q3.p, q2.p, u)) pick = 1;
-    } else {
-      pick = 2;
-    }
-  } else if (k13) {
-    if (edge_drops(q1.p, q3.p, q2.p, u)) pick = 1;
-  } else {
-    pick = 3;
+  const vec3<T> q1 = s.v[n - 1].p;
+  switch (o.kind) {
+    case SO_VERTEX: dir = q1; break;
+    case SO_LINE: dir = onto_line(q1, s.v[o.a].p); break;
+    case SO_PLANE: dir = onto_plane(q1, s.v[o.a].p, s.v[o.b].p); break;
+    case SO_ZERO: dir = v3<T>(T(0), T(0), T(0)); break;
+    default: break;  // undecided: unchanged
   }
-  if (pick == 0) {
-    onto_plane(q1.p, q2.p, q3.p, dir, u);
-  } else if (pick == 1) {
-    onto_line(q1.p, q3.p, dir);
-    keep2(s, q3, q1);
-  } else if (pick == 2) {
-    onto_line(q1.p, q2.p, dir);
-    keep2(s, q1, q2);
-  } else {
-    dir = q1.p;
-    keep1(s, q1);
-  }
-}
-
-// (k, i, j) naming of the three older tetrahedron vertices (openGJK.c:405-417)
-template <class T>
-OGX_HD void name_kij(int which, const Vx<T>& q2, const Vx<T>& q3, const Vx<T>& q4, Vx<T>& sk,
-                     Vx<T>& si, Vx<T>& sj) {
-  if (which == 0) {
-    sk = q2; si = q3; sj = q4;
-  } else if (which == 1) {
-    sk = q3; si = q4; sj = q2;
-  } else {
-    sk = q4; si = q2; sj = q3;
-  }
-}
-
-template <class T>
-OGX_HD void pick_plane(Sx<T>& s, const Vx<T>& a, const Vx<T>& b, const Vx<T>& q1,
-                       const vec3<T>& pp, const vec3<T>& pq, vec3<T>& dir, Unc& u) {
-  keep3(s, a, b, q1);
-  onto_plane(q1.p, pp, pq, dir, u);
-}
-template <class T>
-OGX_HD void pick_line(Sx<T>& s, const Vx<T>& a, const Vx<T>& q1, vec3<T>& dir) {
-  keep2(s, a, q1);
-  onto_line(q1.p, a.p, dir);
-}
-
-// tetrahedron: newest vertex v[3] (decision tree of openGJK.c:315-613)
-template <class T>
-OGX_HD void sub_tetra(Sx<T>& s, vec3<T>& dir, Unc& u) {
-  const Vx<T> q1 = s.v[3], q2 = s.v[2], q3 = s.v[1], q4 = s.v[0];
-  const bool l2 = edge_keeps(q1.p, q2.p, u);
-  const bool l3 = edge_keeps(q1.p, q3.p, u);
-  const bool l4 = edge_keeps(q1.p, q4.p, u);
-  const int nkeep = (int)l2 + (int)l3 + (int)l4;
-  if (nkeep == 0) {
-    dir = q1.p;
-    keep1(s, q1);
-    return;
-  }
-  const vec3<T> e2 = q2.p - q1.p, e3 = q3.p - q1.p, e4 = q4.p - q1.p;
-  const T vol = dot(e3, cross(e4, e2));
-  if (Eps<T>::v != 0.0) {
-    if (tabs(vol) <= T(32.0 * Eps<T>::v) * l1(e2) * l1(e3) * l1(e4)) u.hit = true;
-  }
-  const int neg = vol <= T(0);
-  int f2 = (int)face_drops(q1.p, q3.p, q4.p, u) - neg;
-  int f3 = (int)face_drops(q1.p, q4.p, q2.p, u) - neg;
-  int f4 = (int)face_drops(q1.p, q2.p, q3.p, u) - neg;
-  f2 *= f2;
-  f3 *= f3;
-  f4 *= f4;
-  Vx<T> sk, si, sj;
-  switch (f2 + f3 + f4) {
-    case 3:
-      dir = v3<T>(T(0), T(0), T(0));
-      return;
-    case 2:
-      if (!f2)
-        keep3(s, q4, q3, q1);
-      else if (!f3)
-        keep3(s, q4, q2, q1);
-      else
-        keep3(s, q3, q2, q1);
-      sub_triangle(s, dir, u);
-      return;
-    case 1: {
-      s.n = 3;
-      name_kij(f2 ? 0 : (f3 ? 1 : 2), q2, q3, q4, sk, si, sj);
-      const bool lk = edge_keeps(q1.p, sk.p, u);
-      const bool li = edge_keeps(q1.p, si.p, u);
-      const bool lj = edge_keeps(q1.p, sj.p, u);
-      if (nkeep == 1) {
-        if (lk) {
-          if (!edge_drops(q1.p, sk.p, si.p, u))
-            pick_plane(s, sk, si, q1, si.p, sk.p, dir, u);
-          else if (!edge_drops(q1.p, sk.p, sj.p, u))
-            pick_plane(s, sk, sj, q1, sj.p, sk.p, dir, u);
-          else
-            pick_line(s, sk, q1, dir);
-        } else if (li) {
-          if (!edge_drops(q1.p, si.p, sk.p, u))
-            pick_plane(s, sk, si, q1, si.p, sk.p, dir, u);
-          else
-            pick_line(s, si, q1, dir);
-        } else {
-          if (!edge_drops(q1.p, sj.p, sk.p, u))
-            pick_plane(s, sk, sj, q1, sj.p, sk.p, dir, u);
-          else
-            pick_line(s, sj, q1, dir);
-        }
-      } else if (nkeep == 2) {
-        if (li) {
-          if (!edge_drops(q1.p, sk.p, si.p, u)) {
-            if (!edge_drops(q1.p, si.p, sk.p, u))
-              pick_plane(s, sk, si, q1, si.p, sk.p, dir, u);
-            else
-              pick_line(s, sk, q1, dir);
-          } else if (!edge_drops(q1.p, sk.p, sj.p, u)) {
-            pick_plane(s, sk, sj, q1, sj.p, sk.p, dir, u);
-          } else {
-            pick_line(s, sk, q1, dir);
-          }
-        } else if (lj) {
-          if (!edge_drops(q1.p, sk.p, sj.p, u)) {
-            if (!edge_drops(q1.p, sj.p, sk.p, u))
-              pick_plane(s, sk, sj, q1, sj.p, sk.p, dir, u);
-            else
-              pick_line(s, sj, q1, dir);
-          } else if (!edge_drops(q1.p, sk.p, si.p, u)) {
-            pick_plane(s, sk, si, q1, si.p, sk.p, dir, u);
-          } else {
-            pick_line(s, sk, q1, dir);
-          }
-        } else {
-          u.hit = true;  // inconsistent tests: only possible through rounding
-        }
-      } else {
-        const bool d_ik = edge_drops(q1.p, si.p, sk.p, u);
-        const bool d_jk = edge_drops(q1.p, sj.p, sk.p, u);
-        const bool d_ki = edge_drops(q1.p, sk.p, si.p, u);
-        const bool d_kj = edge_drops(q1.p, sk.p, sj.p, u);
-        if (d_ki && d_kj)
-          pick_line(s, sk, q1, dir);
-        else if (d_ki) {
-          if (d_jk)
-            pick_line(s, sj, q1, dir);
-          else
-            pick_plane(s, sk, sj, q1, sk.p, sj.p, dir, u);
-        } else {
-          if (d_ik)
-            pick_line(s, si, q1, dir);
-          else
-            pick_plane(s, sk, si, q1, sk.p, si.p, dir, u);
-        }
-      }
-      return;
-    }
-    case 0:
-      if (nkeep == 1) {
-        name_kij(l3 ? 0 : (l4 ? 1 : 2), q2, q3, q4, sk, si, sj);
-        if (!edge_drops(q1.p, si.p, sj.p, u))
-          pick_plane(s, sj, si, q1, si.p, sj.p, dir, u);
-        else if (!edge_drops(q1.p, si.p, sk.p, u))
-          pick_plane(s, sk, si, q1, si.p, sk.p, dir, u);
-        else
-          pick_line(s, si, q1, dir);
-      } else if (nkeep == 2) {
-        s.n = 3;
-        name_kij(!l3 ? 0 : (!l4 ? 1 : 2), q2, q3, q4, sk, si, sj);
-        if (!edge_drops(q1.p, sj.p, sk.p, u)) {
-          if (!edge_drops(q1.p, sk.p, sj.p, u))
-            pick_plane(s, sk, sj, q1, sj.p, sk.p, dir, u);
-          else if (!edge_drops(q1.p, sk.p, si.p, u))
-            pick_plane(s, sk, si, q1, sk.p, si.p, dir, u);
-          else
-            pick_line(s, sk, q1, dir);
-        } else if (!edge_drops(q1.p, sj.p, si.p, u)) {
-          pick_plane(s, sj, si, q1, si.p, sj.p, dir, u);
-        } else {
-          pick_line(s, sj, q1, dir);
-        }
-      } else {
-        u.hit = true;  // all three edges keep but no face looks at the origin
-      }
-      return;
-    default:
-      return;
-  }
-}
-
-template <class T>
-OGX_HD void subdistance(Sx<T>& s, vec3<T>& dir, Unc& u) {
-  if (s.n == 4)
-    sub_tetra(s, dir, u);
-  else if (s.n == 3)
-    sub_triangle(s, dir, u);
-  else if (s.n == 2)
-    sub_segment(s, dir, u);
+  if (o.n == 4) return;
+  // (slots are numbered for the tetrahedron, newest = 3)
+  const Vx<T> r0 = s.v[o.s[0] == 3 ? n - 1 : o.s[0]], r1 = s.v[o.s[1] == 3 ? n - 1 : o.s[1]],
+              r2 = s.v[o.s[2] == 3 ? n - 1 : o.s[2]];
+  s.n = o.n;
+  s.v[0] = r0;
+  if (o.n > 1) s.v[1] = r1;
+  if (o.n > 2) s.v[2] = r2;
 }
 
 // --------------------------------------------------------------------------------
@@ -361,7 +138,7 @@ OGX_HD void subdistance(Sx<T>& s, vec3<T>& dir, Unc& u) {
 // (region tests of Ericson, Real-Time Collision Detection, sec. 5.1.5, restated)
 
 template <class T>
-OGX_HD void closest_on_simplex_t(int n, const vec3<T>* P, T* lam, vec3<T>& v) {
+OGX_LEAF void closest_on_simplex_t(int n, const vec3<T>* P, T* lam, vec3<T>& v) {
   const T zero = sc<T>(0.0f), one = sc<T>(1.0f);
   lam[0] = one;
   lam[1] = lam[2] = lam[3] = zero;
@@ -513,7 +290,8 @@ template <class Mem>
 #if defined(__CUDACC__)
 __noinline__
 #endif
-OGX_HD int escalate_step(const Mem B, int n, const int* ia, const int* ib, fv3 vold, int* order, fv3* vout) {
+OGX_HD int escalate_step(const Mem B, int n, const int* ia, const int* ib, fv3 vold, int* order, fv3* vout,
+                         const uint32_t* subtab, uint32_t bits, uint32_t known) {
   Sx<double> sd;
   sd.n = n;
   for (int j = 0; j < n; ++j) {
@@ -521,18 +299,18 @@ OGX_HD int escalate_step(const Mem B, int n, const int* ia, const int* ib, fv3 v
     sd.v[j].k = j;
   }
   dv3 vd = cvt<double>(vold);
-  Unc ud{false};
-  subdistance(sd, vd, ud);
+  subdistance(sd, vd, subtab, bits, known);
   for (int j = 0; j < sd.n; ++j) order[j] = sd.v[j].k;
   *vout = cvt<float>(vd);
   return sd.n;
 }
 
-// GJK as a resumable loop: gjk_start sets the state up, each gjk_iterate runs one
+// GJK as a loop of iterations: gjk_start sets the state up, each gjk_iterate runs one
 // iteration (support, termination tests, sub-distance step) until r.done, gjk_end
 // finishes (witnesses, certification).  gjk_pair chains them.
 struct GjkRun {
   fv3 v;
+  float vv;  // dot(v, v)
   fv3 P[4];  // simplex in registers: slots 0..3, newest last; every index is unrolled
   int IA[4], IB[4];
   int n;
@@ -550,6 +328,7 @@ OGX_HD void gjk_start(const Bodies& B, GjkRun& r, int start_a = 0, int start_b =
   // start), or a warm-start pair of vertex indices (e.g. the previous frame's simplex)
   const fv3 a0 = B.point(0, start_a), b0 = B.point(1, start_b);
   r.v = a0 - b0;
+  r.vv = dot(r.v, r.v);
   r.P[0] = r.v;
   r.P[1] = r.P[2] = r.P[3] = r.v;
   r.IA[0] = start_a;
@@ -567,168 +346,143 @@ OGX_HD void gjk_start(const Bodies& B, GjkRun& r, int start_a = 0, int start_b =
   r.done = false;
 }
 
+// The gap below which FP32 rounding of |v| |w| hides any progress.
+OGX_COLD float gap_floor(const Config cfg, float vv, float ww) {
+  const float nv = sqrtf(vv);
+  return fmaxf(cfg.gjk_eps_tot, cfg.gjk_noise * FLT_EPSILON * nv * (nv + sqrtf(ww)));
+}
+
+// One iteration is a chain of dependent steps (scan, team reduction, support points, gap,
+// predicates, table, projection) that a pair cannot overlap with anything of its own, so
+// what bounds it is the chain's length and, over a full GPU, its instruction count.  Hence:
+// both bodies' reductions side by side and both candidate points loaded at once; the
+// noise floor's square roots only where an upper bound says they can matter; one division
+// for whichever projection the step takes; |w|^2 of the new point alone for the scale (the
+// older points were counted when they joined); one branch for all the exit tests.
 template <class Team, class Bodies>
 OGX_HD void gjk_iterate(const Team& t, const Bodies& B, const Config& cfg, GjkRun& r,
                         const uint32_t* subtab = nullptr) {
   const bool reftol = (cfg.flags & OGX_F_REFERENCE_TOL) != 0;
   const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
-  const float eps_rel2 = cfg.gjk_eps_rel * cfg.gjk_eps_rel;
   // |v| this small against the simplex points is below FP32 resolution: stop
   const float contact = reftol ? cfg.gjk_eps_tot : 0.5f * FLT_EPSILON;
   fv3& v = r.v;
   fv3* P = r.P;
   int* IA = r.IA;
   int* IB = r.IB;
-  int& n = r.n;
-  float& wmax2 = r.wmax2;
-  fv3& sa = r.sa;
-  fv3& sb = r.sb;
-  int& ia = r.ia;
-  int& ib = r.ib;
-  int& k = r.k;
-  ++k;
-    const fv3 mv = -v;
-    float ba, bb;
-    int xa, xb;
-    B.scan(t, 0, mv, ba, xa);
-    B.scan(t, 1, v, bb, xb);
-    t.argmax(ba, xa);
-    t.argmax(bb, xb);
-    if (ba > sdot(sa, mv)) {
-      ia = xa;
-      sa = B.point(0, xa);
-    }
-    if (bb > sdot(sb, v)) {
-      ib = xb;
-      sb = B.point(1, xb);
-    }
-    const fv3 w = sa - sb;
-    const float vv = dot(v, v);
-    const float gap = vv - dot(v, w);
-    float floor_ = cfg.gjk_eps_tot;
-    if (!reftol) {
-      const float nv = sqrtf(vv);
-      floor_ = fmaxf(floor_, cfg.gjk_noise * FLT_EPSILON * nv * (nv + sqrtf(dot(w, w))));
-    }
-    if (gap <= cfg.gjk_eps_rel * vv) {
-      r.exit = GJK_EXIT_GAP_REL;
-      r.done = true;
-      return;
-    }
-    if (gap < floor_) {
-      r.exit = GJK_EXIT_GAP_NOISE;
-      r.done = true;
-      return;
-    }
-    if (vv < eps_rel2) {
-      r.exit = GJK_EXIT_NULL_V;
-      r.done = true;
-      return;
-    }
-    if (!reftol) {
-      bool dup = false;
+  ++r.k;
+  const fv3 mv = -v;
+  float ba, bb;
+  int xa, xb;
+  B.scan(t, 0, mv, ba, xa);
+  B.scan(t, 1, v, bb, xb);
+  t.argmax_pair(ba, xa, bb, xb);
+  // the candidates (a scan that no value won has no index: the last support then)
+  const fv3 pa = B.point(0, ba > -INFINITY ? xa : r.ia), pb = B.point(1, bb > -INFINITY ? xb : r.ib);
+  if (ba > sdot(r.sa, mv)) {
+    r.ia = xa;
+    r.sa = pa;
+  }
+  if (bb > sdot(r.sb, v)) {
+    r.ib = xb;
+    r.sb = pb;
+  }
+  const int ia = r.ia, ib = r.ib;
+  const fv3 w = r.sa - r.sb;
+  const float vv = r.vv, ww = dot(w, w);
+  const float gap = vv - dot(v, w);
+  float floor_ = cfg.gjk_eps_tot;
+  // gap_floor <= noise eps (vv + (vv + ww) / 2), up to rounding that the last factor covers
+  // (where vv is far from the subnormals)
+  const float bound = cfg.gjk_noise * FLT_EPSILON * (1.5f * vv + 0.5f * ww) * 1.0001f;
+  if (!reftol && (gap < bound || vv < 1e-30f)) floor_ = gap_floor(cfg, vv, ww);
+  bool dup = false;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dup |= (j < n) && IA[j] == ia && IB[j] == ib;
-      if (dup) {
-        r.exit = GJK_EXIT_DUPLICATE;
-        r.done = true;
-        return;
-      }
-    }
+  for (int j = 0; j < 4; ++j) dup |= (j < r.n) && IA[j] == ia && IB[j] == ib;
+  const int stop = gap <= cfg.gjk_eps_rel * vv                ? GJK_EXIT_GAP_REL
+                   : gap < floor_                             ? GJK_EXIT_GAP_NOISE
+                   : vv < cfg.gjk_eps_rel * cfg.gjk_eps_rel   ? GJK_EXIT_NULL_V
+                   : (dup && !reftol)                         ? GJK_EXIT_DUPLICATE
+                                                              : 0;
+  if (stop) {
+    r.exit = stop;
+    r.done = true;
+    return;
+  }
+  const int n = r.n + 1;  // w joins in slot n - 1
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j == n) {
-        P[j] = w;
-        IA[j] = ia;
-        IB[j] = ib;
-      }
-    ++n;
+  for (int j = 1; j < 3; ++j)
+    if (j == n - 1) {
+      P[j] = w;
+      IA[j] = ia;
+      IB[j] = ib;
+    }
 
-    StepIn S;
-    uint32_t bits, unc;
-    step_predicates(n, P, S, bits, unc);
-    // the decision: one load from the table on the device, the tree on the host
-    SubOut o;
-#if defined(__CUDA_ARCH__)
-    if (subtab)
-      o = unpack_subout(__ldg(subtab + subtab_index(n, bits)));
-    else
-#endif
-      o = step_decide(n, bits);
-    // degenerate spans make the projection itself unreliable
-    if (o.kind == SO_LINE) {
-      const float ge = o.a == 0 ? S.g[0][0] : (o.a == 1 ? S.g[1][1] : S.g[2][2]);
-      const float lq = l1(S.q1);
-      if (!(ge > 64.0f * FLT_EPSILON * FLT_EPSILON * lq * lq)) unc |= o.used | 1u;
-    } else if (o.kind == SO_PLANE) {
-      const fv3 ea = o.a == 0 ? S.e[0] : (o.a == 1 ? S.e[1] : S.e[2]);
-      const fv3 eb = o.b == 0 ? S.e[0] : (o.b == 1 ? S.e[1] : S.e[2]);
-      const int pab = (o.a < o.b ? o.a : o.b) * 3 + (o.a < o.b ? o.b : o.a);
-      const fv3 c = pab == 1 ? S.c01 : (pab == 2 ? S.c02 : S.c12);
-      const float bc = 32.0f * FLT_EPSILON * l1(ea) * l1(eb);
-      if (!(dot(c, c) > bc * bc)) unc |= o.used | 1u;
-    }
-    int nn;
-    fv3 P2[3];
-    int A2[3], B2[3];
-    if ((unc & o.used) != 0u && escalate) {
-      int order[4] = {0, 1, 2, 3};
-      int ias[4], ibs[4];
+  StepIn S;
+  uint32_t bits, unc;
+  step_predicates(n, P, w, S, bits, unc);
+  const SubOut o = step_decide(n, bits, subtab);
+  // the line through w and slot a, or the plane through w and slots a, b
+  const StepSpan span = step_span(S, o);
+  // degenerate spans make the projection itself unreliable
+  if (span.degenerate) unc |= o.used | 1u;
+  int nn;
+  int slot[3];
+  if ((unc & o.used) != 0u && escalate) {
+    int ias[4], ibs[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        ias[j] = IA[j];
-        ibs[j] = IB[j];
-      }
-      fv3 vd;
-      nn = escalate_step(B.mem_view(), n, ias, ibs, v, order, &vd);
-      v = vd;
-      r.status |= OGX_S_GJK_ESCALATED;
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int sj = order[j];
-        P2[j] = sel3(sj, P[0], P[1], P[2], P[3]);
-        A2[j] = seli(sj, IA[0], IA[1], IA[2], IA[3]);
-        B2[j] = seli(sj, IB[0], IB[1], IB[2], IB[3]);
-      }
-    } else {
-      v = step_direction(n, S, o, v);
-      // slots are numbered for the tetrahedron (newest = 3); map for smaller steps
-      nn = o.n;
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int sj = (o.s[j] == 3) ? (n - 1) : o.s[j];
-        P2[j] = sel3(sj, P[0], P[1], P[2], P[3]);
-        A2[j] = seli(sj, IA[0], IA[1], IA[2], IA[3]);
-        B2[j] = seli(sj, IB[0], IB[1], IB[2], IB[3]);
-      }
-    }
-    if (nn < 4) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        P[j] = P2[j];
-        IA[j] = A2[j];
-        IB[j] = B2[j];
-      }
-    }
-    n = nn;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j < n) wmax2 = fmaxf(wmax2, dot(P[j], P[j]));
-    if (dot(v, v) <= contact * contact * wmax2) {
-      r.exit = GJK_EXIT_CONTACT;
-      r.done = true;
-      return;
+    for (int j = 0; j < 3; ++j) {
+      ias[j] = IA[j];
+      ibs[j] = IB[j];
     }
     if (n == 4) {
-      r.exit = GJK_EXIT_ENCLOSED;
-      r.done = true;
-      return;
+      ias[3] = ia;
+      ibs[3] = ib;
     }
-    if (k == cfg.gjk_max_iter) {
-      r.exit = GJK_EXIT_CAP;
-      r.done = true;
-      return;
+    int order[4] = {0, 1, 2, 3};
+    fv3 vd;
+    nn = escalate_step(B.mem_view(), n, ias, ibs, v, order, &vd, subtab, bits, ~unc);
+    v = vd;
+    r.status |= OGX_S_GJK_ESCALATED;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) slot[j] = order[j];
+  } else {
+    v = step_direction(w, span, o, v);
+    nn = o.n;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) slot[j] = o.s[j];
+  }
+  // does w stay?  (an undecided step keeps the older three)
+  const bool kept = nn == 4 || slot[0] == n - 1 || (nn > 1 && slot[1] == n - 1) || (nn > 2 && slot[2] == n - 1);
+  if (kept) r.wmax2 = fmaxf(r.wmax2, ww);
+  if (r.k == 1 && nn == 2) r.wmax2 = fmaxf(r.wmax2, dot(P[0], P[0]));  // the starting point stays
+  if (nn < 4) {
+    fv3 P2[3];
+    int A2[3], B2[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      P2[j] = sel3(slot[j], P[0], P[1], P[2], w);
+      A2[j] = seli(slot[j], IA[0], IA[1], IA[2], ia);
+      B2[j] = seli(slot[j], IB[0], IB[1], IB[2], ib);
     }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      P[j] = P2[j];
+      IA[j] = A2[j];
+      IB[j] = B2[j];
+    }
+  } else {
+    P[3] = w;
+    IA[3] = ia;
+    IB[3] = ib;
+  }
+  r.n = nn;
+  r.vv = dot(v, v);
+  r.exit = r.vv <= contact * contact * r.wmax2 ? GJK_EXIT_CONTACT
+           : nn == 4                           ? GJK_EXIT_ENCLOSED
+           : r.k == cfg.gjk_max_iter           ? GJK_EXIT_CAP
+                                               : 0;
+  r.done = r.exit != 0;
 }
 
 template <class Team, class Bodies>
@@ -824,46 +578,76 @@ OGX_HD void gjk_pair(const Team& t, const Bodies& B, const Config& cfg, GjkState
 // Exact (FP64) support index of body w along d.  An FP32 scan finds the maximum m of
 // fl(x . d32); every point whose exact value could exceed the true maximum satisfies
 // fl(x . d32) >= m - 2e with e >= |fl(x . d32) - x . d| <= 2 FLT_EPSILON |x|_max |d|_1
-// (rounding of d to FP32 plus the FP32 dot product), so only those few candidates are
-// evaluated in FP64.  Ties go to the lowest index.
+// (rounding of d to FP32 plus the FP32 dot product).  Almost always the maximum is alone in
+// that band (the scan keeps the runner-up) and is the support with no FP64 work -- an FP64
+// instruction costs 65 cycles on this part, an exact support evaluated in FP64 ~4,000 --;
+// otherwise the band's points are evaluated in FP64, ties to the lowest index.
+// amax: the body's largest |coordinate|, or negative to have it found (and returned there).
+// val (may be null): the exact value; err (may be null): e.
 template <class Team, class Bodies, class T>
-OGX_HD int exact_support(const Team& t, const Bodies& B, int w, vec3<T> d, T& val) {
-  const auto& M = B.mem_view();  // points by index (posed where the bodies are)
+OGX_LEAF int exact_support_of(const Team t, const Bodies B, int w, vec3<T> d, float* amax, T* val, float* err) {
   const fv3 fd = v3<float>(to_float(d.x), to_float(d.y), to_float(d.z));
-  const int n = M.n[w];
-  float m = -INFINITY, amax = 0.0f;
-  for (int i = t.lane(); i < n; i += Team::L) {
-    const fv3 p = M.point(w, i);
-    m = fmaxf(m, sdot(p, fd));
-    amax = fmaxf(amax, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
+  const int n = B.n[w];
+  float am = *amax;
+  float best, second;
+  int bi;
+  if (am < 0.0f) {
+    B.template scan_top<true>(t, w, fd, best, bi, second, am);
+    *amax = am = t.fmax_(am);
+  } else {
+    float unused;
+    B.template scan_top<false>(t, w, fd, best, bi, second, unused);
   }
-  m = t.fmax_(m);
-  amax = t.fmax_(amax);
+  float m = best;
+  int mi = bi;
+  t.argmax(m, mi);
   // bodies given in double: the float points are the inputs rounded (half an ulp each),
   // one more FLT_EPSILON * amax * |d|_1 of difference to cover
   const float ef = Bodies::kExact64 ? 5.0f : 4.0f;
-  const float e = ef * FLT_EPSILON * amax * (fabsf(fd.x) + fabsf(fd.y) + fabsf(fd.z)) + FLT_MIN;
+  const float e = ef * FLT_EPSILON * am * (fabsf(fd.x) + fabsf(fd.y) + fabsf(fd.z)) + FLT_MIN;
+  if (err) *err = e;
   const float lo = m - 2.0f * e;
-  T best = sc<T>(-INFINITY);
-  int bi = 0x7fffffff;
-  for (int i = t.lane(); i < n; i += Team::L) {
-    const fv3 pf = M.point(w, i);
-    if (sdot(pf, fd) < lo) continue;
-    T x;
+  auto exact = [&](int i) -> T {
     if constexpr (Bodies::kExact64) {
       const dv3 p = B.dpoint(w, i);
-      x = p.x * d.x + p.y * d.y + p.z * d.z;
+      return p.x * d.x + p.y * d.y + p.z * d.z;
     } else {
-      x = sc<T>(pf.x) * d.x + sc<T>(pf.y) * d.y + sc<T>(pf.z) * d.z;
+      const fv3 p = B.point(w, i);
+      return sc<T>(p.x) * d.x + sc<T>(p.y) * d.y + sc<T>(p.z) * d.z;
     }
-    if (x > best || (x == best && i < bi)) {
-      best = x;
-      bi = i;
+  };
+  if (m > -INFINITY && !t.any((best >= lo && bi != mi) || second >= lo)) {
+    if (val) *val = exact(mi);
+    return mi;
+  }
+  T x1 = sc<T>(-INFINITY);
+  int i1 = 0x7fffffff;
+#pragma unroll 1
+  for (int i = t.lane(); i < n; i += Team::L) {
+    if (sdot(B.point(w, i), fd) < lo) continue;
+    const T x = exact(i);
+    if (x > x1 || (x == x1 && i < i1)) {
+      x1 = x;
+      i1 = i;
     }
   }
-  t.argmax_t(best, bi);
-  val = best;
-  return bi;
+  t.argmax_t(x1, i1);
+  if (val) *val = x1;
+  return i1;
+}
+// (on copies of the team and of the points-by-index view, so that the caller's body source
+// keeps its registers)
+template <class Team, class Bodies, class T>
+OGX_HD int exact_support(const Team& t, const Bodies& B, int w, vec3<T> d, float& amax, T* val = nullptr,
+                         float* err = nullptr) {
+  float am = amax;
+  int i;
+  if constexpr (Bodies::kExact64)
+    i = exact_support_of(t, B, w, d, &am, val, err);
+  else
+    i = exact_support_of(t, B.mem_view(), w, d, &am, val, err);
+  amax = am;
+  return i;
 }
 
 // the Minkowski point a_i - b_j exactly (double), or as double-float components
@@ -893,6 +677,7 @@ struct RefineStateT {
   vec3<T> v;
   T lam[4];   // barycentric weights of v on s (valid while no step changed s)
   bool lam_valid;
+  T vv;       // dot(v, v)
   T wmax2;
   int it, max_iter;
   bool done, enclosed;
@@ -947,6 +732,7 @@ OGX_HD void refine_begin(const Bodies& B, const GjkState& g, int max_iter, Refin
   }
   r.wmax2 = zero;
   for (int j = 0; j < s.n; ++j) r.wmax2 = tmax(r.wmax2, dot(s.v[j].p, s.v[j].p));
+  r.vv = dot(r.v, r.v);
   r.max_iter = max_iter;
   r.enclosed = false;
   r.it = g.certain ? max_iter + 1 : 0;  // the FP32 pass proved the simplex final
@@ -972,6 +758,7 @@ OGX_COLD void closest_exhaustive(Sx<T>& s, vec3<T>& v) {
   T best = T(INFINITY);
   int best_mask = 1 << nw, best_k = 5;
   vec3<T> best_v = s.v[nw].p;
+#pragma unroll 1
   for (int mask = 1; mask < (1 << n); ++mask) {
     if (!(mask & (1 << nw))) continue;
     int idx[4], k = 0;
@@ -1047,26 +834,51 @@ OGX_COLD void closest_exhaustive(Sx<T>& s, vec3<T>& v) {
   v = best_v;
 }
 
-// one iteration with the exact supports xa (body 1 along -v) and xb (body 2 along v)
+// One iteration with the exact supports xa (body 1 along -v) and xb (body 2 along v).  FP64 is
+// spent on the point, the gap, the projection and the predicates FP32 cannot decide; what
+// only guards against rounding is bounded in FP32 first.
 template <class Bodies, class T>
-OGX_HD void refine_step(const Bodies& B, RefineStateT<T>& r, int xa, int xb) {
+OGX_HD void refine_step(const Bodies& B, RefineStateT<T>& r, int xa, int xb, const uint32_t* subtab) {
   Sx<T>& s = r.s;
   const vec3<T> w = mpoint(Tag<T>(), B, xa, xb);
-  const T vv = dot(r.v, r.v);
+  const fv3 wf = v3<float>(to_float(w.x), to_float(w.y), to_float(w.z));
+  fv3 Pf[3];
+  const T vv = r.vv;
   // FP64 gap test.  In exact arithmetic v.p_j = |v|^2 for every vertex p_j of the
   // current feature, so the gap |v|^2 - v.w equals v.(p_j - w); that form rounds in
   // proportion to |p_j - w| (small near convergence) instead of |w|^2.  Relative
   // tolerance of the FP64 oracle (eps * 1e4) and a rounding floor.
-  T gap = sc<T>(INFINITY), dmax = sc<T>(0.0f);
-  for (int j = 0; j < s.n; ++j) {
-    const vec3<T> e = s.v[j].p - w;
-    gap = tmin(gap, dot(r.v, e));
-    dmax = tmax(dmax, dot(e, e));
+  T gap = sc<T>(INFINITY);
+  float dmaxf = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    if (j < s.n) {
+      gap = tmin(gap, dot(r.v, s.v[j].p - w));
+      Pf[j] = v3<float>(to_float(s.v[j].p.x), to_float(s.v[j].p.y), to_float(s.v[j].p.z));
+      const fv3 e = Pf[j] - wf;
+      dmaxf = fmaxf(dmaxf, dot(e, e));
+    } else {
+      Pf[j] = wf;
+    }
   }
-  const T floor64 = T(4.0 * prec_eps<T>()) * tsqrt(r.wmax2) * tsqrt(dmax);
-  if (gap <= T(1e-12) * vv || gap <= floor64) {
+  if (gap <= T(1e-12) * vv) {
     r.done = true;
     return;
+  }
+  // The rounding floor 4 eps max|p| max|p - w|, bounded in FP32 (the rounded points' difference
+  // is within 2^-22 max(|p|, |w|) of the exact one).
+  const float wm = fmaxf(to_float(r.wmax2), dot(wf, wf));
+  const float bound = (float)(4.2 * prec_eps<T>()) * sqrtf(wm) * (sqrtf(dmaxf) + 5e-7f * sqrtf(wm)) + FLT_MIN;
+  if (!(to_float(gap) > bound)) {
+    T dmax = sc<T>(0.0f);
+    for (int j = 0; j < s.n; ++j) {
+      const vec3<T> e = s.v[j].p - w;
+      dmax = tmax(dmax, dot(e, e));
+    }
+    if (gap <= T(4.0 * prec_eps<T>()) * tsqrt(r.wmax2) * tsqrt(dmax)) {
+      r.done = true;
+      return;
+    }
   }
   bool dup = false;
   for (int j = 0; j < s.n; ++j) dup |= (r.ia[j] == xa && r.ib[j] == xb);
@@ -1081,15 +893,20 @@ OGX_HD void refine_step(const Bodies& B, RefineStateT<T>& r, int xa, int xb) {
     pb[j] = r.ib[j];
   }
   const vec3<T> vprev = r.v;
-  s.v[s.n].p = w;
-  s.v[s.n].k = s.n;
-  r.ia[s.n] = xa;
-  r.ib[s.n] = xb;
+  const int nw = s.n;  // the new point's slot
+  s.v[nw].p = w;
+  s.v[nw].k = nw;
+  r.ia[nw] = xa;
+  r.ib[nw] = xb;
   s.n++;
-  Unc u{false};
-  subdistance(s, r.v, u);
+  // predicates outside their FP32 rounding bound on the rounded points are decided there
+  StepIn S;
+  uint32_t bits, unc;
+  step_predicates(s.n, Pf, wf, S, bits, unc);
+  subdistance(s, r.v, subtab, bits, ~unc);
+  T vnew = dot(r.v, r.v);
   r.lam_valid = false;
-  if (s.n != 4 && !(dot(r.v, r.v) < vv * T(1.0 - 1e-12))) {
+  if (s.n != 4 && !(vnew < vv * T(1.0 - 1e-12))) {
     // the region decisions made no progress although the gap says progress is possible:
     // solve the step again by exhaustive search on the grown simplex
     Sx<T> t = prev;
@@ -1101,9 +918,10 @@ OGX_HD void refine_step(const Bodies& B, RefineStateT<T>& r, int xa, int xb) {
     if (t.n == 4 || dot(vt, vt) < vv * T(1.0 - 1e-12)) {
       s = t;
       r.v = vt;
+      vnew = dot(vt, vt);
     }
   }
-  if (s.n != 4 && !(dot(r.v, r.v) < vv * T(1.0 - 1e-12))) {
+  if (s.n != 4 && !(vnew < vv * T(1.0 - 1e-12))) {
     // still none: a tie support spanning a degenerate simplex -- keep the last answer
     s = prev;
     r.v = vprev;
@@ -1114,8 +932,12 @@ OGX_HD void refine_step(const Bodies& B, RefineStateT<T>& r, int xa, int xb) {
     r.done = true;
     return;
   }
+  r.vv = vnew;
+  // (the older vertices are in wmax2 already)
+  bool kept = false;
   int na[4], nb[4];
   for (int j = 0; j < s.n; ++j) {
+    kept = kept || s.v[j].k == nw;
     na[j] = r.ia[s.v[j].k];
     nb[j] = r.ib[s.v[j].k];
   }
@@ -1123,8 +945,8 @@ OGX_HD void refine_step(const Bodies& B, RefineStateT<T>& r, int xa, int xb) {
     r.ia[j] = na[j];
     r.ib[j] = nb[j];
     s.v[j].k = j;
-    r.wmax2 = tmax(r.wmax2, dot(s.v[j].p, s.v[j].p));
   }
+  if (kept && dot(wf, wf) * 1.00001f >= to_float(r.wmax2)) r.wmax2 = tmax(r.wmax2, dot(w, w));
   if (s.n == 4) {
     r.enclosed = true;
     r.done = true;
@@ -1232,18 +1054,19 @@ OGX_HD void refine_certain(const Bodies& B, GjkState& g) {
 }
 
 template <class Team, class Bodies>
-OGX_HD void gjk_refine(const Team& t, const Bodies& B, GjkState& g, int max_iter) {
+OGX_HD void gjk_refine(const Team& t, const Bodies& B, GjkState& g, int max_iter,
+                       const uint32_t* subtab = nullptr) {
   if (g.certain) {
     refine_certain(B, g);
     return;
   }
   RefineState r;
   refine_begin(B, g, max_iter, r);
+  float ma = -1.0f, mb = -1.0f;
   while (!r.done) {
-    double va, vb;
-    const int xa = exact_support(t, B, 0, -r.v, va);
-    const int xb = exact_support(t, B, 1, r.v, vb);
-    refine_step(B, r, xa, xb);
+    const int xa = exact_support(t, B, 0, -r.v, ma);
+    const int xb = exact_support(t, B, 1, r.v, mb);
+    refine_step(B, r, xa, xb, subtab);
   }
   refine_end(B, r, g);
 }

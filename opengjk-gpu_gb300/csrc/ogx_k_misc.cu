@@ -37,13 +37,6 @@ __device__ __forceinline__ bool pair_ok(const DevBatch& B, int2 pr) {
   return pr.x >= 0 && pr.x < B.nbodies && pr.y >= 0 && pr.y < B.nbodies;
 }
 
-__device__ __forceinline__ void mark_bad(const DevBatch& B, int p) {
-  B.dist[p] = __int_as_float(0x7fc00000);
-  if (B.status) B.status[p] = OGX_S_BAD_INPUT;
-  if (B.nrm) store3(B.nrm + 3 * (size_t)p, v3<float>(1.f, 0.f, 0.f));
-  if (B.mode != kModeEpa) B.smp[p].nvrtx = 0;
-}
-
 __global__ void k_bin(DevBatch B) {
   const int stride = gridDim.x * blockDim.x;
   const int n32 = (B.npairs + 31) & ~31;
@@ -120,90 +113,64 @@ __device__ __forceinline__ void bind_mem(Posed<MemBodies>& mb, const DevBatch& B
                                          BodyRef rb) {
   mb.bind_posed(B.pool, ra, rb, B.xf + 12 * (size_t)pr.x, B.xf + 12 * (size_t)pr.y);
 }
-// lane j's bodies, for a scan by the whole warp
+// the bodies of lane j's pair (j may differ from lane to lane)
 __device__ __forceinline__ void shfl_bodies(MemBodies& to, const MemBodies& from, int j) {
+#pragma unroll
   for (int w = 0; w < 2; ++w) {
     to.base[w] = reinterpret_cast<const float*>(
         __shfl_sync(0xffffffffu, reinterpret_cast<long long>(from.base[w]), j));
     to.n[w] = __shfl_sync(0xffffffffu, from.n[w], j);
-    to.n4[w] = __shfl_sync(0xffffffffu, from.n4[w], j);
+    to.n4[w] = round4(to.n[w]);
   }
 }
 __device__ __forceinline__ void shfl_bodies(Posed<MemBodies>& to, const Posed<MemBodies>& from, int j) {
   shfl_bodies(static_cast<MemBodies&>(to), static_cast<const MemBodies&>(from), j);
+#pragma unroll
   for (int w = 0; w < 2; ++w)
     to.xf[w] = reinterpret_cast<const float*>(
         __shfl_sync(0xffffffffu, reinterpret_cast<long long>(from.xf[w]), j));
 }
 
-// Re-solve of separated pairs (one thread per pair).  Pairs whose final support the GJK
-// kernel proved exact only need the exact closest point of their simplex, computed in
-// double-float arithmetic; the others are passed to k_refine_lane / k_refine_full.
+// Re-solve of the separated pairs whose final support the GJK kernel proved exact (one
+// thread per pair): the exact closest point of their simplex in double-float arithmetic.
 template <bool kPosed>
 __global__ void __launch_bounds__(128) k_refine(DevBatch B) {
   const int cnt = B.counts[kCntRefine];
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
-    const RefineRec rr = B.refine[k];
-    const int p = rr.pair;
-    const int2 pr = B.pairs[p];
-    const BodyRef ra = B.bodies[pr.x], rb = B.bodies[pr.y];
-    if (!rr.certain) {
-      if ((ra.n > rb.n ? ra.n : rb.n) <= kRefineLaneMax) {
-        const int q = atomicAdd(B.counts + kCntRefineFull, 1);
-        B.refine_full[q] = p;
-      } else {
-        const int q = atomicAdd(B.counts + kCntRefineBig, 1);
-        B.refine_full[B.npairs - 1 - q] = p;
-      }
-      continue;
-    }
-    typename PoseOf<kPosed, MemBodies>::type mb;
-    bind_mem(mb, B, pr, ra, rb);
-    GjkState g;
-    load_simplex(B.smp + p, B.dist[p], g);
-    g.certain = true;
-    SerialTeam one;
-    gjk_refine(one, mb, g, kRefineIters);
-    refine_store(B, p, ra, rb, g);
-  }
-}
-
-// FP64 continuation of GJK for the pairs with an uncertain FP32 support and bodies of
-// at most kRefineLaneMax points: one thread per pair, so that each FP64 instruction
-// serves 32 pairs (FP64 issues at 1/64 of the FP32 rate here).
-template <bool kPosed>
-__global__ void __launch_bounds__(128) k_refine_lane(DevBatch B) {
-  const int cnt = B.counts[kCntRefineFull];
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
-    const int p = B.refine_full[k];
+    const int p = B.refine[k].pair;
     const int2 pr = B.pairs[p];
     const BodyRef ra = B.bodies[pr.x], rb = B.bodies[pr.y];
     typename PoseOf<kPosed, MemBodies>::type mb;
     bind_mem(mb, B, pr, ra, rb);
     GjkState g;
     load_simplex(B.smp + p, B.dist[p], g);
-    g.certain = false;
-    SerialTeam one;
-    gjk_refine(one, mb, g, kRefineIters);
+    refine_certain(mb, g);
     refine_store(B, p, ra, rb, g);
   }
 }
 
-// The same for larger bodies: a warp takes 32 pairs, one per lane; each FP64 iteration
-// runs the exact-support scans of every unfinished pair with all 32 lanes (pair j's
-// bodies and direction broadcast from lane j), then each lane takes its own pair's FP64
-// sub-distance step, so the scalar FP64 work serves 32 pairs per instruction.
-template <bool kPosed>
-__global__ void __launch_bounds__(128) k_refine_full(DevBatch B) {
-  const WarpTeam<32> t;
+// FP64 continuation of GJK for the pairs whose FP32 support was not certain.  An FP64
+// instruction holds its SM quadrant's FP64 unit for about 65 cycles however many lanes are
+// active (measured, GB300), and a pair's continuation is a chain of a few hundred of them,
+// so what counts is that every quadrant has a warp of its own and that a warp's
+// instructions serve several pairs only once there are more pairs than that: a warp takes
+// ceil(pairs / warps) pairs (1 to 32), one per lane.  Each FP64 iteration scans the warp's
+// unfinished pairs for their exact supports, 32 / TL at a time with teams of TL lanes, then
+// every lane takes its own pair's FP64 sub-distance step.  (32 pairs per warp always, and
+// one thread's serial scans for bodies of at most 128 points, left most SMs idle: 92 + 265
+// us for the 6,600 continuations of 200k power-law pairs.)
+template <int TL, bool kPosed>
+__device__ __forceinline__ void continue_list(const DevBatch& B, int cnt, const int* list, int dir, int warp,
+                                              int nwarps) {
+  const WarpTeam<TL> t;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int cnt = B.counts[kCntRefineBig];
-  for (int base = 32 * warp; base < cnt; base += 32 * nwarps) {
+  constexpr int kTeams = 32 / TL;
+  const int per = min(32, max(1, (cnt + nwarps - 1) / nwarps));
+#pragma unroll 1
+  for (int base = per * warp; base < cnt; base += per * nwarps) {
     const int k = base + lane;
-    const bool valid = k < cnt;
+    const bool valid = lane < per && k < cnt;
     int p = -1;
     BodyRef ra{0u, 1}, rb{0u, 1};
     typename PoseOf<kPosed, MemBodies>::type mb;
@@ -212,7 +179,7 @@ __global__ void __launch_bounds__(128) k_refine_full(DevBatch B) {
     RefineState r;
     r.done = true;
     if (valid) {
-      p = B.refine_full[B.npairs - 1 - k];
+      p = list[dir * k];
       const int2 pr = B.pairs[p];
       ra = B.bodies[pr.x];
       rb = B.bodies[pr.y];
@@ -221,31 +188,58 @@ __global__ void __launch_bounds__(128) k_refine_full(DevBatch B) {
       g.certain = false;
       refine_begin(mb, g, kRefineIters, r);
     }
+#pragma unroll 1
     for (;;) {
       const unsigned m = __ballot_sync(full, !r.done);
       if (m == 0u) break;
       int my_xa = 0, my_xb = 0;
-      for (unsigned mm = m; mm != 0u; mm &= mm - 1u) {
-        const int j = __ffs(mm) - 1;
+#pragma unroll 1
+      for (int j0 = 0; j0 < per; j0 += kTeams) {
+        if (((m >> j0) & ((kTeams == 32 ? 0u : (1u << kTeams)) - 1u)) == 0u) continue;
+        const int j = j0 + lane / TL;  // this team's pair (lane j & 31's)
         typename PoseOf<kPosed, MemBodies>::type bj;
-        shfl_bodies(bj, mb, j);
-        const dv3 vj = v3<double>(__shfl_sync(full, r.v.x, j), __shfl_sync(full, r.v.y, j),
-                                  __shfl_sync(full, r.v.z, j));
-        double va, vb;
-        const int xa = exact_support(t, bj, 0, -vj, va);
-        const int xb = exact_support(t, bj, 1, vj, vb);
-        if (lane == j) {
+        shfl_bodies(bj, mb, j & 31);
+        const dv3 vj = v3<double>(__shfl_sync(full, r.v.x, j & 31), __shfl_sync(full, r.v.y, j & 31),
+                                  __shfl_sync(full, r.v.z, j & 31));
+        int xa = 0, xb = 0;
+        if (j < 32 && ((m >> j) & 1u)) {
+          float ma = -1.0f, mb2 = -1.0f;
+          xa = exact_support(t, bj, 0, -vj, ma);
+          xb = exact_support(t, bj, 1, vj, mb2);
+        }
+        __syncwarp();
+        const int src = ((lane - j0) * TL) & 31;  // the first lane of the team that scanned this lane's pair
+        xa = __shfl_sync(full, xa, src);
+        xb = __shfl_sync(full, xb, src);
+        if (lane >= j0 && lane < j0 + kTeams) {
           my_xa = xa;
           my_xb = xb;
         }
       }
-      if (!r.done) refine_step(mb, r, my_xa, my_xb);
+      if (!r.done) refine_step(mb, r, my_xa, my_xb, B.subtab);
+      __syncwarp();
     }
     if (valid) {
       refine_end(mb, r, g);
       refine_store(B, p, ra, rb, g);
     }
+    __syncwarp();
   }
+}
+
+// the first half of the blocks take the larger bodies' list (filled from the end of
+// refine_full), the others the small ones', each list over the whole grid when the other
+// is empty
+template <bool kPosed>
+__global__ void __launch_bounds__(128, 3) k_refine_cont(DevBatch B) {
+  const int big = B.counts[kCntRefineBig], small = B.counts[kCntRefineFull];
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int split = small == 0 ? nwarps : (big == 0 ? 0 : nwarps / 2);
+  if (warp < split)
+    continue_list<32, kPosed>(B, big, B.refine_full + (B.npairs - 1), -1, warp, split);
+  else
+    continue_list<8, kPosed>(B, small, B.refine_full, 1, warp - split, nwarps - split);
 }
 
 template <bool kPosed>
@@ -381,28 +375,29 @@ cudaError_t launch_polish(const DevBatch& B, int grid, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// k_refine routes the continuations; the two continuation kernels are independent and
-// run on st and st2 (the same stream when st2 == st; the caller joins st2 back)
-cudaError_t launch_refine(const DevBatch& B, int grid, int grid_full, cudaStream_t st, cudaStream_t st2,
-                          cudaEvent_t routed) {
-  if (B.xf)
-    k_refine<true><<<grid, 128, 0, st>>>(B);
-  else
-    k_refine<false><<<grid, 128, 0, st>>>(B);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess && st2 != st) {
-    e = cudaEventRecord(routed, st);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(st2, routed, 0);
+// k_refine and the FP64 continuations touch disjoint pairs and run on st and st2, beside one
+// another when the streams differ (st2 then starts behind `ready`, recorded here; the caller
+// joins it back)
+cudaError_t launch_refine(const DevBatch& B, int grid, int grid_cont, cudaStream_t st, cudaStream_t st2,
+                          cudaEvent_t ready) {
+  cudaError_t e = cudaSuccess;
+  if (st2 != st) {
+    e = cudaEventRecord(ready, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st2, ready, 0);
   }
   if (e != cudaSuccess) return e;
   if (B.xf) {
-    k_refine_lane<true><<<grid, 128, 0, st>>>(B);
-    k_refine_full<true><<<grid_full, 128, 0, st2>>>(B);
+    k_refine_cont<true><<<grid_cont, 128, 0, st2>>>(B);
+    k_refine<true><<<grid, 128, 0, st>>>(B);
   } else {
-    k_refine_lane<false><<<grid, 128, 0, st>>>(B);
-    k_refine_full<false><<<grid_full, 128, 0, st2>>>(B);
+    k_refine_cont<false><<<grid_cont, 128, 0, st2>>>(B);
+    k_refine<false><<<grid, 128, 0, st>>>(B);
   }
   return cudaGetLastError();
+}
+
+cudaError_t continue_occupancy(int block, int* per_sm) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_refine_cont<false>, block, 0);
 }
 
 cudaError_t refine_occupancy(int block, int* per_sm) {

@@ -27,8 +27,10 @@ OGX_HD int bucket_of(int m) {
   return m <= 16 ? 0 : m <= 32 ? 1 : m <= 64 ? 2 : m <= 128 ? 3 : m <= 256 ? 4 : m <= 512 ? 5 : 6;
 }
 
-// FP64 refinement request of a separated pair: the support pair along the final
-// direction and whether the FP32 pass proved it exact
+OGX_HD int bucket_max(int b) { return b == kBuckets - 1 ? 0x7fffffff : 16 << b; }
+
+// FP64 refinement request of a separated pair whose support pair (wa, wb) along the final
+// direction the FP32 pass proved exact
 struct RefineRec {
   int pair;
   int wa, wb;
@@ -48,15 +50,15 @@ enum { kModeGjk = 1, kModeGjkEpa = 2, kModeEpa = 3 };
 constexpr int kCntGjk = 0;                  // [0, kBuckets)
 constexpr int kCntEpa = kBuckets;           // [kBuckets, 2 kBuckets)
 constexpr int kCntPolish = 2 * kBuckets;    // EPA faces to re-solve in FP64
-constexpr int kCntRefine = 2 * kBuckets + 1;  // separated pairs to refine in FP64
-constexpr int kCntRefineFull = 2 * kBuckets + 2;  // of those, the ones to continue in FP64
+constexpr int kCntRefine = 2 * kBuckets + 1;  // separated pairs to re-solve (support certified)
+constexpr int kCntRefineFull = 2 * kBuckets + 2;  // separated pairs to continue in FP64, bodies <= 128 points
 constexpr int kCntSpill = 2 * kBuckets + 3;  // contacts that outgrew the small EPA capacity
-constexpr int kCntRefineBig = 2 * kBuckets + 4;  // of the FP64 continuations, bodies > 128 points
+constexpr int kCntRefineBig = 2 * kBuckets + 4;  // the same, larger bodies
 constexpr int kCntSpillLate = 2 * kBuckets + 5;  // contacts found by the FP64 refinement
 constexpr int kCntResume = 2 * kBuckets + 6;  // capacity spills saved for the full pass to resume
 constexpr int kCntSlots = 2 * kBuckets + 7;
-// FP64 continuations of pairs whose bodies have at most this many points run one thread
-// per pair (FP64 instructions then serve 32 pairs); larger ones one warp per pair
+// FP64 continuations of pairs whose bodies have at most this many points are scanned by
+// teams of 8 lanes, larger ones by whole warps
 constexpr int kRefineLaneMax = 128;
 constexpr int kRefineIters = 16;
 
@@ -143,6 +145,14 @@ __device__ __forceinline__ void store3(float* p, fv3 v) {
   p[2] = v.z;
 }
 
+// a pair that cannot be run: status OGX_PAIR_BAD_INPUT, distance NaN, normal (1, 0, 0)
+__device__ __forceinline__ void mark_bad(const DevBatch& B, int p) {
+  B.dist[p] = __int_as_float(0x7fc00000);
+  if (B.status) B.status[p] = OGX_S_BAD_INPUT;
+  if (B.nrm) store3(B.nrm + 3 * (size_t)p, v3<float>(1.f, 0.f, 0.f));
+  if (B.mode != kModeEpa) B.smp[p].nvrtx = 0;
+}
+
 // ---------------------------------------------------------------------------------
 // source of body points for bucket kernels: registers (K > 0), memory (K == 0), or
 // memory staged through D shared-memory slots per lane (K == 0, D > 0)
@@ -222,15 +232,21 @@ __device__ __forceinline__ void gjk_store(const DevBatch& B, int bucket, int p, 
   const bool to_epa = lead && B.mode == kModeGjkEpa && contact;
   const int e = warp_append(B.counts + kCntEpa + bucket, to_epa);
   if (to_epa) B.elists[(size_t)bucket * B.npairs + e] = p;
-  const int q = warp_append(B.counts + kCntRefine, lead && g.polish);
-  if (lead && g.polish) {
+  const bool refine = lead && g.polish;
+  const int q = warp_append(B.counts + kCntRefine, refine && g.certain);
+  if (refine && g.certain) {
     RefineRec r;
     r.pair = p;
     r.wa = g.wa;
     r.wb = g.wb;
-    r.certain = g.certain ? 1 : 0;
+    r.certain = 1;
     B.refine[q] = r;
   }
+  // the others go to the FP64 continuation's lists at once, so that it need not wait for
+  // the pass over the certain ones
+  const bool small = bucket_max(bucket) <= kRefineLaneMax;
+  const int u = warp_append(B.counts + (small ? kCntRefineFull : kCntRefineBig), refine && !g.certain);
+  if (refine && !g.certain) B.refine_full[small ? u : B.npairs - 1 - u] = p;
 }
 
 template <int L, int K, int OCC = 1, int D = 0, bool kPosed = false>
@@ -392,8 +408,9 @@ int epa_variants_d(const KernelInfo** out);
 void posed_variants(const KernelInfo** gjk, const KernelInfo** epa);
 
 // non-template kernels (ogx_k_misc.cu)
-cudaError_t launch_refine(const DevBatch& B, int grid, int grid_full, cudaStream_t st, cudaStream_t st2,
-                          cudaEvent_t routed);
+cudaError_t launch_refine(const DevBatch& B, int grid, int grid_cont, cudaStream_t st, cudaStream_t st2,
+                          cudaEvent_t ready);
+cudaError_t continue_occupancy(int block, int* per_sm);
 cudaError_t launch_epa_spill(const DevBatch& B, int grid, cudaStream_t st, bool late = false);
 cudaError_t epa_spill_occupancy(int block, int* per_sm);
 cudaError_t refine_occupancy(int block, int* per_sm);

@@ -55,7 +55,7 @@ struct Setup {
   KernelInfo gjk[kBuckets], epa[kBuckets];
   int grid_gjk[kBuckets], grid_epa[kBuckets];
   size_t smem_epa[kBuckets];
-  int grid_bin = 0, grid_refine = 0, grid_polish = 0, grid_spill = 0;
+  int grid_bin = 0, grid_refine = 0, grid_cont = 0, grid_polish = 0, grid_spill = 0;
 };
 
 std::mutex g_mu;
@@ -118,6 +118,9 @@ ogx_status setup(int dev, Setup** out) {
   e = refine_occupancy(kNoAllocBlock, &per);
   if (e != cudaSuccess) return ogx_cuda_fail(e, "occupancy");
   s.grid_refine = std::max(1, per) * sms;
+  e = continue_occupancy(kNoAllocBlock, &per);
+  if (e != cudaSuccess) return ogx_cuda_fail(e, "occupancy");
+  s.grid_cont = std::min(2, std::max(1, per)) * sms;
   e = epa_spill_occupancy(kNoAllocBlock, &per);
   if (e != cudaSuccess) return ogx_cuda_fail(e, "occupancy");
   s.grid_spill = std::max(1, per) * sms;
@@ -191,7 +194,7 @@ extern "C" ogx_status ogx_gjk_epa_noalloc(const float* d_points, const void* d_b
     S->gjk[b].fn<<<S->grid_gjk[b], kNoAllocBlock, 0, s>>>(B, b);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess && (c.flags & OGX_F_FP64_POLISH)) e = launch_refine(B, S->grid_refine, S->grid_bin, s, s, nullptr);
+  if (e == cudaSuccess && (c.flags & OGX_F_FP64_POLISH)) e = launch_refine(B, S->grid_refine, S->grid_cont, s, s, nullptr);
   for (int b = kBuckets - 1; b >= 0 && e == cudaSuccess; --b) {
     S->epa[b].fn<<<S->grid_epa[b], kNoAllocBlock, S->smem_epa[b], s>>>(B, b);
     e = cudaGetLastError();

@@ -183,7 +183,7 @@ OGX_HD SubOut tetra_tree(Bits& B) {
 }
 
 // ------------------------------------------------------------------------------
-// The decision as a table: every outcome of step_decide packed in 32 bits, indexed by
+// The decision as a table: every outcome of the tree packed in 32 bits, indexed by
 // the predicate bits the decision can read (13 for a tetrahedron step, 4 for a triangle,
 // 1 for a segment).  One load replaces the branches of the tree, which the lanes of a
 // warp (different pairs, different bits) would otherwise take one path after another.
@@ -220,12 +220,13 @@ OGX_HD SubOut unpack_subout(uint32_t c) {
 // FP32 predicate values and bounds
 
 struct StepIn {
-  fv3 q1;      // newest point
-  fv3 e[3];    // older points minus q1
-  float a[3];  // q1 . e_k
+  fv3 e[3];    // older points minus the newest
+  float le[3];  // their 1-norms
+  float lq;    // 1-norm of the newest point
+  float a[3];  // newest . e_k
   float g[3][3];
   fv3 c01, c02, c12;  // e0 x e1, e0 x e2, e1 x e2
-  float qc01, qc02, qc12;  // q1 . c
+  float qc01, qc02, qc12;  // newest . c
 };
 
 OGX_HD fv3 sel3(int s, fv3 a, fv3 b, fv3 c, fv3 d) {
@@ -233,16 +234,14 @@ OGX_HD fv3 sel3(int s, fv3 a, fv3 b, fv3 c, fv3 d) {
 }
 OGX_HD int seli(int s, int a, int b, int c, int d) { return s == 0 ? a : (s == 1 ? b : (s == 2 ? c : d)); }
 
-// predicate bits of the n-point step (n = 2, 3, 4; newest point P[n-1]) and the bits of
-// the decisions that fall inside their rounding bound
-OGX_HD void step_predicates(int n, const fv3* P, StepIn& S, uint32_t& bits, uint32_t& unc) {
+// predicate bits of the n-point step (n = 2, 3, 4; older points P[0..n-1), newest q1) and
+// the bits of the decisions that fall inside their rounding bound
+OGX_HD void step_predicates(int n, const fv3* P, fv3 q1, StepIn& S, uint32_t& bits, uint32_t& unc) {
   const float E = FLT_EPSILON;
-  const fv3 q1 = n == 4 ? P[3] : (n == 3 ? P[2] : P[1]);
-  S.q1 = q1;
-  const float lq = l1(q1);
+  const float lq = S.lq = l1(q1);
   bits = 0u;
   unc = 0u;
-  float le[3];
+  float* le = S.le;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     S.e[k] = P[k] - q1;
@@ -294,8 +293,8 @@ OGX_HD void step_predicates(int n, const fv3* P, StepIn& S, uint32_t& bits, uint
   }
 }
 
-// decision of the n-point step from its predicate bits
-OGX_HD SubOut step_decide(int n, uint32_t bits) {
+// decision of the n-point step from its predicate bits, walked through the tree
+OGX_LEAF SubOut step_decide_tree(int n, uint32_t bits) {
   Bits B{bits, 0u};
   SubOut o;
   if (n == 4) {
@@ -309,34 +308,61 @@ OGX_HD SubOut step_decide(int n, uint32_t bits) {
   o.used = B.used;
   return o;
 }
-
-// the whole table (host): entry i is step_decide of the bits that index i
-inline void fill_subtab(uint32_t* tab) {
-  for (uint32_t bits = 0; bits < (1u << 13); ++bits) tab[bits] = pack_subout(step_decide(4, bits));
-  for (uint32_t k = 0; k < 16; ++k) {
-    const uint32_t bits = (k & 3u) | (((k >> 2) & 1u) << (PB_D + 0)) | (((k >> 3) & 1u) << (PB_D + 1));
-    tab[kSubTab3 + k] = pack_subout(step_decide(3, bits));
-  }
-  for (uint32_t k = 0; k < 2; ++k) tab[kSubTab2 + k] = pack_subout(step_decide(2, k));
+// the same: one load from the table where the caller has it (device), else the tree
+OGX_HD SubOut step_decide(int n, uint32_t bits, const uint32_t* subtab) {
+#if defined(__CUDA_ARCH__)
+  if (subtab) return unpack_subout(__ldg(subtab + subtab_index(n, bits)));
+#endif
+  return step_decide_tree(n, bits);
 }
 
-// new direction v from the outcome (all candidates computed, then selected)
-OGX_HD fv3 step_direction(int n, const StepIn& S, const SubOut& o, fv3 vold) {
-  // line through q1 and P_a: v = q1 - e_a (a_a / g_aa)
+// the whole table (host): entry i is step_decide_tree of the bits that index i
+inline void fill_subtab(uint32_t* tab) {
+  for (uint32_t bits = 0; bits < (1u << 13); ++bits) tab[bits] = pack_subout(step_decide_tree(4, bits));
+  for (uint32_t k = 0; k < 16; ++k) {
+    const uint32_t bits = (k & 3u) | (((k >> 2) & 1u) << (PB_D + 0)) | (((k >> 3) & 1u) << (PB_D + 1));
+    tab[kSubTab3 + k] = pack_subout(step_decide_tree(3, bits));
+  }
+  for (uint32_t k = 0; k < 2; ++k) tab[kSubTab2 + k] = pack_subout(step_decide_tree(2, k));
+}
+
+// What the outcome projects the origin on: the line through the newest point along d = e_a
+// or the plane with normal d = e_a x e_b (its sign is irrelevant), the projection's
+// parameter num / den, and whether the span is too degenerate for FP32.
+struct StepSpan {
+  fv3 d;
+  float num, den;
+  bool degenerate;
+};
+OGX_HD StepSpan step_span(const StepIn& S, const SubOut& o) {
   const int a = o.a, b = o.b;
-  const fv3 ea = a == 0 ? S.e[0] : (a == 1 ? S.e[1] : S.e[2]);
-  const float aa = a == 0 ? S.a[0] : (a == 1 ? S.a[1] : S.a[2]);
-  const float gaa = a == 0 ? S.g[0][0] : (a == 1 ? S.g[1][1] : S.g[2][2]);
-  const fv3 vline = S.q1 - ea * (aa / gaa);
-  // plane through q1, P_a, P_b: normal c = e_a x e_b (sign irrelevant), v = c (q1.c)/(c.c)
-  const int pab = (a < b ? a : b) * 3 + (a < b ? b : a);  // 1 -> 01, 2 -> 02, 5 -> 12
-  const fv3 c = pab == 1 ? S.c01 : (pab == 2 ? S.c02 : S.c12);
-  const float qc = pab == 1 ? S.qc01 : (pab == 2 ? S.qc02 : S.qc12);
-  const fv3 vplane = c * (qc / dot(c, c));
+  StepSpan r;
+  const float lq = S.lq;
+  if (o.kind == SO_PLANE) {
+    const int pab = (a < b ? a : b) * 3 + (a < b ? b : a);  // 1 -> 01, 2 -> 02, 5 -> 12
+    r.d = pab == 1 ? S.c01 : (pab == 2 ? S.c02 : S.c12);
+    r.num = pab == 1 ? S.qc01 : (pab == 2 ? S.qc02 : S.qc12);
+    r.den = dot(r.d, r.d);
+    const float la = a == 0 ? S.le[0] : (a == 1 ? S.le[1] : S.le[2]);
+    const float lb = b == 0 ? S.le[0] : (b == 1 ? S.le[1] : S.le[2]);
+    const float bc = 32.0f * FLT_EPSILON * la * lb;
+    r.degenerate = !(r.den > bc * bc);
+  } else {
+    r.d = a == 0 ? S.e[0] : (a == 1 ? S.e[1] : S.e[2]);
+    r.num = a == 0 ? S.a[0] : (a == 1 ? S.a[1] : S.a[2]);
+    r.den = a == 0 ? S.g[0][0] : (a == 1 ? S.g[1][1] : S.g[2][2]);
+    r.degenerate = o.kind == SO_LINE && !(r.den > 64.0f * FLT_EPSILON * FLT_EPSILON * lq * lq);
+  }
+  return r;
+}
+
+// new direction v from the outcome: line v = q1 - d num / den, plane v = d num / den
+OGX_HD fv3 step_direction(fv3 q1, const StepSpan& s, const SubOut& o, fv3 vold) {
+  const float q = s.num / s.den;
   switch (o.kind) {
-    case SO_VERTEX: return S.q1;
-    case SO_LINE: return vline;
-    case SO_PLANE: return vplane;
+    case SO_VERTEX: return q1;
+    case SO_LINE: return q1 - s.d * q;
+    case SO_PLANE: return s.d * q;
     case SO_ZERO: return v3<float>(0.f, 0.f, 0.f);
     default: return vold;
   }
