@@ -29,33 +29,85 @@
 
 namespace ogx {
 
-// Shared-memory working set of one pair, for at most VMAX polytope vertices and FMAX
-// faces (5728 bytes at 68 / 132, the capacity of 64 expansions; 2288 bytes at 28 / 52).
+// A set of faces: one bit per slot, in registers.  put() takes the bits of slots f0..f0+31
+// (f0 a multiple of the team's width, so they lie in one word).
+template <int W>
+struct FaceSet {
+  uint64_t w[W];
+  OGX_HD void clear() {
+#pragma unroll
+    for (int i = 0; i < W; ++i) w[i] = 0u;
+  }
+  OGX_HD void put(int f0, uint32_t bits) {
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+      if (W == 1 || i == (f0 >> 6)) w[i] |= (uint64_t)bits << (f0 & 63);
+  }
+  OGX_HD bool has(int f) const {
+    uint64_t x = w[0];
+#pragma unroll
+    for (int i = 1; i < W; ++i)
+      if (i == (f >> 6)) x = w[i];
+    return (x >> (f & 63) & 1u) != 0u;
+  }
+  OGX_HD int count() const {
+    int n = 0;
+#pragma unroll
+    for (int i = 0; i < W; ++i) n += popc64(w[i]);
+    return n;
+  }
+  // the k-th face of the set (k < count())
+  OGX_HD int nth(int k) const {
+    uint64_t m = w[0];
+    int base = 0;
+#pragma unroll
+    for (int i = 1; i < W; ++i) {
+      const int c = popc64(m);
+      if (base == 64 * (i - 1) && k >= c) {
+        k -= c;
+        m = w[i];
+        base = 64 * i;
+      }
+    }
+#pragma unroll 1
+    for (; k > 0; --k) m &= m - 1u;
+    return base + lowest64(m);
+  }
+};
+
+// Shared-memory working set of one pair, for at most VMAX polytope vertices and FMAX faces.
+// A retired face keeps no flag: its plane is at infinity (never visible, never the closest).
 template <int VMAX, int FMAX>
 struct EpaMemT {
   static constexpr int kV = VMAX;
   static constexpr int kF = FMAX;
-  float4 fn[FMAX];          // unit outward normal, w = plane distance from origin
-  float4 vp[VMAX];          // polytope vertices (Minkowski points)
-  int2 vid[VMAX];           // (index in body 1, index in body 2)
-  uint8_t fv[FMAX][4];      // face vertices a, b, c; [3] = 1 when the face is alive
-  uint8_t fa[FMAX][4];      // fa[f][e]: face across edge e = (v_e, v_{e+1 mod 3})
-  uint8_t vis[FMAX];        // visible from the new point (this step)
-  uint8_t vlist[FMAX];      // visible faces in increasing order (this step)
-  uint8_t hz[FMAX][4];      // horizon edges (this step): a, b, face beyond
-  uint8_t hstart[VMAX];     // new face whose horizon edge starts at vertex
-  uint8_t hend[VMAX];       // new face whose horizon edge ends at vertex
+  typedef FaceSet<(FMAX + 63) / 64> Faces;
+  float4 fn[FMAX];       // unit outward normal, w = plane distance from origin
+  float4 vp[VMAX];       // polytope vertices (Minkowski points)
+  int2 vid[VMAX];        // (index in body 1, index in body 2)
+  uint32_t fv[FMAX];     // face vertices a | b << 8 | c << 16
+  uint16_t fa[FMAX][4];  // across edge e = (v_e, v_{e+1 mod 3}): face | its edge << 8
+  uint32_t hz[FMAX];     // horizon edges (this step): a | b << 8 | face beyond << 16 | its edge << 24
+  uint8_t hstart[VMAX];  // new face whose horizon edge starts at vertex
+  uint8_t hend[VMAX];    // new face whose horizon edge ends at vertex
+  OGX_HD int vertex(int f, int k) const { return (int)((fv[f] >> (8 * k)) & 0xffu); }
+  OGX_HD int beyond(int f, int e) const { return fa[f][e] & 0xff; }
+  OGX_HD bool alive(int f) const { return fn[f].w < INFINITY; }
 };
-// full capacity: every pair within the 64-expansion cap
-typedef EpaMemT<kEpaVmax, kEpaFmax> EpaMem;
-// small capacity: 24 expansions; a pair that needs more is handed to a full-capacity pass
+// small capacity: 24 expansions (2.4 KB); a pair that needs more is handed to a
+// full-capacity pass
 constexpr int kEpaSmallIters = 24;
-typedef EpaMemT<4 + kEpaSmallIters, 4 + 2 * kEpaSmallIters> EpaMemSmall;
-// full capacity for the certified re-run: every face's plane is also kept in FP64
-struct EpaMemCert : EpaMem {
-  double4 fn64[kEpaFmax];  // unit outward normal and plane distance, FP64 from exact points
+struct EpaMemSmall : EpaMemT<4 + kEpaSmallIters, 4 + 2 * kEpaSmallIters> {
+  static constexpr bool kFull = false;
 };
-OGX_HD double4* plane64_slot(EpaMemCert& M, int f) { return &M.fn64[f]; }
+// full capacity: every pair within the 64-expansion cap (68 vertices, 132 faces); for the
+// certified run every face's plane and every vertex are also kept in FP64
+struct EpaMemCert : EpaMemT<kEpaVmax, kEpaFmax> {
+  static constexpr bool kFull = true;
+  double4 fn64[kEpaFmax];  // unit outward normal and plane distance, from exact points
+  dv3 vp64[kEpaVmax];      // exact Minkowski points
+};
+
 // A small-capacity expansion that ran out of room, kept for the full-capacity pass to
 // continue from instead of starting again: the polytope and the loop state at the top of
 // the iteration that overflowed.  The full pass makes the same decisions up to there (the
@@ -66,8 +118,8 @@ struct EpaResume {
   float4 fn[EpaMemSmall::kF];
   float4 vp[EpaMemSmall::kV];
   int2 vid[EpaMemSmall::kV];
-  uint8_t fv[EpaMemSmall::kF][4];
-  uint8_t fa[EpaMemSmall::kF][4];
+  uint32_t fv[EpaMemSmall::kF];
+  uint16_t fa[EpaMemSmall::kF][4];
 };
 // where a spilling expansion saves itself: cap records in buf, *count the next free one
 // (buf null or full: the full pass restarts the contact)
@@ -76,9 +128,6 @@ struct EpaResumeSink {
   int* count;
   int cap;
 };
-template <class Mem>
-OGX_HD double4* plane64_slot(Mem&, int) { return nullptr; }
-
 // The certified re-run.  An FP32 expansion that stops with the support still above the
 // closest face by more than rounding (kEpaCertGain * scale; the FP32 test accepts up to
 // epa_rel * scale), or whose support repeats a vertex before converging, is run again at
@@ -98,6 +147,10 @@ constexpr float kEpaThin = 1e-3f;
 // origin's projection moves to, for the FP32 pass to accept the neighbour's result.
 constexpr float kEpaHopSin2 = 1e-10f;
 constexpr double kEpaCertVis = 1e-12;
+// Certified runs decide visibility on FP64 heights; the FP32 height of the rounded point
+// over the rounded plane differs from it by less than 8 x 2^-24 x (|q|_1 + |w|) < 1.5e-6 scale
+// (q and w at most scale), so farther from zero than this its sign is enough.
+constexpr float kEpaVisBand = 4e-6f;
 
 struct EpaOut {
   float dist;   // -depth for contacts, the GJK distance otherwise
@@ -177,11 +230,14 @@ OGX_HD double4 face_plane64(const Mem& M, const Bodies& B, int a, int b, int c) 
                  B.dpoint(0, M.vid[c].x) - B.dpoint(1, M.vid[c].y));
 }
 
+// (degenerate: w infinite, never the closest face, never visible)
+OGX_HD float4 rounded(double4 p) { return make_float4_((float)p.x, (float)p.y, (float)p.z, (float)p.w); }
+
 // Thin-contact check at FP32 convergence: true when exact supports along face f's FP64
 // plane improve on the face by more than tol.
 template <class Team, class Bodies, class Mem>
 OGX_HD bool thin_gain_exceeds(const Team& t, const Bodies& B, const Mem& M, int f, float tol) {
-  const double4 p = face_plane64(M, B, M.fv[f][0], M.fv[f][1], M.fv[f][2]);
+  const double4 p = face_plane64(M, B, M.vertex(f, 0), M.vertex(f, 1), M.vertex(f, 2));
   if (!(p.w < (double)INFINITY)) return false;
   const dv3 n64 = v3<double>(p.x, p.y, p.z);
   double ha, hb;
@@ -194,7 +250,7 @@ OGX_HD bool thin_gain_exceeds(const Team& t, const Bodies& B, const Mem& M, int 
 // plane of face (a, b, c): FP32, FP64 from exact points for slivers
 template <class Mem, class Bodies>
 OGX_HD float4 face_plane(const Mem& M, const Bodies& B, int a, int b, int c, bool escalate, bool all64,
-                         int& status, double4* p64 = nullptr) {
+                         int& status) {
   const float4 P0 = M.vp[a], P1 = M.vp[b], P2 = M.vp[c];
   const fv3 p0 = v3<float>(P0.x, P0.y, P0.z);
   const fv3 e0 = v3<float>(P1.x, P1.y, P1.z) - p0;
@@ -206,13 +262,7 @@ OGX_HD float4 face_plane(const Mem& M, const Bodies& B, int a, int b, int c, boo
   if (all64 || (escalate && nn < 1e-6f * s * s)) {
     // sine of the face angle below ~1e-3: FP32 normal unreliable
     status |= OGX_S_EPA_ESCALATED;
-    const double4 p = face_plane64(M, B, a, b, c);
-    if (p64) *p64 = p;
-    r.x = (float)p.x;  // degenerate: w infinite, never the closest face, never visible
-    r.y = (float)p.y;
-    r.z = (float)p.z;
-    r.w = (float)p.w;
-    return r;
+    return rounded(face_plane64(M, B, a, b, c));
   }
   if (nn > 0.0f) {
     const float inv = 1.0f / sqrtf(nn);
@@ -283,21 +333,23 @@ template <class Mem, class Bodies>
 // itself, whose closest face is picked on the planes rounded to float, so two faces a
 // rounding apart can swap), the result comes from that near-coplanar neighbour, which
 // holds the projection.
-OGX_HD bool epa_emit(const Mem& M, const Bodies& B, int f, float tie, EpaOut& o, bool rerun_ok) {
-  int a = M.fv[f][0], b = M.fv[f][1], c = M.fv[f][2];
+// dead: faces retired by a step that was not completed.
+OGX_HD bool epa_emit(const Mem& M, const Bodies& B, int f, float tie, EpaOut& o, bool rerun_ok,
+                     const typename Mem::Faces dead) {
+  int a = M.vertex(f, 0), b = M.vertex(f, 1), c = M.vertex(f, 2);
   float l[3];
 #pragma unroll 1
   for (int hop = 0; hop < 4; ++hop) {
-    a = M.fv[f][0];
-    b = M.fv[f][1];
-    c = M.fv[f][2];
+    a = M.vertex(f, 0);
+    b = M.vertex(f, 1);
+    c = M.vertex(f, 2);
     const float4 P0 = M.vp[a], P1 = M.vp[b], P2 = M.vp[c];
     const int out = tri_weights(v3<float>(P0.x, P0.y, P0.z), v3<float>(P1.x, P1.y, P1.z),
                                 v3<float>(P2.x, P2.y, P2.z), l);
     if (out < 0) break;
-    const int g2 = M.fa[f][out];
+    const int g2 = M.beyond(f, out);
     const float4 nf = M.fn[f], ng = M.fn[g2];
-    const bool near = M.fv[g2][3] && fabsf(ng.w - nf.w) <= tie &&
+    const bool near = M.alive(g2) && !dead.has(g2) && fabsf(ng.w - nf.w) <= tie &&
                       (nf.x * ng.x + nf.y * ng.y + nf.z * ng.z) > 1.0f - 1e-5f;
     if (!near) break;
     // In exact arithmetic the origin projects into the closest face of the convex
@@ -396,9 +448,10 @@ OGX_HD void epa_polish(const Bodies& B, EpaOut& o) {
   o.status |= OGX_S_POLISHED;
 }
 
+// saves a small expansion for the full pass
 template <class Team, class Mem>
-OGX_HD void epa_save(const Team& t, const Mem& M, const EpaResumeSink& sink, EpaOut& o, int nv, int fend,
-                     int it, int st, float scale2) {
+OGX_HD void epa_save(const Team& t, const Mem& M, const EpaResumeSink& sink, EpaOut& o, int nv, int fend, int it,
+                     int st, float scale2) {
   if (!sink.buf) return;
   int slot = -1;
   if (t.lane() == 0) {
@@ -419,10 +472,8 @@ OGX_HD void epa_save(const Team& t, const Mem& M, const EpaResumeSink& sink, Epa
 #pragma unroll 1
   for (int f = t.lane(); f < fend; f += Team::L) {
     R.fn[f] = M.fn[f];
-    for (int k = 0; k < 4; ++k) {
-      R.fv[f][k] = M.fv[f][k];
-      R.fa[f][k] = M.fa[f][k];
-    }
+    R.fv[f] = M.fv[f];
+    for (int k = 0; k < 3; ++k) R.fa[f][k] = M.fa[f][k];
   }
   if (t.lane() == 0) {
     R.nv = nv;
@@ -435,32 +486,10 @@ OGX_HD void epa_save(const Team& t, const Mem& M, const EpaResumeSink& sink, Epa
   o.resume = slot;
 }
 
-// Run EPA for one pair whose GJK result is g.  `M` is this pair's shared working set.
-//
-// One expansion step, with the faces of the polytope split over the team's lanes
-// (face f on lane f mod L):
-//   1. every lane tests its live faces for visibility from the new point q and keeps the
-//      closest face that stays (not visible);
-//   2. visible faces are ranked in increasing slot order and horizon edges in increasing
-//      (face, edge) order with ballots, so slot assignment does not depend on L; new face
-//      k takes the k-th visible slot, then fresh slots at the end of the used range;
-//   3. faces beyond the horizon are relinked to the new faces, the visible faces retired;
-//   4. new faces are linked to each other through the per-vertex tables and their planes
-//      computed; the closest new face joins the lane's candidate.
-// The next step's closest face is the team's minimum over the candidates.
-// kCert (the full-capacity re-run only): with FP64 face planes on, run the certified
-// expansion described at kEpaCertGain.
-// sink: where a capacity spill saves itself (small pass); rs: a saved expansion to
-// continue instead of starting from the GJK simplex (full pass).
-template <bool kCert = false, class Team, class Bodies, class Mem>
-OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const GjkState& g,
-                     Mem& M, EpaOut& o, bool can_spill, EpaResumeSink sink = EpaResumeSink{nullptr, nullptr, 0},
-                     const EpaResume* rs = nullptr) {
-  const int L = Team::L;
-  const int lane = t.lane();
-  const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
-  const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
-  const bool cert = kCert && all64;
+// What both capacities start with: the output's defaults, and the GJK simplex grown to a
+// tetrahedron (EPA.c:369-583).  False: the pair is finished (separated, or only touching).
+template <class Team, class Bodies>
+OGX_HD bool epa_begin(const Team& t, const Bodies& B, const GjkState& g, EpaOut& o) {
   o.status = 0;
   o.iters = 0;
   o.polish = false;
@@ -471,48 +500,12 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
   o.w0 = g.w0;
   o.w1 = g.w1;
   o.nrm = unit_or_x(g.w1 - g.w0);
-  if (g.n != 4 && g.dist > FLT_EPSILON) return;  // separated (EPA.c:369-373)
+  if (g.n != 4 && g.dist > FLT_EPSILON) return false;  // separated (EPA.c:369-373)
   o.status |= OGX_S_EPA_RUN;
-  float scale2 = 0.0f;
-  int st = 0;
-  // per-lane closest candidate (slot, plane distance); -1 = none
-  float cbd = INFINITY;
-  int cbest = -1;
-  int nv = 4, fend = 4;
-  int it = 0;
-  if (rs) {
-    nv = rs->nv;
-    fend = rs->fend;
-    it = rs->it;
-    st = rs->st;
-    scale2 = rs->scale2;
-    o.status = rs->status;
-#pragma unroll 1
-    for (int j = lane; j < nv; j += L) {
-      M.vp[j] = rs->vp[j];
-      M.vid[j] = rs->vid[j];
-    }
-#pragma unroll 1
-    for (int f = lane; f < fend; f += L) {
-      M.fn[f] = rs->fn[f];
-      for (int k = 0; k < 4; ++k) {
-        M.fv[f][k] = rs->fv[f][k];
-        M.fa[f][k] = rs->fa[f][k];
-      }
-    }
-    t.sync();
-#pragma unroll 1
-    for (int f = lane; f < fend; f += L)
-      if (M.fv[f][3] && M.fn[f].w < cbd) {
-        cbd = M.fn[f].w;
-        cbest = f;
-      }
-  } else {
-
-  // ---- grow the simplex to a tetrahedron (EPA.c:375-583)
-  // simplex in registers: every index below is a constant after unrolling
-  fv3 P[4];
-  int IA[4], IB[4];
+  return true;
+}
+template <class Team, class Bodies>
+OGX_HD bool epa_grow(const Team& t, const Bodies& B, const GjkState& g, EpaOut& o, fv3* P, int* IA, int* IB) {
   int n = g.n;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -563,55 +556,151 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
       flip = true;
     } else {
       epa_touch(B.point(0, qa), B.point(1, qb), o);
-      return;
+      return false;
     }
   }
+  return true;
+}
 
-  // ---- tetrahedron
-  const float vol = dot(P[1] - P[0], cross(P[2] - P[0], P[3] - P[0]));
-  // outward faces of a positively oriented tetrahedron (0,1,2,3); swap 1 and 2 otherwise:
-  // (0, i2, i1), (0, i1, 3), (i1, i2, 3), (i2, 0, 3).  Face across edge k of face f
-  // (edge k = vertices k, k+1 mod 3) is the same for both orientations.
-  const int i1 = vol >= 0.0f ? 1 : 2, i2 = vol >= 0.0f ? 2 : 1;
-  if (lane == 0) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      M.vp[j] = make_float4_(P[j].x, P[j].y, P[j].z, 0.0f);
-      M.vid[j] = make_int2_(IA[j], IB[j]);
+// the plane of face (a, b, c) into slot s
+template <bool kCert, class Mem, class Bodies>
+OGX_HD float4 set_plane(Mem& M, const Bodies& B, int s, int a, int b, int c, bool escalate, bool all64, bool cert,
+                        int& st) {
+  float4 pl;
+  if constexpr (kCert) {
+    if (cert) {
+      st |= OGX_S_EPA_ESCALATED;
+      const double4 p = plane64(M.vp64[a], M.vp64[b], M.vp64[c]);
+      M.fn64[s] = p;
+      pl = rounded(p);
+      M.fn[s] = pl;
+      return pl;
     }
   }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) scale2 = fmaxf(scale2, dot(P[j], P[j]));
-  t.sync();
+  pl = face_plane(M, B, a, b, c, escalate, all64, st);
+  M.fn[s] = pl;
+  return pl;
+}
+
+// EPA for one pair whose GJK result is g.  `M` is this pair's shared working set.
+//
+// One expansion step, with the faces of the polytope split over the team's lanes
+// (face f on lane f mod L):
+//   1. every lane tests its live faces for visibility from the new point q and keeps the
+//      closest face that stays (not visible);
+//   2. visible faces are ranked in increasing slot order and horizon edges in increasing
+//      (face, edge) order with ballots, so slot assignment does not depend on L; new face
+//      k takes the k-th visible slot, then fresh slots at the end of the used range;
+//   3. faces beyond the horizon are relinked to the new faces, the visible faces retired;
+//   4. new faces are linked to each other through the per-vertex tables and their planes
+//      computed; the closest new face joins the lane's candidate.
+// The next step's closest face is the team's minimum over the candidates.
+//
+// The steps are arranged for the length of the dependent chain, which is what bounds a
+// contact (an expansion by one warp took ~11,000 cycles as byte flags, per-face lists and
+// searched links in shared memory, ~4,000 now): the visible set is a bit set in registers,
+// the horizon one ballot over the visible faces' edges, the relinking one store per edge (a
+// link carries the neighbour's edge), and the scale's square root is taken only when the
+// scale grows.
+//
+// EpaMemSmall: can_spill (always set in the pipelines) lets a contact that needs the full
+// capacity or the certified run leave with o.spill set; sink: where a capacity spill saves
+// itself.  EpaMemCert: no larger capacity; rs: a saved expansion to continue instead of
+// starting from the GJK simplex.  kCert (full capacity only): with FP64 face planes on, run
+// the certified expansion described at kEpaCertGain.
+template <bool kCert = false, class Team, class Bodies, class Mem>
+OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const GjkState& g, Mem& M, EpaOut& o,
+                     bool can_spill, EpaResumeSink sink = EpaResumeSink{nullptr, nullptr, 0},
+                     const EpaResume* rs = nullptr) {
+  static_assert(Mem::kFull || !kCert, "certified runs need the full capacity");
+  const int L = Team::L;
+  const int lane = t.lane();
+  const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
+  const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
+  const bool cert = kCert && all64;
+  // may the contact be run again with FP64 planes?
+  const bool rerun = !Mem::kFull && can_spill && escalate;
+  if (!epa_begin(t, B, g, o)) return;
+  float scale2 = 0.0f;
+  int st = 0;
+  // per-lane closest candidate (slot, plane distance); -1 = none
+  float cbd = INFINITY;
+  int cbest = -1;
+  int nv = 4, fend = 4;
+  int it = 0;
+  if (Mem::kFull && rs) {
+    nv = rs->nv;
+    fend = rs->fend;
+    it = rs->it;
+    st = rs->st;
+    scale2 = rs->scale2;
+    o.status = rs->status;
 #pragma unroll 1
-  for (int f = lane; f < 4; f += L) {
-    const int va = f == 2 ? i1 : (f == 3 ? i2 : 0);
-    const int vb = f == 0 ? i2 : (f == 1 ? i1 : (f == 2 ? i2 : 0));
-    const int vc = f == 0 ? i1 : 3;
-    M.fv[f][0] = (uint8_t)va;
-    M.fv[f][1] = (uint8_t)vb;
-    M.fv[f][2] = (uint8_t)vc;
-    M.fv[f][3] = 1;
-    // {3,2,1}, {0,2,3}, {0,3,1}, {0,1,2}
-    M.fa[f][0] = (uint8_t)(f == 0 ? 3 : 0);
-    M.fa[f][1] = (uint8_t)(f == 0 || f == 1 ? 2 : (f == 2 ? 3 : 1));
-    M.fa[f][2] = (uint8_t)(f == 0 ? 1 : (f == 1 ? 3 : (f == 2 ? 1 : 2)));
-    const float4 pl = face_plane(M, B, va, vb, vc, escalate, all64, st, plane64_slot(M, f));
-    M.fn[f] = pl;
-    if (pl.w < cbd) {
-      cbd = pl.w;
-      cbest = f;
+    for (int j = lane; j < nv; j += L) {
+      M.vp[j] = rs->vp[j];
+      M.vid[j] = rs->vid[j];
     }
+#pragma unroll 1
+    for (int f = lane; f < fend; f += L) {
+      const float4 pl = rs->fn[f];
+      M.fn[f] = pl;
+      M.fv[f] = rs->fv[f];
+      for (int k = 0; k < 3; ++k) M.fa[f][k] = rs->fa[f][k];
+      if (pl.w < cbd) {
+        cbd = pl.w;
+        cbest = f;
+      }
+    }
+    t.sync();
+  } else {
+    fv3 P[4];
+    int IA[4], IB[4];
+    if (!epa_grow(t, B, g, o, P, IA, IB)) return;
+    // outward faces of a positively oriented tetrahedron (0,1,2,3); swap 1 and 2 otherwise:
+    // (0, i2, i1), (0, i1, 3), (i1, i2, 3), (i2, 0, 3).  The face across edge k of face f
+    // (edge k = vertices k, k+1 mod 3) and its edge are the same for both orientations:
+    // {3,2,1}, {0,2,3}, {0,3,1}, {0,1,2} across edges {0,0,0}, {2,2,1}, {1,2,1}, {0,2,1}.
+    const float vol = dot(P[1] - P[0], cross(P[2] - P[0], P[3] - P[0]));
+    const int i1 = vol >= 0.0f ? 1 : 2, i2 = vol >= 0.0f ? 2 : 1;
+    if (lane == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        M.vp[j] = make_float4_(P[j].x, P[j].y, P[j].z, 0.0f);
+        M.vid[j] = make_int2_(IA[j], IB[j]);
+        if constexpr (kCert)
+          if (cert) M.vp64[j] = B.dpoint(0, IA[j]) - B.dpoint(1, IB[j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) scale2 = fmaxf(scale2, dot(P[j], P[j]));
+    t.sync();
+#pragma unroll 1
+    for (int f = lane; f < 4; f += L) {
+      const int va = f == 2 ? i1 : (f == 3 ? i2 : 0);
+      const int vb = f == 0 ? i2 : (f == 1 ? i1 : (f == 2 ? i2 : 0));
+      const int vc = f == 0 ? i1 : 3;
+      M.fv[f] = (uint32_t)(va | vb << 8 | vc << 16);
+      M.fa[f][0] = (uint16_t)(f == 0 ? 3 : (f == 1 ? 0 | 2 << 8 : (f == 2 ? 0 | 1 << 8 : 0)));
+      M.fa[f][1] = (uint16_t)(f == 0 ? 2 : (f == 1 ? 2 | 2 << 8 : (f == 2 ? 3 | 2 << 8 : 1 | 2 << 8)));
+      M.fa[f][2] = (uint16_t)(f == 0 ? 1 : (f == 1 ? 3 | 1 << 8 : (f == 2 ? 1 | 1 << 8 : 2 | 1 << 8)));
+      const float4 pl = set_plane<kCert>(M, B, f, va, vb, vc, escalate, all64, cert, st);
+      if (pl.w < cbd) {
+        cbd = pl.w;
+        cbest = f;
+      }
+    }
+    t.sync();
   }
-  t.sync();
-  }
-
-  const float tol_floor = cfg.epa_tol;
+  float root = sqrtf(scale2);  // of scale2
   int best = -1;
   bool done = false;
   bool thin = false;
   float thin_tol = 0.0f;
+  typename Mem::Faces dead;  // faces retired by a step that stops half way
+  dead.clear();
+  bool again = false;  // leave for the certified run
   float amax0 = -1.0f, amax1 = -1.0f;  // the bodies' largest |coordinate| (certified run)
+#pragma unroll 1
   while (it < cfg.epa_max_iter) {
     ++it;
     // closest live face
@@ -624,42 +713,58 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
       done = true;
       break;
     }
-    const float4 nf = M.fn[best];
-    const fv3 n = v3<float>(nf.x, nf.y, nf.z);
     int qa, qb;
     fv3 q;
     dv3 q64 = v3<double>(0.0, 0.0, 0.0);
-    float scale;
+    float qq, scale;  // |q|^2, sqrt(max(scale2, |q|^2))
     bool conv;
-    float gain = 0.0f;
-    if (cert) {
-      // exact supports along the closest face's FP64 normal
-      const double4 pl = *plane64_slot(M, best);
-      const dv3 n64 = v3<double>(pl.x, pl.y, pl.z);
-      double ha, hb;
-      qa = exact_support(t, B, 0, n64, amax0, &ha);
-      qb = exact_support(t, B, 1, -n64, amax1, &hb);
-      q = B.point(0, qa) - B.point(1, qb);
-      q64 = B.dpoint(0, qa) - B.dpoint(1, qb);
-      scale = sqrtf(fmaxf(scale2, dot(q, q)));
-      conv = !(ha + hb - pl.w > kEpaCertTol * fmax(1.0, (double)scale));
+    float gain = 0.0f, tol = 0.0f;
+    if (kCert && cert) {
+      if constexpr (kCert) {
+        // exact supports along the closest face's FP64 normal
+        const double4 pl = M.fn64[best];
+        const dv3 n64 = v3<double>(pl.x, pl.y, pl.z);
+        float ea, eb;
+        qa = exact_support<Team, Bodies, double>(t, B, 0, n64, amax0, nullptr, &ea);
+        qb = exact_support<Team, Bodies, double>(t, B, 1, -n64, amax1, nullptr, &eb);
+        const fv3 pa = B.point(0, qa), pb = B.point(1, qb);
+        q = pa - pb;
+        q64 = B.dpoint(0, qa) - B.dpoint(1, qb);
+        qq = dot(q, q);
+        scale = qq > scale2 ? sqrtf(qq) : root;
+        // The support's gain over the face.  Its FP32 value is within ea + eb (the supports'
+        // bounds) and a few roundings of the terms; only a gain nearer the tolerance than that
+        // is evaluated in FP64.
+        const float fa = sdot(pa, v3<float>((float)pl.x, (float)pl.y, (float)pl.z));
+        const float fb = sdot(pb, v3<float>((float)-pl.x, (float)-pl.y, (float)-pl.z));
+        const float fw = (float)pl.w;
+        const float slack = 2.0f * (ea + eb) + 4.0f * FLT_EPSILON * (fabsf(fa) + fabsf(fb) + fabsf(fw)) +
+                            2e-10f * fmaxf(1.0f, scale);
+        conv = !(fa + fb - fw > slack);
+        if (conv) {
+          const dv3 xa = B.dpoint(0, qa), xb = B.dpoint(1, qb);
+          const double ha = xa.x * n64.x + xa.y * n64.y + xa.z * n64.z;
+          const double hb = xb.x * -n64.x + xb.y * -n64.y + xb.z * -n64.z;
+          conv = !(ha + hb - pl.w > kEpaCertTol * fmax(1.0, (double)scale));
+        }
+      }
     } else {
+      const float4 nf = M.fn[best];
+      const fv3 n = v3<float>(nf.x, nf.y, nf.z);
       q = msupport(t, B, n, qa, qb);
-      scale = sqrtf(fmaxf(scale2, dot(q, q)));
-      const float tol = fmaxf(tol_floor, cfg.epa_rel * scale);
+      qq = dot(q, q);
+      scale = qq > scale2 ? sqrtf(qq) : root;
+      tol = fmaxf(cfg.epa_tol, cfg.epa_rel * scale);
       gain = dot(n, q) - bd;
       conv = gain < tol;
-      // a thin contact: the FP32 test may have been fooled by the face normal's rounding;
-      // checked after the loop (its FP64 scans would weigh on the loop's registers)
-      thin = conv && !all64 && escalate && can_spill && !(gain > kEpaCertGain * scale) && bd < kEpaThin * scale;
-      thin_tol = tol;
     }
     if (conv) {
-      if (!cert && escalate && can_spill && !all64 && gain > kEpaCertGain * scale) {
-        o.spill = true;
-        o.spill64 = true;
-        return;
-      }
+      // with room left for an improvement, the certified run decides
+      again = rerun && !all64 && gain > kEpaCertGain * scale;
+      // a thin contact: the FP32 test may have been fooled by the face normal's rounding;
+      // checked after the loop (its FP64 scans would weigh on the loop's registers)
+      thin = rerun && !all64 && !(gain > kEpaCertGain * scale) && bd < kEpaThin * scale;
+      thin_tol = tol;
       o.status |= OGX_S_EPA_CONVERGED;
       done = true;
       break;
@@ -673,17 +778,13 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
     if (t.any(dup)) {
       // the support is already a vertex although the closest face is not converged:
       // FP32 planes put a vertex in front of a face; re-run certified
-      if (!cert && escalate && can_spill && !all64) {
-        o.spill = true;
-        o.spill64 = true;
-        return;
-      }
+      again = rerun && !all64;
       o.status |= OGX_S_EPA_DUPLICATE;
       done = true;
       break;
     }
     if (nv >= Mem::kV) {
-      if (can_spill) {
+      if (!Mem::kFull && can_spill) {
         epa_save(t, M, sink, o, nv, fend, it - 1, st, scale2);
         o.spill = true;
         return;
@@ -696,88 +797,77 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
     if (lane == 0) {
       M.vp[p] = make_float4_(q.x, q.y, q.z, 0.0f);
       M.vid[p] = make_int2_(qa, qb);
+      if constexpr (kCert)
+        if (cert) M.vp64[p] = q64;
     }
     ++nv;
-    scale2 = fmaxf(scale2, dot(q, q));
+    scale2 = fmaxf(scale2, qq);
+    root = scale;
     const float vis_eps = cfg.epa_vis * scale;
 
     // 1. faces seen from q; the closest face that stays
     cbd = INFINITY;
     cbest = -1;
-    int nvis = 0;
+    typename Mem::Faces vis;
+    vis.clear();
 #pragma unroll 1
     for (int f0 = 0; f0 < fend; f0 += L) {
       const int f = f0 + lane;
-      bool s = false;
-      if (f < fend && M.fv[f][3]) {
-        const float4 fp = M.fn[f];
+      float4 fp = make_float4_(0.0f, 0.0f, 0.0f, INFINITY);
+      if (f < fend) fp = M.fn[f];
+      const float h = (fp.x * q.x + fp.y * q.y + fp.z * q.z) - fp.w;
+      bool s = h > vis_eps;
+      if constexpr (kCert) {
         if (cert) {
-          const double4 pl = *plane64_slot(M, f);
-          s = (pl.x * q64.x + pl.y * q64.y + pl.z * q64.z) - pl.w > kEpaCertVis * (double)scale;
-        } else {
-          s = (fp.x * q.x + fp.y * q.y + fp.z * q.z) - fp.w > vis_eps;
-        }
-        if (!s && fp.w < cbd) {
-          cbd = fp.w;
-          cbest = f;
+          // the rounded plane and point are within 2e-6 scale of the FP64 height: only
+          // heights nearer zero than that need it
+          s = h > 0.0f;
+          if (f < fend && fabsf(h) <= kEpaVisBand * scale) {
+            const double4 pl = M.fn64[f];
+            s = (pl.x * q64.x + pl.y * q64.y + pl.z * q64.z) - pl.w > kEpaCertVis * (double)scale;
+          }
         }
       }
-      if (f < fend) M.vis[f] = s;
-      const uint32_t m = t.ballot(s);
-      if (s) M.vlist[nvis + popc32(m & t.below())] = (uint8_t)f;
-      nvis += popc32(m);
-    }
-    t.sync();
-    // the closest face must be seen (gain >= tol > vis threshold); otherwise stop (or,
-    // from the small pass, start again with FP64 planes in the full pass)
-    if (!M.vis[best]) {
-      if (can_spill && escalate) {
-        o.spill = true;
-        o.spill64 = true;
-        return;
+      if (!s && fp.w < cbd) {
+        cbd = fp.w;
+        cbest = f;
       }
-      o.status |= OGX_S_EPA_TOPOLOGY;
-      done = true;
-      break;
+      vis.put(f0, t.ballot(s));
     }
     // 2. horizon edges: edge e of a visible face whose neighbour is not visible
+    const int nvis = vis.count();
     int htot = 0;
 #pragma unroll 1
-    for (int k0 = 0; k0 < nvis; k0 += L) {
-      const int k = k0 + lane;
-      bool h[3] = {false, false, false};
-      int f = 0;
-      if (k < nvis) {
-        f = M.vlist[k];
-        for (int e = 0; e < 3; ++e) h[e] = !M.vis[M.fa[f][e]];
+    for (int i0 = 0; i0 < 3 * nvis; i0 += L) {
+      const int i = i0 + lane;
+      bool h = false;
+      uint32_t edge = 0u;
+      if (i < 3 * nvis) {
+        const int k = (int)(((uint32_t)i * 43691u) >> 17);  // i / 3
+        const int e = i - 3 * k;
+        const int f = vis.nth(k);
+        const uint32_t nb = M.fa[f][e], v = M.fv[f];
+        h = !vis.has((int)(nb & 0xffu));
+        edge = ((v >> (8 * e)) & 0xffu) | ((v >> (e == 2 ? 0 : 8 * e + 8)) & 0xffu) << 8 | (nb & 0xffu) << 16 |
+               (nb >> 8) << 24;
       }
-      const uint32_t m0 = t.ballot(h[0]), m1 = t.ballot(h[1]), m2 = t.ballot(h[2]);
-      const uint32_t lo = t.below();
-      int r = htot + popc32(m0 & lo) + popc32(m1 & lo) + popc32(m2 & lo);
-      for (int e = 0; e < 3; ++e) {
-        if (!h[e]) continue;
-        if (r < Mem::kF) {
-          M.hz[r][0] = M.fv[f][e];
-          M.hz[r][1] = M.fv[f][(e + 1) % 3];
-          M.hz[r][2] = M.fa[f][e];
-        }
-        ++r;
-      }
-      htot += popc32(m0) + popc32(m1) + popc32(m2);
+      const uint32_t m = t.ballot(h);
+      const int r = htot + popc32(m & t.below());
+      if (h && r < Mem::kF) M.hz[r] = edge;
+      htot += popc32(m);
     }
-    // new face k goes to vlist[k] (k < nvis), else to fresh slot fend + k - nvis
-    if (htot < 3) {
-      if (can_spill && escalate) {
-        o.spill = true;
-        o.spill64 = true;
-        return;
-      }
+    // the closest face must be seen (gain >= tol > vis threshold) and have a horizon;
+    // otherwise stop, or start again with FP64 planes in the full pass
+    if (!vis.has(best) || htot < 3) {
+      again = rerun;
       o.status |= OGX_S_EPA_TOPOLOGY;
       done = true;
       break;
     }
-    if (fend + (htot > nvis ? htot - nvis : 0) > Mem::kF) {
-      if (can_spill) {
+    // new face k goes to the k-th visible slot, else to fresh slot fend + k - nvis
+    const int fresh = htot > nvis ? htot - nvis : 0;
+    if (fend + fresh > Mem::kF) {
+      if (!Mem::kFull && can_spill) {
         epa_save(t, M, sink, o, nv - 1, fend, it - 1, st, scale2);  // before q was added
         o.spill = true;
         return;
@@ -787,84 +877,74 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
       break;
     }
     t.sync();
-    // 3. relink the faces outside the horizon, index the horizon by its vertices, retire
-    // the visible faces
+    // 3. relink the faces outside the horizon, index the horizon by its vertices
 #pragma unroll 1
     for (int k = lane; k < htot; k += L) {
-      const int s = k < nvis ? M.vlist[k] : fend + k - nvis;
-      const int a = M.hz[k][0], b = M.hz[k][1], g2 = M.hz[k][2];
-      for (int m = 0; m < 3; ++m)
-        if (M.fv[g2][m] == b && M.fv[g2][(m + 1) % 3] == a) M.fa[g2][m] = (uint8_t)s;
-      M.hstart[a] = (uint8_t)s;
-      M.hend[b] = (uint8_t)s;
+      const int s = k < nvis ? vis.nth(k) : fend + k - nvis;
+      const uint32_t h = M.hz[k];
+      M.fa[(h >> 16) & 0xffu][h >> 24] = (uint16_t)s;
+      M.hstart[h & 0xffu] = (uint8_t)s;
+      M.hend[(h >> 8) & 0xffu] = (uint8_t)s;
     }
-#pragma unroll 1
-    for (int k = lane; k < nvis; k += L) M.fv[M.vlist[k]][3] = 0;
     t.sync();
     // a vertex that starts (or ends) two horizon edges means the horizon is not one
     // simple loop; keep the closest face found this step and stop
     bool bad = false;
 #pragma unroll 1
     for (int k = lane; k < htot; k += L) {
-      const int s = k < nvis ? M.vlist[k] : fend + k - nvis;
-      bad |= (M.hstart[M.hz[k][0]] != s) || (M.hend[M.hz[k][1]] != s);
+      const int s = k < nvis ? vis.nth(k) : fend + k - nvis;
+      const uint32_t h = M.hz[k];
+      bad |= (M.hstart[h & 0xffu] != s) || (M.hend[(h >> 8) & 0xffu] != s);
     }
     if (t.any(bad)) {
-      if (can_spill && escalate) {
-        o.spill = true;
-        o.spill64 = true;
-        return;
-      }
+      again = rerun;
       o.status |= OGX_S_EPA_TOPOLOGY;
+      dead = vis;
       done = true;
       break;
     }
     // 4. new face (a, b, p) across each horizon edge a->b
 #pragma unroll 1
     for (int k = lane; k < htot; k += L) {
-      const int s = k < nvis ? M.vlist[k] : fend + k - nvis;
-      const int a = M.hz[k][0], b = M.hz[k][1];
-      M.fv[s][0] = (uint8_t)a;
-      M.fv[s][1] = (uint8_t)b;
-      M.fv[s][2] = (uint8_t)p;
-      M.fa[s][0] = M.hz[k][2];
-      M.fa[s][1] = M.hstart[b];
-      M.fa[s][2] = M.hend[a];
-      const float4 pl = face_plane(M, B, a, b, p, escalate, all64, st, plane64_slot(M, s));
-      M.fn[s] = pl;
-      M.fv[s][3] = 1;
+      const int s = k < nvis ? vis.nth(k) : fend + k - nvis;
+      const uint32_t h = M.hz[k];
+      const int a = (int)(h & 0xffu), b = (int)((h >> 8) & 0xffu);
+      M.fv[s] = (h & 0xffffu) | (uint32_t)p << 16;
+      M.fa[s][0] = (uint16_t)((h >> 16 & 0xffu) | (h >> 24) << 8);
+      M.fa[s][1] = (uint16_t)(M.hstart[b] | 2u << 8);
+      M.fa[s][2] = (uint16_t)(M.hend[a] | 1u << 8);
+      const float4 pl = set_plane<kCert>(M, B, s, a, b, p, escalate, all64, cert, st);
       if (pl.w < cbd || (pl.w == cbd && s < cbest)) {
         cbd = pl.w;
         cbest = s;
       }
     }
-    if (htot > nvis) fend += htot - nvis;
+#pragma unroll 1
+    for (int k = htot + lane; k < nvis; k += L) {
+      const int s = vis.nth(k);
+      M.fn[s] = make_float4_(0.0f, 0.0f, 0.0f, INFINITY);
+    }
+    fend += fresh;
     t.sync();
   }
-  o.iters = it;
-  o.status |= st ? OGX_S_EPA_ESCALATED : 0;
-  o.status |= cert ? OGX_S_EPA_CERTIFIED : 0;
-  if (!done) {
-    // iteration cap: closest current face
-    float bd = cbd;
-    best = cbest;
-    t.argmin(bd, best);
-    o.status |= OGX_S_EPA_CAP;
-  }
-  if (thin && best >= 0 && thin_gain_exceeds(t, B, M, best, thin_tol)) {
-    o.spill = true;
-    o.spill64 = true;
-    return;
-  }
-  if (best >= 0) {
-    const bool rerun = !cert && escalate && can_spill && !all64;
-    if (epa_emit(M, B, best, fmaxf(cfg.epa_tol, cfg.epa_rel * sqrtf(scale2)), o, rerun)) {
-      o.spill = true;
-      o.spill64 = true;
-      return;
+  if (!again) {
+    o.iters = it;
+    o.status |= st ? OGX_S_EPA_ESCALATED : 0;
+    o.status |= cert ? OGX_S_EPA_CERTIFIED : 0;
+    if (!done) {
+      // iteration cap: closest current face
+      float bd = cbd;
+      best = cbest;
+      t.argmin(bd, best);
+      o.status |= OGX_S_EPA_CAP;
     }
-    o.polish = (cfg.flags & OGX_F_FP64_POLISH) != 0;
+    if (!Mem::kFull && thin && best >= 0) again = thin_gain_exceeds(t, B, M, best, thin_tol);
+    if (!again && best >= 0) {
+      again = epa_emit(M, B, best, fmaxf(cfg.epa_tol, cfg.epa_rel * sqrtf(scale2)), o, rerun && !all64, dead);
+      o.polish = !again && (cfg.flags & OGX_F_FP64_POLISH) != 0;
+    }
   }
+  o.spill = o.spill64 = again;
 }
 
 }  // namespace ogx
