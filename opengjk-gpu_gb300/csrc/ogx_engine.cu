@@ -3,7 +3,7 @@
 //
 // Pipeline of one batched call (all on the context's stream, no host synchronisation):
 //   memset counters -> k_bin -> k_gjk x 7 buckets (largest first) -> k_epa x 7 ->
-//   k_polish
+//   k_polish; for small batches memset counters -> k_warp_pair
 // Grids are fixed per kernel (occupancy x SM count) and the kernels stride over
 // device-side work lists, so a call is a fixed sequence of launches that can be
 // captured in a CUDA graph by the caller.
@@ -100,11 +100,15 @@ std::vector<Launch> g_gjkv, g_epav;  // all compiled variants
 std::vector<Launch> g_gjkp, g_epap;  // the posed kernels, one per bucket
 
 constexpr int kBlock = 128;
+// largest batches of the one-warp-per-pair pipeline (distances only / with EPA) and of EPA
+// with one warp per contact in the bucket kernels (ogx_run has the measurements)
+constexpr int kWarpPairsGjk = 4096, kWarpPairsEpa = 2048, kWideEpaPairs = 24576;
 constexpr int kBucketCap[kBuckets] = {16, 32, 64, 128, 256, 512, 0};
 
 std::mutex g_init_mu;
 int g_init_device = -1;
 int g_grid_bin = 0, g_grid_polish = 0, g_grid_pack = 0, g_grid_refine = 0, g_grid_cont = 0, g_grid_spill = 0;
+int g_epa_wide[kBuckets];  // EPA variant with one warp per contact, per bucket
 uint32_t* g_subtab = nullptr;  // sub-distance decision table on the initialised device
 // per-device autotuned choices (variant index per bucket), -1 = not tuned
 int g_tuned[16][2][kBuckets];
@@ -229,6 +233,7 @@ ogx_status init_kernels(int device) {
       if (s) return s;
     }
   }
+  for (int b = 0; b < kBuckets; ++b) g_epa_wide[b] = warp_choice(g_epav, b);
   g_grid_bin = 4 * sms;
   g_grid_pack = 8 * sms;
   int per_sm = 0;
@@ -759,6 +764,21 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
                                            "epa<=256", "epa<=512", "epa>512"};
   cudaError_t e = cudaMemsetAsync(ctx->d_counts, 0, kCntSlots * sizeof(int), st);
   if (e != cudaSuccess) return ogx_cuda_fail(e, "counter reset");
+  // Small batches: the whole pipeline with one warp per pair, one launch.  Measured against
+  // the bucket kernels (device pairs, one call after another): 256 power-law pairs 54 us
+  // against 146, 2,000 160 against 250, 3,000 278 against 265; distances only, 3,000 pairs of
+  // 32-point bodies 50 us against 93, 4,000 of 16-point ones 62 against 81, 10,000 117 against 81.
+  const int warp_max = mode == kModeGjk ? kWarpPairsGjk : kWarpPairsEpa;
+  if (npairs <= warp_max && !d_xf && !ctx->choice_set && !ctx->timing && !ctx->stages) {
+    e = launch_warp_pairs(B, st);
+    if (e != cudaSuccess) return ogx_cuda_fail(e, "k_warp_pair launch");
+    ctx->last_launches = 1;
+    return OGX_OK;
+  }
+  // EPA with one warp per contact where the contacts of a batch cannot fill the GPU with
+  // narrower teams: a contact then ends sooner (10,000 pairs 253-286 us against 289-335;
+  // 20,000 318-342 against 349-353; 50,000 586-599 against 524-574).
+  const bool wide_epa = npairs <= kWideEpaPairs && !d_xf && !ctx->choice_set;
   const int bin_grid = std::min(g_grid_bin, (npairs + 255) / 256);
   ctx->mark("bin");
   e = launch_bin(B, bin_grid, st);
@@ -822,7 +842,7 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   const bool refine = mode != kModeEpa && (ctx->cfg.flags & OGX_F_FP64_POLISH);
   if (mode != kModeGjk) {
     for (int b = kBuckets - 1; b >= 0 && e == cudaSuccess; --b) {
-      const Launch& k = d_xf ? g_epap[b] : g_epav[ctx->choice[1][b]];
+      const Launch& k = d_xf ? g_epap[b] : g_epav[wide_epa ? g_epa_wide[b] : ctx->choice[1][b]];
       ctx->mark(kEpaName[b]);
       k.fn<<<fit_grid(k.grid, npairs, k.L), kBlock, k.smem, bucket_stream(b)>>>(B, b);
       stage(kEpaName[b], bucket_stream(b));
@@ -937,6 +957,7 @@ extern "C" ogx_status ogx_ctx_set_kernel_choice(ogx_ctx* ctx, int kind, int buck
   for (int i = 0; i < (int)vs.size(); ++i)
     if (vs[i].L == lanes && vs[i].K == blocks && serves(vs[i], bucket)) {
       ctx->choice[kind][bucket] = i;
+      ctx->choice_set = true;
       return OGX_OK;
     }
   return ogx_fail(OGX_ERR_INVALID, "no variant (%d lanes, %d blocks) for bucket %d", lanes, blocks, bucket);
@@ -1049,7 +1070,8 @@ extern "C" ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npair
       best[kind][b] = INFINITY;
       pick[kind][b] = pick_prior[kind][b] = ctx->choice[kind][b];
     }
-  const bool was_timing = ctx->timing;
+  const bool was_timing = ctx->timing, was_set = ctx->choice_set;
+  ctx->choice_set = true;  // the bucket kernels are what is timed, at every batch size
   ogx_status s = ogx_ctx_set_timing(ctx, 1);
   for (int r = 0; r < rounds && !s; ++r) {
     for (int kind = 0; kind < 2; ++kind)
@@ -1119,6 +1141,7 @@ extern "C" ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npair
         for (int b = 0; b < kBuckets; ++b) pick[kind][b] = prior[kind][b];
   }
   ogx_ctx_set_timing(ctx, was_timing);
+  ctx->choice_set = was_set;
   cudaFree(smp);
   cudaFree(dist);
   cudaFree(nrm);

@@ -33,6 +33,7 @@ struct ogx_ctx {
   size_t d_stage_bytes = 0;
   int last_launches = 0;
   int choice[2][ogx::kBuckets] = {};  // kernel variant per bucket: [0] GJK, [1] EPA
+  bool choice_set = false;  // the caller chose a variant: every call runs the bucket kernels
   // optional per-launch timing (CUDA events recorded between the launches of a call)
   bool timing = false;
   static constexpr int kMaxTimed = 32;
