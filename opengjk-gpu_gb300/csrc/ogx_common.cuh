@@ -345,6 +345,8 @@ struct SerialTeam {
   template <class T>
   OGX_HD void argmax_t(T&, int&) const {}
   OGX_HD bool any(bool p) const { return p; }
+  OGX_HD bool warp_any(bool p) const { return p; }
+  OGX_HD int warp_max(int x) const { return x; }
   OGX_HD uint32_t ballot(bool p) const { return p ? 1u : 0u; }
   OGX_HD uint32_t below() const { return 0u; }
   OGX_HD int excl_scan(int x, int& total) const {
@@ -368,8 +370,12 @@ __device__ __forceinline__ uint32_t order_key(float v) {
 __device__ __forceinline__ float order_value(uint32_t k) {
   return __uint_as_float(k ^ (~(uint32_t)((int32_t)k >> 31) | 0x80000000u));
 }
-// L consecutive lanes of a warp (L a power of two <= 32).
-template <int L_>
+// L consecutive lanes of a warp (L a power of two <= 32).  kAll: the warp's teams go through
+// every operation together (the caller's control flow is the same for the whole warp, with
+// teams that have nothing to do passing `live` = false), so the operations name all 32 lanes
+// and the teams cannot drift apart and run one after another.  Otherwise each team is on its
+// own.
+template <int L_, bool kAll = false>
 struct WarpTeam {
   static constexpr int L = L_;
   unsigned mask;
@@ -380,6 +386,11 @@ struct WarpTeam {
     mask = (L == 32) ? 0xffffffffu : (((1u << L) - 1u) << (wl & ~(L - 1)));
   }
   __device__ int lane() const { return ln; }
+  __device__ unsigned lanes() const { return kAll ? 0xffffffffu : mask; }
+  // for the bounds of loops that contain team operations: does any team (of the warp, where
+  // they run together) still need a turn, and the most turns that one needs
+  __device__ bool warp_any(bool p) const { return kAll ? __any_sync(0xffffffffu, p) != 0 : any(p); }
+  __device__ int warp_max(int x) const { return kAll ? __reduce_max_sync(0xffffffffu, x) : x; }
   // max value, ties to the smaller index
   __device__ void argmax(float& v, int& i) const {
     if constexpr (L == 32) {
@@ -391,8 +402,8 @@ struct WarpTeam {
     }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
-      const float v2 = __shfl_xor_sync(mask, v, o);
-      const int i2 = __shfl_xor_sync(mask, i, o);
+      const float v2 = __shfl_xor_sync(lanes(), v, o);
+      const int i2 = __shfl_xor_sync(lanes(), i, o);
       if (v2 > v || (v2 == v && i2 < i)) {
         v = v2;
         i = i2;
@@ -414,23 +425,23 @@ struct WarpTeam {
     int i = odd ? ib : ia;
     const float sv = odd ? va : vb;
     const int si = odd ? ia : ib;
-    float v2 = __shfl_xor_sync(mask, sv, 1);
-    int i2 = __shfl_xor_sync(mask, si, 1);
+    float v2 = __shfl_xor_sync(lanes(), sv, 1);
+    int i2 = __shfl_xor_sync(lanes(), si, 1);
     if (v2 > v || (v2 == v && i2 < i)) {
       v = v2;
       i = i2;
     }
 #pragma unroll
     for (int o = 2; o < L; o <<= 1) {
-      v2 = __shfl_xor_sync(mask, v, o);
-      i2 = __shfl_xor_sync(mask, i, o);
+      v2 = __shfl_xor_sync(lanes(), v, o);
+      i2 = __shfl_xor_sync(lanes(), i, o);
       if (v2 > v || (v2 == v && i2 < i)) {
         v = v2;
         i = i2;
       }
     }
-    v2 = __shfl_xor_sync(mask, v, 1);
-    i2 = __shfl_xor_sync(mask, i, 1);
+    v2 = __shfl_xor_sync(lanes(), v, 1);
+    i2 = __shfl_xor_sync(lanes(), i, 1);
     va = odd ? v2 : v;
     ia = odd ? i2 : i;
     vb = odd ? v : v2;
@@ -450,8 +461,8 @@ struct WarpTeam {
     }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
-      const double v2 = __shfl_xor_sync(mask, v, o);
-      const int i2 = __shfl_xor_sync(mask, i, o);
+      const double v2 = __shfl_xor_sync(lanes(), v, o);
+      const int i2 = __shfl_xor_sync(lanes(), i, o);
       if (v2 > v || (v2 == v && i2 < i)) {
         v = v2;
         i = i2;
@@ -462,8 +473,8 @@ struct WarpTeam {
   __device__ void argmax_t(df& v, int& i) const {
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
-      const df v2 = mk_df(__shfl_xor_sync(mask, v.hi, o), __shfl_xor_sync(mask, v.lo, o));
-      const int i2 = __shfl_xor_sync(mask, i, o);
+      const df v2 = mk_df(__shfl_xor_sync(lanes(), v.hi, o), __shfl_xor_sync(lanes(), v.lo, o));
+      const int i2 = __shfl_xor_sync(lanes(), i, o);
       if (v2 > v || (v2 == v && i2 < i)) {
         v = v2;
         i = i2;
@@ -474,9 +485,9 @@ struct WarpTeam {
   __device__ void argmax2(float& b1, int& i1, float& b2) const {
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
-      const float c1 = __shfl_xor_sync(mask, b1, o);
-      const int j1 = __shfl_xor_sync(mask, i1, o);
-      const float c2 = __shfl_xor_sync(mask, b2, o);
+      const float c1 = __shfl_xor_sync(lanes(), b1, o);
+      const int j1 = __shfl_xor_sync(lanes(), i1, o);
+      const float c2 = __shfl_xor_sync(lanes(), b2, o);
       const float lo = fminf(b1, c1);
       if (c1 > b1 || (c1 == b1 && j1 < i1)) {
         b1 = c1;
@@ -496,8 +507,8 @@ struct WarpTeam {
     }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
-      const float v2 = __shfl_xor_sync(mask, v, o);
-      const int i2 = __shfl_xor_sync(mask, i, o);
+      const float v2 = __shfl_xor_sync(lanes(), v, o);
+      const int i2 = __shfl_xor_sync(lanes(), i, o);
       const bool take = (i < 0) ? (i2 >= 0) : (i2 >= 0 && (v2 < v || (v2 == v && i2 < i)));
       if (take) {
         v = v2;
@@ -505,10 +516,10 @@ struct WarpTeam {
       }
     }
   }
-  __device__ bool any(bool p) const { return (__ballot_sync(mask, p) & mask) != 0u; }
+  __device__ bool any(bool p) const { return (__ballot_sync(lanes(), p) & mask) != 0u; }
   // bit l = predicate of team lane l
   __device__ uint32_t ballot(bool p) const {
-    const uint32_t b = __ballot_sync(mask, p);
+    const uint32_t b = __ballot_sync(lanes(), p);
     return L == 32 ? b : (b >> ((threadIdx.x & 31) & ~(L - 1))) & ((1u << L) - 1u);
   }
   // team lanes below this one
@@ -517,25 +528,25 @@ struct WarpTeam {
     int inc = x;
 #pragma unroll
     for (int o = 1; o < L; o <<= 1) {
-      const int y = __shfl_up_sync(mask, inc, o, L);
+      const int y = __shfl_up_sync(lanes(), inc, o, L);
       if (ln >= o) inc += y;
     }
-    total = __shfl_sync(mask, inc, L - 1, L);
+    total = __shfl_sync(lanes(), inc, L - 1, L);
     return inc - x;
   }
   __device__ int imax(int x) const {
     if constexpr (L == 32) return __reduce_max_sync(0xffffffffu, x);
 #pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) x = max(x, __shfl_xor_sync(mask, x, o));
+    for (int o = L / 2; o > 0; o >>= 1) x = max(x, __shfl_xor_sync(lanes(), x, o));
     return x;
   }
   __device__ float fmax_(float x) const {
     if constexpr (L == 32) return order_value(__reduce_max_sync(0xffffffffu, order_key(x)));
 #pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(mask, x, o));
+    for (int o = L / 2; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(lanes(), x, o));
     return x;
   }
-  __device__ void sync() const { __syncwarp(mask); }
+  __device__ void sync() const { __syncwarp(lanes()); }
 };
 #endif
 

@@ -56,6 +56,17 @@ struct FaceSet {
     for (int i = 0; i < W; ++i) n += popc64(w[i]);
     return n;
   }
+  OGX_HD void save(uint32_t* m) const {
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      m[2 * i] = (uint32_t)w[i];
+      m[2 * i + 1] = (uint32_t)(w[i] >> 32);
+    }
+  }
+  OGX_HD void load(const uint32_t* m) {
+#pragma unroll
+    for (int i = 0; i < W; ++i) w[i] = (uint64_t)m[2 * i] | (uint64_t)m[2 * i + 1] << 32;
+  }
   // the k-th face of the set (k < count())
   OGX_HD int nth(int k) const {
     uint64_t m = w[0];
@@ -164,6 +175,7 @@ struct EpaOut {
   bool spill64;    // ... because the FP32 expansion met an inconsistent horizon: the re-run
                    // solves every face plane in FP64
   int resume;      // a capacity spill saved to this EpaResume record (-1: none)
+  bool kept;       // no face was found: the GJK distance and witnesses stay (not set here)
 };
 
 OGX_HD fv3 unit_or_x(fv3 d) {
@@ -367,6 +379,7 @@ OGX_HD bool epa_emit(const Mem& M, const Bodies& B, int f, float tie, EpaOut& o,
   o.w0 = B.point(0, ia.x) * l[0] + B.point(0, ib.x) * l[1] + B.point(0, ic.x) * l[2];
   o.w1 = B.point(1, ia.y) * l[0] + B.point(1, ib.y) * l[1] + B.point(1, ic.y) * l[2];
   const float4 n = M.fn[f];
+  o.kept = false;
   o.nrm = v3<float>(n.x, n.y, n.z);
   o.dist = -n.w;
   o.face[0][0] = ia.x;
@@ -379,6 +392,7 @@ OGX_HD bool epa_emit(const Mem& M, const Bodies& B, int f, float tie, EpaOut& o,
 }
 
 OGX_HD void epa_touch(fv3 a, fv3 b, EpaOut& o) {
+  o.kept = false;
   o.dist = 0.0f;
   o.w0 = a;
   o.w1 = b;
@@ -486,7 +500,7 @@ OGX_HD void epa_save(const Team& t, const Mem& M, const EpaResumeSink& sink, Epa
   o.resume = slot;
 }
 
-// What both capacities start with: the output's defaults, and the GJK simplex grown to a
+// What both capacities start with: the output's flags, and the GJK simplex grown to a
 // tetrahedron (EPA.c:369-583).  False: the pair is finished (separated, or only touching).
 template <class Team, class Bodies>
 OGX_HD bool epa_begin(const Team& t, const Bodies& B, const GjkState& g, EpaOut& o) {
@@ -496,10 +510,7 @@ OGX_HD bool epa_begin(const Team& t, const Bodies& B, const GjkState& g, EpaOut&
   o.spill = false;
   o.spill64 = false;
   o.resume = -1;
-  o.dist = g.dist;
-  o.w0 = g.w0;
-  o.w1 = g.w1;
-  o.nrm = unit_or_x(g.w1 - g.w0);
+  o.kept = true;
   if (g.n != 4 && g.dist > FLT_EPSILON) return false;  // separated (EPA.c:369-373)
   o.status |= OGX_S_EPA_RUN;
   return true;
@@ -608,24 +619,42 @@ OGX_HD float4 set_plane(Mem& M, const Bodies& B, int s, int a, int b, int c, boo
 // itself.  EpaMemCert: no larger capacity; rs: a saved expansion to continue instead of
 // starting from the GJK simplex.  kCert (full capacity only): with FP64 face planes on, run
 // the certified expansion described at kEpaCertGain.
+// The loop state of one expansion (registers that live through the loop: kept few).
+template <class Mem>
+struct EpaRun {
+  int nv, fend, it, st;
+  float scale2, root;  // largest |vertex|^2, and its square root (at convergence: of the last scale)
+  // per-lane closest candidate (slot, plane distance); -1 = none
+  float cbd;
+  int cbest;
+  int best;        // the step's closest face
+  uint32_t flags;  // kRun*: how the loop ended
+  float amax0, amax1;  // the bodies' largest |coordinate| (certified run)
+};
+constexpr uint32_t kRunDone = 1;    // ended, not by the iteration cap
+constexpr uint32_t kRunAgain = 2;   // leaves for the certified run
+constexpr uint32_t kRunThin = 4;    // a thin contact, to be checked
+constexpr uint32_t kRunHalted = 8;  // stopped half way through a step: the faces it retired are in M.hz
+constexpr uint32_t kRunLate = 16;   // capacity spill found after the vertex was added
+
+// The polytope's first faces.  False: the pair is finished already, its result in o.
 template <bool kCert = false, class Team, class Bodies, class Mem>
-OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const GjkState& g, Mem& M, EpaOut& o,
-                     bool can_spill, EpaResumeSink sink = EpaResumeSink{nullptr, nullptr, 0},
-                     const EpaResume* rs = nullptr) {
-  static_assert(Mem::kFull || !kCert, "certified runs need the full capacity");
+OGX_HD bool epa_start(const Team& t, const Bodies& B, const Config& cfg, const GjkState& g, Mem& M, EpaOut& o,
+                      EpaRun<Mem>& r, const EpaResume* rs = nullptr) {
   const int L = Team::L;
   const int lane = t.lane();
   const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
   const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
   const bool cert = kCert && all64;
-  // may the contact be run again with FP64 planes?
-  const bool rerun = !Mem::kFull && can_spill && escalate;
-  if (!epa_begin(t, B, g, o)) return;
-  float scale2 = 0.0f;
-  int st = 0;
-  // per-lane closest candidate (slot, plane distance); -1 = none
-  float cbd = INFINITY;
-  int cbest = -1;
+  if (!epa_begin(t, B, g, o)) return false;
+  float& scale2 = r.scale2;
+  float& cbd = r.cbd;
+  int& cbest = r.cbest;
+  int& st = r.st;
+  scale2 = 0.0f;
+  st = 0;
+  cbd = INFINITY;
+  cbest = -1;
   int nv = 4, fend = 4;
   int it = 0;
   if (Mem::kFull && rs) {
@@ -655,7 +684,7 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
   } else {
     fv3 P[4];
     int IA[4], IB[4];
-    if (!epa_grow(t, B, g, o, P, IA, IB)) return;
+    if (!epa_grow(t, B, g, o, P, IA, IB)) return false;
     // outward faces of a positively oriented tetrahedron (0,1,2,3); swap 1 and 2 otherwise:
     // (0, i2, i1), (0, i1, 3), (i1, i2, 3), (i2, 0, 3).  The face across edge k of face f
     // (edge k = vertices k, k+1 mod 3) and its edge are the same for both orientations:
@@ -691,47 +720,63 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
     }
     t.sync();
   }
-  float root = sqrtf(scale2);  // of scale2
-  int best = -1;
-  bool done = false;
-  bool thin = false;
-  float thin_tol = 0.0f;
-  typename Mem::Faces dead;  // faces retired by a step that stops half way
-  dead.clear();
-  bool again = false;  // leave for the certified run
-  float amax0 = -1.0f, amax1 = -1.0f;  // the bodies' largest |coordinate| (certified run)
-#pragma unroll 1
-  while (it < cfg.epa_max_iter) {
-    ++it;
-    // closest live face
-    float bd = cbd;
-    best = cbest;
-    t.argmin(bd, best);
+  r.nv = nv;
+  r.fend = fend;
+  r.it = it;
+  r.root = sqrtf(scale2);
+  r.best = -1;
+  r.flags = 0u;
+  r.amax0 = r.amax1 = -1.0f;
+  return true;
+}
+
+// One expansion (r.it < the cap).  False: the loop has ended.  live = false: a team that only
+// takes part in the operations of its warp's other teams.
+template <bool kCert = false, class Team, class Bodies, class Mem>
+OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, EpaOut& o, EpaRun<Mem>& r,
+                     bool can_spill, bool live = true) {
+  static_assert(Mem::kFull || !kCert, "certified runs need the full capacity");
+  const int L = Team::L;
+  const int lane = t.lane();
+  const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
+  const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
+  const bool cert = kCert && all64;
+  // may the contact be run again with FP64 planes?
+  const bool rerun = !Mem::kFull && can_spill && escalate;
+  // closest live face
+  float bd = live ? r.cbd : INFINITY;
+  int best = live ? r.cbest : -1;
+  t.argmin(bd, best);
+  if (live) {
+    ++r.it;
+    r.best = best;
     if (best < 0 || !(bd < INFINITY)) {
       o.status |= OGX_S_EPA_TOPOLOGY;
-      best = -1;
-      done = true;
-      break;
+      r.best = -1;
+      r.flags = kRunDone;
+      live = false;
     }
-    int qa, qb;
-    fv3 q;
-    dv3 q64 = v3<double>(0.0, 0.0, 0.0);
-    float qq, scale;  // |q|^2, sqrt(max(scale2, |q|^2))
-    bool conv;
-    float gain = 0.0f, tol = 0.0f;
-    if (kCert && cert) {
-      if constexpr (kCert) {
+  }
+  int qa = 0, qb = 0;
+  fv3 q = v3<float>(0.0f, 0.0f, 0.0f);
+  dv3 q64 = v3<double>(0.0, 0.0, 0.0);
+  float qq = 0.0f, scale = 0.0f;  // |q|^2, sqrt(max(scale2, |q|^2))
+  bool conv = false;
+  float gain = 0.0f, tol = 0.0f;
+  if (kCert && cert) {
+    if constexpr (kCert) {
+      if (live) {
         // exact supports along the closest face's FP64 normal
         const double4 pl = M.fn64[best];
         const dv3 n64 = v3<double>(pl.x, pl.y, pl.z);
         float ea, eb;
-        qa = exact_support<Team, Bodies, double>(t, B, 0, n64, amax0, nullptr, &ea);
-        qb = exact_support<Team, Bodies, double>(t, B, 1, -n64, amax1, nullptr, &eb);
+        qa = exact_support<Team, Bodies, double>(t, B, 0, n64, r.amax0, nullptr, &ea);
+        qb = exact_support<Team, Bodies, double>(t, B, 1, -n64, r.amax1, nullptr, &eb);
         const fv3 pa = B.point(0, qa), pb = B.point(1, qb);
         q = pa - pb;
         q64 = B.dpoint(0, qa) - B.dpoint(1, qb);
         qq = dot(q, q);
-        scale = qq > scale2 ? sqrtf(qq) : root;
+        scale = qq > r.scale2 ? sqrtf(qq) : r.root;
         // The support's gain over the face.  Its FP32 value is within ea + eb (the supports'
         // bounds) and a few roundings of the terms; only a gain nearer the tolerance than that
         // is evaluated in FP64.
@@ -748,203 +793,278 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
           conv = !(ha + hb - pl.w > kEpaCertTol * fmax(1.0, (double)scale));
         }
       }
-    } else {
+    }
+  } else {
+    fv3 n = v3<float>(0.0f, 0.0f, 0.0f);
+    float ba = -INFINITY, bb = -INFINITY;
+    if (live) {
       const float4 nf = M.fn[best];
-      const fv3 n = v3<float>(nf.x, nf.y, nf.z);
-      q = msupport(t, B, n, qa, qb);
+      n = v3<float>(nf.x, nf.y, nf.z);
+      B.scan(t, 0, n, ba, qa);
+      B.scan(t, 1, -n, bb, qb);
+    }
+    t.argmax_pair(ba, qa, bb, qb);
+    if (live) {
+      q = B.point(0, qa) - B.point(1, qb);
       qq = dot(q, q);
-      scale = qq > scale2 ? sqrtf(qq) : root;
+      scale = qq > r.scale2 ? sqrtf(qq) : r.root;
       tol = fmaxf(cfg.epa_tol, cfg.epa_rel * scale);
       gain = dot(n, q) - bd;
       conv = gain < tol;
     }
-    if (conv) {
-      // with room left for an improvement, the certified run decides
-      again = rerun && !all64 && gain > kEpaCertGain * scale;
-      // a thin contact: the FP32 test may have been fooled by the face normal's rounding;
-      // checked after the loop (its FP64 scans would weigh on the loop's registers)
-      thin = rerun && !all64 && !(gain > kEpaCertGain * scale) && bd < kEpaThin * scale;
-      thin_tol = tol;
-      o.status |= OGX_S_EPA_CONVERGED;
-      done = true;
-      break;
-    }
-    bool dup = false;
+  }
+  if (live && conv) {
+    // with room left for an improvement, the certified run decides
+    const bool room = rerun && !all64 && gain > kEpaCertGain * scale;
+    // a thin contact: the FP32 test may have been fooled by the face normal's rounding;
+    // checked after the loop (its FP64 scans would weigh on the loop's registers)
+    const bool thin = rerun && !all64 && !(gain > kEpaCertGain * scale) && bd < kEpaThin * scale;
+    r.flags = kRunDone | (room ? kRunAgain : 0u) | (thin ? kRunThin : 0u);
+    r.root = scale;
+    o.status |= OGX_S_EPA_CONVERGED;
+    live = false;
+  }
+  bool dup = false;
+  if (live) {
 #pragma unroll 1
-    for (int j = lane; j < nv; j += L) {
+    for (int j = lane; j < r.nv; j += L) {
       const int2 id = M.vid[j];
       dup |= (id.x == qa && id.y == qb);
     }
-    if (t.any(dup)) {
-      // the support is already a vertex although the closest face is not converged:
-      // FP32 planes put a vertex in front of a face; re-run certified
-      again = rerun && !all64;
-      o.status |= OGX_S_EPA_DUPLICATE;
-      done = true;
-      break;
-    }
-    if (nv >= Mem::kV) {
-      if (!Mem::kFull && can_spill) {
-        epa_save(t, M, sink, o, nv, fend, it - 1, st, scale2);
-        o.spill = true;
-        return;
-      }
+  }
+  if (t.any(dup)) {
+    // the support is already a vertex although the closest face is not converged:
+    // FP32 planes put a vertex in front of a face; re-run certified
+    r.flags = kRunDone | (rerun && !all64 ? kRunAgain : 0u);
+    o.status |= OGX_S_EPA_DUPLICATE;
+    live = false;
+  }
+  if (live && r.nv >= Mem::kV) {
+    r.flags = kRunDone;
+    if (!Mem::kFull && can_spill)
+      o.spill = true;
+    else
       o.status |= OGX_S_EPA_CAPACITY;
-      done = true;
-      break;
-    }
-    const int p = nv;
+    live = false;
+  }
+  const int p = r.nv;
+  float vis_eps = 0.0f;
+  float cbd = INFINITY;
+  int cbest = -1;
+  if (live) {
     if (lane == 0) {
       M.vp[p] = make_float4_(q.x, q.y, q.z, 0.0f);
       M.vid[p] = make_int2_(qa, qb);
       if constexpr (kCert)
         if (cert) M.vp64[p] = q64;
     }
-    ++nv;
-    scale2 = fmaxf(scale2, qq);
-    root = scale;
-    const float vis_eps = cfg.epa_vis * scale;
+    ++r.nv;
+    r.scale2 = fmaxf(r.scale2, qq);
+    r.root = scale;
+    vis_eps = cfg.epa_vis * scale;
+  }
 
-    // 1. faces seen from q; the closest face that stays
-    cbd = INFINITY;
-    cbest = -1;
-    typename Mem::Faces vis;
-    vis.clear();
+  // 1. faces seen from q; the closest face that stays
+  typename Mem::Faces vis;
+  vis.clear();
+  const int rounds = t.warp_max(live ? r.fend : 0);
 #pragma unroll 1
-    for (int f0 = 0; f0 < fend; f0 += L) {
-      const int f = f0 + lane;
-      float4 fp = make_float4_(0.0f, 0.0f, 0.0f, INFINITY);
-      if (f < fend) fp = M.fn[f];
-      const float h = (fp.x * q.x + fp.y * q.y + fp.z * q.z) - fp.w;
-      bool s = h > vis_eps;
-      if constexpr (kCert) {
-        if (cert) {
-          // the rounded plane and point are within 2e-6 scale of the FP64 height: only
-          // heights nearer zero than that need it
-          s = h > 0.0f;
-          if (f < fend && fabsf(h) <= kEpaVisBand * scale) {
-            const double4 pl = M.fn64[f];
-            s = (pl.x * q64.x + pl.y * q64.y + pl.z * q64.z) - pl.w > kEpaCertVis * (double)scale;
-          }
+  for (int f0 = 0; f0 < rounds; f0 += L) {
+    const int f = f0 + lane;
+    float4 fp = make_float4_(0.0f, 0.0f, 0.0f, INFINITY);
+    if (live && f < r.fend) fp = M.fn[f];
+    const float h = (fp.x * q.x + fp.y * q.y + fp.z * q.z) - fp.w;
+    bool s = h > vis_eps;
+    if constexpr (kCert) {
+      if (cert) {
+        // the rounded plane and point are within 2e-6 scale of the FP64 height: only
+        // heights nearer zero than that need it
+        s = h > 0.0f;
+        if (f < r.fend && fabsf(h) <= kEpaVisBand * scale) {
+          const double4 pl = M.fn64[f];
+          s = (pl.x * q64.x + pl.y * q64.y + pl.z * q64.z) - pl.w > kEpaCertVis * (double)scale;
         }
       }
-      if (!s && fp.w < cbd) {
-        cbd = fp.w;
-        cbest = f;
-      }
-      vis.put(f0, t.ballot(s));
     }
-    // 2. horizon edges: edge e of a visible face whose neighbour is not visible
-    const int nvis = vis.count();
-    int htot = 0;
-#pragma unroll 1
-    for (int i0 = 0; i0 < 3 * nvis; i0 += L) {
-      const int i = i0 + lane;
-      bool h = false;
-      uint32_t edge = 0u;
-      if (i < 3 * nvis) {
-        const int k = (int)(((uint32_t)i * 43691u) >> 17);  // i / 3
-        const int e = i - 3 * k;
-        const int f = vis.nth(k);
-        const uint32_t nb = M.fa[f][e], v = M.fv[f];
-        h = !vis.has((int)(nb & 0xffu));
-        edge = ((v >> (8 * e)) & 0xffu) | ((v >> (e == 2 ? 0 : 8 * e + 8)) & 0xffu) << 8 | (nb & 0xffu) << 16 |
-               (nb >> 8) << 24;
-      }
-      const uint32_t m = t.ballot(h);
-      const int r = htot + popc32(m & t.below());
-      if (h && r < Mem::kF) M.hz[r] = edge;
-      htot += popc32(m);
+    if (!s && fp.w < cbd) {
+      cbd = fp.w;
+      cbest = f;
     }
-    // the closest face must be seen (gain >= tol > vis threshold) and have a horizon;
-    // otherwise stop, or start again with FP64 planes in the full pass
-    if (!vis.has(best) || htot < 3) {
-      again = rerun;
-      o.status |= OGX_S_EPA_TOPOLOGY;
-      done = true;
-      break;
-    }
-    // new face k goes to the k-th visible slot, else to fresh slot fend + k - nvis
-    const int fresh = htot > nvis ? htot - nvis : 0;
-    if (fend + fresh > Mem::kF) {
-      if (!Mem::kFull && can_spill) {
-        epa_save(t, M, sink, o, nv - 1, fend, it - 1, st, scale2);  // before q was added
-        o.spill = true;
-        return;
-      }
-      o.status |= OGX_S_EPA_CAPACITY;
-      done = true;
-      break;
-    }
-    t.sync();
-    // 3. relink the faces outside the horizon, index the horizon by its vertices
-#pragma unroll 1
-    for (int k = lane; k < htot; k += L) {
-      const int s = k < nvis ? vis.nth(k) : fend + k - nvis;
-      const uint32_t h = M.hz[k];
-      M.fa[(h >> 16) & 0xffu][h >> 24] = (uint16_t)s;
-      M.hstart[h & 0xffu] = (uint8_t)s;
-      M.hend[(h >> 8) & 0xffu] = (uint8_t)s;
-    }
-    t.sync();
-    // a vertex that starts (or ends) two horizon edges means the horizon is not one
-    // simple loop; keep the closest face found this step and stop
-    bool bad = false;
-#pragma unroll 1
-    for (int k = lane; k < htot; k += L) {
-      const int s = k < nvis ? vis.nth(k) : fend + k - nvis;
-      const uint32_t h = M.hz[k];
-      bad |= (M.hstart[h & 0xffu] != s) || (M.hend[(h >> 8) & 0xffu] != s);
-    }
-    if (t.any(bad)) {
-      again = rerun;
-      o.status |= OGX_S_EPA_TOPOLOGY;
-      dead = vis;
-      done = true;
-      break;
-    }
-    // 4. new face (a, b, p) across each horizon edge a->b
-#pragma unroll 1
-    for (int k = lane; k < htot; k += L) {
-      const int s = k < nvis ? vis.nth(k) : fend + k - nvis;
-      const uint32_t h = M.hz[k];
-      const int a = (int)(h & 0xffu), b = (int)((h >> 8) & 0xffu);
-      M.fv[s] = (h & 0xffffu) | (uint32_t)p << 16;
-      M.fa[s][0] = (uint16_t)((h >> 16 & 0xffu) | (h >> 24) << 8);
-      M.fa[s][1] = (uint16_t)(M.hstart[b] | 2u << 8);
-      M.fa[s][2] = (uint16_t)(M.hend[a] | 1u << 8);
-      const float4 pl = set_plane<kCert>(M, B, s, a, b, p, escalate, all64, cert, st);
-      if (pl.w < cbd || (pl.w == cbd && s < cbest)) {
-        cbd = pl.w;
-        cbest = s;
-      }
-    }
-#pragma unroll 1
-    for (int k = htot + lane; k < nvis; k += L) {
-      const int s = vis.nth(k);
-      M.fn[s] = make_float4_(0.0f, 0.0f, 0.0f, INFINITY);
-    }
-    fend += fresh;
-    t.sync();
+    vis.put(f0, t.ballot(s));
   }
+  // 2. horizon edges: edge e of a visible face whose neighbour is not visible
+  const int nvis = vis.count();
+  int htot = 0;
+  const int edges = t.warp_max(3 * nvis);
+#pragma unroll 1
+  for (int i0 = 0; i0 < edges; i0 += L) {
+    const int i = i0 + lane;
+    bool h = false;
+    uint32_t edge = 0u;
+    if (i < 3 * nvis) {
+      const int k = (int)(((uint32_t)i * 43691u) >> 17);  // i / 3
+      const int e = i - 3 * k;
+      const int f = vis.nth(k);
+      const uint32_t nb = M.fa[f][e], v = M.fv[f];
+      h = !vis.has((int)(nb & 0xffu));
+      edge = ((v >> (8 * e)) & 0xffu) | ((v >> (e == 2 ? 0 : 8 * e + 8)) & 0xffu) << 8 | (nb & 0xffu) << 16 |
+             (nb >> 8) << 24;
+    }
+    const uint32_t m = t.ballot(h);
+    const int k = htot + popc32(m & t.below());
+    if (h && k < Mem::kF) M.hz[k] = edge;
+    htot += popc32(m);
+  }
+  // new face k goes to the k-th visible slot, else to fresh slot fend + k - nvis
+  const int fresh = htot > nvis ? htot - nvis : 0;
+  if (live) {
+    if (!vis.has(best) || htot < 3) {
+      // the closest face must be seen (gain >= tol > vis threshold) and have a horizon;
+      // otherwise stop, or start again with FP64 planes in the full pass
+      r.flags = kRunDone | (rerun ? kRunAgain : 0u);
+      o.status |= OGX_S_EPA_TOPOLOGY;
+      live = false;
+    } else if (r.fend + fresh > Mem::kF) {
+      r.flags = kRunDone | kRunLate;
+      if (!Mem::kFull && can_spill)
+        o.spill = true;
+      else
+        o.status |= OGX_S_EPA_CAPACITY;
+      live = false;
+    }
+  }
+  if (!live) htot = 0;
+  t.sync();
+  // 3. relink the faces outside the horizon, index the horizon by its vertices.  The lane's
+  // first edge stays in registers; only a horizon longer than the team is wide loops.
+  auto slot_of = [&](int k) { return k < nvis ? vis.nth(k) : r.fend + k - nvis; };
+  auto relink = [&](uint32_t h, int s) {
+    M.fa[(h >> 16) & 0xffu][h >> 24] = (uint16_t)s;
+    M.hstart[h & 0xffu] = (uint8_t)s;
+    M.hend[(h >> 8) & 0xffu] = (uint8_t)s;
+  };
+  uint32_t h0 = 0u;
+  int s0 = 0;
+  if (lane < htot) {
+    h0 = M.hz[lane];
+    s0 = slot_of(lane);
+    relink(h0, s0);
+  }
+#pragma unroll 1
+  for (int k = lane + L; k < htot; k += L) relink(M.hz[k], slot_of(k));
+  t.sync();
+  // a vertex that starts (or ends) two horizon edges means the horizon is not one
+  // simple loop; keep the closest face found this step and stop
+  const int a0 = (int)(h0 & 0xffu), b0 = (int)((h0 >> 8) & 0xffu);
+  bool bad = false;
+  int link1 = 0, link2 = 0;  // the new faces across the new face's edges b-p and p-a
+  if (lane < htot) {
+    bad = M.hstart[a0] != s0 || M.hend[b0] != s0;
+    link1 = M.hstart[b0];
+    link2 = M.hend[a0];
+  }
+#pragma unroll 1
+  for (int k = lane + L; k < htot; k += L) {
+    const int s = slot_of(k);
+    const uint32_t h = M.hz[k];
+    bad |= (M.hstart[h & 0xffu] != s) || (M.hend[(h >> 8) & 0xffu] != s);
+  }
+  if (t.any(bad)) {
+    r.flags = kRunDone | kRunHalted | (rerun ? kRunAgain : 0u);
+    o.status |= OGX_S_EPA_TOPOLOGY;
+    if (lane == 0) vis.save(M.hz);
+    live = false;
+    htot = 0;
+  }
+  // 4. new face (a, b, p) across each horizon edge a->b
+#pragma unroll 1
+  for (int k = lane; k < htot; k += L) {
+    if (k >= L) {
+      s0 = slot_of(k);
+      h0 = M.hz[k];
+      link1 = M.hstart[(h0 >> 8) & 0xffu];
+      link2 = M.hend[h0 & 0xffu];
+    }
+    M.fv[s0] = (h0 & 0xffffu) | (uint32_t)p << 16;
+    M.fa[s0][0] = (uint16_t)((h0 >> 16 & 0xffu) | (h0 >> 24) << 8);
+    M.fa[s0][1] = (uint16_t)(link1 | 2u << 8);
+    M.fa[s0][2] = (uint16_t)(link2 | 1u << 8);
+    const float4 pl = set_plane<kCert>(M, B, s0, (int)(h0 & 0xffu), (int)((h0 >> 8) & 0xffu), p, escalate, all64,
+                                       cert, r.st);
+    if (pl.w < cbd || (pl.w == cbd && s0 < cbest)) {
+      cbd = pl.w;
+      cbest = s0;
+    }
+  }
+  if (live) {
+#pragma unroll 1
+    for (int k = htot + lane; k < nvis; k += L) M.fn[vis.nth(k)] = make_float4_(0.0f, 0.0f, 0.0f, INFINITY);
+    r.fend += fresh;
+    r.cbd = cbd;
+    r.cbest = cbest;
+  }
+  t.sync();
+  return live;
+}
+
+// The result once the loop has ended; a capacity spill (o.spill, at the top of its last
+// expansion) saves itself.
+template <bool kCert = false, class Team, class Bodies, class Mem>
+OGX_HD void epa_finish(const Team& t, const Bodies& B, const Config& cfg, Mem& M, EpaOut& o, const EpaRun<Mem>& r,
+                       bool can_spill, const EpaResumeSink& sink) {
+  if (o.spill) {
+    // the polytope as it was at the top of the last expansion
+    if constexpr (!Mem::kFull)
+      epa_save(t, M, sink, o, r.flags & kRunLate ? r.nv - 1 : r.nv, r.fend, r.it - 1, r.st, r.scale2);
+    return;
+  }
+  const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
+  const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
+  const bool cert = kCert && all64;
+  const bool rerun = !Mem::kFull && can_spill && escalate;
+  bool again = (r.flags & kRunAgain) != 0u;
   if (!again) {
-    o.iters = it;
-    o.status |= st ? OGX_S_EPA_ESCALATED : 0;
+    o.iters = r.it;
+    o.status |= r.st ? OGX_S_EPA_ESCALATED : 0;
     o.status |= cert ? OGX_S_EPA_CERTIFIED : 0;
-    if (!done) {
+    int best = r.best;
+    if (!(r.flags & kRunDone)) {
       // iteration cap: closest current face
-      float bd = cbd;
-      best = cbest;
+      float bd = r.cbd;
+      best = r.cbest;
       t.argmin(bd, best);
       o.status |= OGX_S_EPA_CAP;
     }
-    if (!Mem::kFull && thin && best >= 0) again = thin_gain_exceeds(t, B, M, best, thin_tol);
+    if (!Mem::kFull && (r.flags & kRunThin) && best >= 0)
+      again = thin_gain_exceeds(t, B, M, best, fmaxf(cfg.epa_tol, cfg.epa_rel * r.root));
     if (!again && best >= 0) {
-      again = epa_emit(M, B, best, fmaxf(cfg.epa_tol, cfg.epa_rel * sqrtf(scale2)), o, rerun && !all64, dead);
+      typename Mem::Faces dead;
+      dead.clear();
+      if (r.flags & kRunHalted) dead.load(M.hz);
+      again = epa_emit(M, B, best, fmaxf(cfg.epa_tol, cfg.epa_rel * sqrtf(r.scale2)), o, rerun && !all64, dead);
       o.polish = !again && (cfg.flags & OGX_F_FP64_POLISH) != 0;
     }
   }
   o.spill = o.spill64 = again;
+}
+
+template <bool kCert = false, class Team, class Bodies, class Mem>
+OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const GjkState& g, Mem& M, EpaOut& o,
+                     bool can_spill, EpaResumeSink sink = EpaResumeSink{nullptr, nullptr, 0},
+                     const EpaResume* rs = nullptr) {
+  EpaRun<Mem> r;
+  if (epa_start<kCert>(t, B, cfg, g, M, o, r, rs)) {
+#pragma unroll 1
+    while (r.it < cfg.epa_max_iter && epa_step<kCert>(t, B, cfg, M, o, r, can_spill)) {
+    }
+    epa_finish<kCert>(t, B, cfg, M, o, r, can_spill, sink);
+  }
+  if (o.kept) {
+    o.dist = g.dist;
+    o.w0 = g.w0;
+    o.w1 = g.w1;
+    o.nrm = unit_or_x(g.w1 - g.w0);
+  }
 }
 
 }  // namespace ogx

@@ -307,7 +307,8 @@ OGX_HD int escalate_step(const Mem B, int n, const int* ia, const int* ib, fv3 v
 
 // GJK as a loop of iterations: gjk_start sets the state up, each gjk_iterate runs one
 // iteration (support, termination tests, sub-distance step) until r.done, gjk_end
-// finishes (witnesses, certification).  gjk_pair chains them.
+// finishes (witnesses, certification).  gjk_pair chains them.  live = false: a team that only
+// takes part in the operations of its warp's other teams.
 struct GjkRun {
   fv3 v;
   float vv;  // dot(v, v)
@@ -361,7 +362,7 @@ OGX_COLD float gap_floor(const Config cfg, float vv, float ww) {
 // older points were counted when they joined); one branch for all the exit tests.
 template <class Team, class Bodies>
 OGX_HD void gjk_iterate(const Team& t, const Bodies& B, const Config& cfg, GjkRun& r,
-                        const uint32_t* subtab = nullptr) {
+                        const uint32_t* subtab = nullptr, bool live = true) {
   const bool reftol = (cfg.flags & OGX_F_REFERENCE_TOL) != 0;
   const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
   // |v| this small against the simplex points is below FP32 resolution: stop
@@ -370,13 +371,16 @@ OGX_HD void gjk_iterate(const Team& t, const Bodies& B, const Config& cfg, GjkRu
   fv3* P = r.P;
   int* IA = r.IA;
   int* IB = r.IB;
-  ++r.k;
   const fv3 mv = -v;
-  float ba, bb;
-  int xa, xb;
-  B.scan(t, 0, mv, ba, xa);
-  B.scan(t, 1, v, bb, xb);
+  float ba = -INFINITY, bb = -INFINITY;
+  int xa = 0, xb = 0;
+  if (live) {
+    B.scan(t, 0, mv, ba, xa);
+    B.scan(t, 1, v, bb, xb);
+  }
   t.argmax_pair(ba, xa, bb, xb);
+  if (!live) return;
+  ++r.k;
   // the candidates (a scan that no value won has no index: the last support then)
   const fv3 pa = B.point(0, ba > -INFINITY ? xa : r.ia), pb = B.point(1, bb > -INFINITY ? xb : r.ib);
   if (ba > sdot(r.sa, mv)) {

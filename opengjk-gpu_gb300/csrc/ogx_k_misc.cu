@@ -242,12 +242,25 @@ __global__ void __launch_bounds__(128, 3) k_refine_cont(DevBatch B) {
     continue_list<8, kPosed>(B, small, B.refine_full, 1, warp - split, nwarps - split);
 }
 
+// The bucket kernels' contacts, list after list, each with the record at its pair's index
 template <bool kPosed>
 __global__ void __launch_bounds__(128) k_polish(DevBatch B) {
-  const int cnt = B.counts[kCntPolish];
+  int first[kBuckets + 1];
+  first[0] = 0;
+#pragma unroll
+  for (int b = 0; b < kBuckets; ++b) first[b + 1] = first[b] + B.counts[kCntEpa + b];
+  const int cnt = first[kBuckets];
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
-    const PolishRec r = B.polish[k];
-    const int p = r.pair;
+    int b = 0, f = 0;
+#pragma unroll
+    for (int q = 1; q < kBuckets; ++q)
+      if (k >= first[q]) {
+        b = q;
+        f = first[q];
+      }
+    const int p = B.elists[(size_t)b * B.npairs + (k - f)];
+    const PolishRec r = B.polish[p];
+    if (r.kind != 1) continue;
     const int2 pr = B.pairs[p];
     typename PoseOf<kPosed, MemBodies>::type mb;
     bind_mem(mb, B, pr, B.bodies[pr.x], B.bodies[pr.y]);

@@ -37,7 +37,8 @@ struct RefineRec {
   int certain;
 };
 
-// FP64 re-solve request: GJK simplex (kind 0) or the final EPA face (kind 1)
+// re-solve request of a contact, at its pair's index: none (kind 0), or the final EPA face
+// (kind 1)
 struct PolishRec {
   int pair;
   int kind;
@@ -219,6 +220,23 @@ __device__ __forceinline__ const float* pose_of(const DevBatch& B, int i) {
   return kPosed ? B.xf + 12 * (size_t)i : nullptr;
 }
 
+// A team's next pair, loaded one pair ahead: the chain list -> pair -> bodies is three
+// dependent loads, which otherwise start every pair.
+struct NextPair {
+  int p;
+  int2 pr;
+  BodyRef ra, rb;
+  __device__ __forceinline__ void load(const DevBatch& B, const int* list, int j, int cnt) {
+    p = -1;
+    if (j < cnt) {
+      p = list[j];
+      pr = B.pairs[p];
+      ra = B.bodies[pr.x];
+      rb = B.bodies[pr.y];
+    }
+  }
+};
+
 // Store one finished pair's GJK result and route it (EPA list, FP64 refinement list).
 __device__ __forceinline__ void gjk_store(const DevBatch& B, int bucket, int p, const GjkState& g, bool lead) {
   const bool contact = gjk_contact(g);
@@ -229,24 +247,40 @@ __device__ __forceinline__ void gjk_store(const DevBatch& B, int bucket, int p, 
     if (B.mode == kModeGjkEpa && !contact && !g.polish) store3(B.nrm + 3 * (size_t)p, sep_normal(g));
     // pairs sent to the FP64 refinement get their normal there
   }
+  // The lists' slots: one atomic per list for the converged lanes, all three on their way
+  // before the first is waited for.  Certified pairs are re-solved; the uncertain ones go to
+  // the FP64 continuation's lists.
   const bool to_epa = lead && B.mode == kModeGjkEpa && contact;
-  const int e = warp_append(B.counts + kCntEpa + bucket, to_epa);
-  if (to_epa) B.elists[(size_t)bucket * B.npairs + e] = p;
-  const bool refine = lead && g.polish;
-  const int q = warp_append(B.counts + kCntRefine, refine && g.certain);
-  if (refine && g.certain) {
-    RefineRec r;
-    r.pair = p;
-    r.wa = g.wa;
-    r.wb = g.wb;
-    r.certain = 1;
-    B.refine[q] = r;
-  }
-  // the others go to the FP64 continuation's lists at once, so that it need not wait for
-  // the pass over the certain ones
+  const bool certain = lead && g.polish && g.certain, uncertain = lead && g.polish && !g.certain;
   const bool small = bucket_max(bucket) <= kRefineLaneMax;
-  const int u = warp_append(B.counts + (small ? kCntRefineFull : kCntRefineBig), refine && !g.certain);
-  if (refine && !g.certain) B.refine_full[small ? u : B.npairs - 1 - u] = p;
+  const unsigned act = __activemask();
+  const unsigned me = __ballot_sync(act, to_epa), mc = __ballot_sync(act, certain), mu = __ballot_sync(act, uncertain);
+  const int wl = threadIdx.x & 31;
+  const unsigned below = (1u << wl) - 1u;
+  int be = 0, bc = 0, bu = 0;
+  if (me && wl == __ffs(me) - 1) be = atomicAdd(B.counts + kCntEpa + bucket, __popc(me));
+  if (mc && wl == __ffs(mc) - 1) bc = atomicAdd(B.counts + kCntRefine, __popc(mc));
+  if (mu && wl == __ffs(mu) - 1) bu = atomicAdd(B.counts + (small ? kCntRefineFull : kCntRefineBig), __popc(mu));
+  if (me) {
+    be = __shfl_sync(act, be, __ffs(me) - 1);
+    if (to_epa) B.elists[(size_t)bucket * B.npairs + be + __popc(me & below)] = p;
+  }
+  if (mc) {
+    bc = __shfl_sync(act, bc, __ffs(mc) - 1);
+    if (certain) {
+      RefineRec r;
+      r.pair = p;
+      r.wa = g.wa;
+      r.wb = g.wb;
+      r.certain = 1;
+      B.refine[bc + __popc(mc & below)] = r;
+    }
+  }
+  if (mu) {
+    bu = __shfl_sync(act, bu, __ffs(mu) - 1);
+    const int u = bu + __popc(mu & below);
+    if (uncertain) B.refine_full[small ? u : B.npairs - 1 - u] = p;
+  }
 }
 
 template <int L, int K, int OCC = 1, int D = 0, bool kPosed = false>
@@ -254,24 +288,38 @@ __global__ void __launch_bounds__(kStageStride, OCC) k_gjk(DevBatch B, int bucke
   extern __shared__ __align__(16) unsigned char smem_raw[];  // staging slots (D > 0)
   float4* slots = reinterpret_cast<float4*>(smem_raw) + threadIdx.x;
   const WarpTeam<L> t;
+  const WarpTeam<L, true> all;  // the iterations, by all teams of the warp together
   const int team = (blockIdx.x * blockDim.x + threadIdx.x) / L;
   const int nteams = (gridDim.x * blockDim.x) / L;
   const int cnt = B.counts[kCntGjk + bucket];
   const int* list = B.lists + (size_t)bucket * B.npairs;
-  for (int j = team; j < cnt; j += nteams) {
-    const int p = list[j];
-    const int2 pr = B.pairs[p];
-    const BodyRef ra = B.bodies[pr.x], rb = B.bodies[pr.y];
+  NextPair next;
+  next.load(B, list, team, cnt);
+#pragma unroll 1
+  for (int j = team; all.warp_any(j < cnt); j += nteams) {
+    const bool have = j < cnt;
     typename PoseOf<kPosed, typename GjkSrcOf<L, K, D>::type>::type src;
-    bind_src<L>(src, B.pool, ra, rb, t.lane(), slots, pose_of<kPosed>(B, pr.x), pose_of<kPosed>(B, pr.y));
-    int2 ws = make_int2(0, 0);
-    if (B.warm) {
-      ws = B.warm[p];
-      if (ws.x < 0 || ws.x >= ra.n || ws.y < 0 || ws.y >= rb.n) ws = make_int2(0, 0);
+    GjkRun r;
+    const int p = next.p;
+    r.done = true;
+    if (have) {
+      bind_src<L>(src, B.pool, next.ra, next.rb, t.lane(), slots, pose_of<kPosed>(B, next.pr.x),
+                  pose_of<kPosed>(B, next.pr.y));
+      int2 ws = make_int2(0, 0);
+      if (B.warm) {
+        ws = B.warm[p];
+        if (ws.x < 0 || ws.x >= next.ra.n || ws.y < 0 || ws.y >= next.rb.n) ws = make_int2(0, 0);
+      }
+      gjk_start(src, r, ws.x, ws.y);
     }
-    GjkState g;
-    gjk_pair(t, src, B.cfg, g, ws.x, ws.y, B.subtab);
-    gjk_store(B, bucket, p, g, t.lane() == 0);
+#pragma unroll 1
+    while (all.warp_any(!r.done)) gjk_iterate(all, src, B.cfg, r, B.subtab, !r.done);
+    next.load(B, list, j + nteams, cnt);  // on its way while this pair is finished
+    if (have) {
+      GjkState g;
+      gjk_end(t, src, B.cfg, r, g);
+      gjk_store(B, bucket, p, g, t.lane() == 0);
+    }
   }
   if constexpr (D > 0) cp_async_wait<0>();  // no copy outlives the block
 }
@@ -284,6 +332,60 @@ __global__ void __launch_bounds__(kStageStride, OCC) k_gjk(DevBatch B, int bucke
 constexpr int kSpill64 = 1 << 30;      // the re-run solves every face plane in FP64
 constexpr int kSpillResume = 1 << 29;  // low bits: the EpaResume record to continue
 
+__device__ __forceinline__ int status_so_far(const DevBatch& B, int p) {
+  return B.status && B.mode != kModeEpa ? B.status[p] : 0;
+}
+
+// Stores a contact's result, or (false) its spill list code.
+// before: the pair's status so far (0 for EPA-only calls)
+template <bool kFull, class Team, class Src>
+__device__ __forceinline__ bool epa_store(const Team& t, const DevBatch& B, int p, int before, const Src& src,
+                                          EpaOut& o, int* spill_code) {
+  const bool lead = t.lane() == 0;
+  if (o.spill) {
+    if (o.resume >= 0 && lead) B.resume[o.resume].pair = p;
+    if (lead && !kFull) B.polish[p].kind = 0;  // the full pass polishes its own
+    if (spill_code) *spill_code = o.resume >= 0 ? (kSpillResume | o.resume) : (p | (o.spill64 ? kSpill64 : 0));
+    return false;
+  }
+  if (kFull && lead && o.polish) {
+    epa_polish(src, o);
+    o.polish = false;
+  }
+  if (lead && o.kept) {
+    const gkSimplex& s = B.smp[p];
+    store3(B.nrm + 3 * (size_t)p, unit_or_x(v3<float>(s.witnesses[1][0] - s.witnesses[0][0],
+                                                      s.witnesses[1][1] - s.witnesses[0][1],
+                                                      s.witnesses[1][2] - s.witnesses[0][2])));
+    if (B.status) B.status[p] = before | o.status;
+  } else if (lead) {
+    B.dist[p] = o.dist;
+    gkSimplex* s = B.smp + p;
+    s->witnesses[0][0] = o.w0.x;
+    s->witnesses[0][1] = o.w0.y;
+    s->witnesses[0][2] = o.w0.z;
+    s->witnesses[1][0] = o.w1.x;
+    s->witnesses[1][1] = o.w1.y;
+    s->witnesses[1][2] = o.w1.z;
+    store3(B.nrm + 3 * (size_t)p, o.nrm);
+    if (B.status) B.status[p] = before | o.status;
+  }
+  if (lead && o.polish) {
+    PolishRec r;
+    r.pair = p;
+    r.kind = 1;
+    for (int k = 0; k < 3; ++k) {
+      r.face[k][0] = o.face[k][0];
+      r.face[k][1] = o.face[k][1];
+    }
+    B.polish[p] = r;
+    atomicAdd(B.counts + kCntPolish, 1);  // (a count only: nothing waits for its value)
+  } else if (lead && !kFull) {
+    B.polish[p].kind = 0;
+  }
+  return true;
+}
+
 template <int L, int K, bool kFull = false, int D = 0, bool kPosed = false, class Mem>
 __device__ __forceinline__ bool epa_item(const WarpTeam<L>& t, const DevBatch& B, const Config& cfg, int p,
                                          Mem& M, bool can_spill, int* spill_code = nullptr,
@@ -295,42 +397,10 @@ __device__ __forceinline__ bool epa_item(const WarpTeam<L>& t, const DevBatch& B
   GjkState g;
   load_simplex(B.smp + p, B.dist[p], g);
   EpaOut o;
+  const int before = status_so_far(B, p);
   const EpaResumeSink sink{can_spill ? B.resume : nullptr, B.counts + kCntResume, B.resume_cap};
   epa_pair<kFull>(t, src, cfg, g, M, o, can_spill, sink, rs);
-  if (o.spill) {
-    if (o.resume >= 0 && t.lane() == 0) B.resume[o.resume].pair = p;
-    if (spill_code) *spill_code = o.resume >= 0 ? (kSpillResume | o.resume) : (p | (o.spill64 ? kSpill64 : 0));
-    return false;
-  }
-  const bool lead = t.lane() == 0;
-  if (kFull && lead && o.polish) {
-    epa_polish(src, o);
-    o.polish = false;
-  }
-  if (lead) {
-    B.dist[p] = o.dist;
-    gkSimplex* s = B.smp + p;
-    s->witnesses[0][0] = o.w0.x;
-    s->witnesses[0][1] = o.w0.y;
-    s->witnesses[0][2] = o.w0.z;
-    s->witnesses[1][0] = o.w1.x;
-    s->witnesses[1][1] = o.w1.y;
-    s->witnesses[1][2] = o.w1.z;
-    store3(B.nrm + 3 * (size_t)p, o.nrm);
-    if (B.status) B.status[p] = (B.mode == kModeEpa ? 0 : B.status[p]) | o.status;
-  }
-  const int q = warp_append(B.counts + kCntPolish, lead && o.polish);
-  if (lead && o.polish) {
-    PolishRec r;
-    r.pair = p;
-    r.kind = 1;
-    for (int k = 0; k < 3; ++k) {
-      r.face[k][0] = o.face[k][0];
-      r.face[k][1] = o.face[k][1];
-    }
-    B.polish[q] = r;
-  }
-  return true;
+  return epa_store<kFull>(t, B, p, before, src, o, spill_code);
 }
 
 // EPA over one bucket's contacts with the small working set (EpaMemSmall per team in
@@ -359,14 +429,44 @@ __global__ void __launch_bounds__(kStageStride, OCC) k_epa(DevBatch B, int bucke
   const int nteams = (gridDim.x * blockDim.x) / L;
   const int cnt = B.counts[kCntEpa + bucket];
   const int* list = B.elists + (size_t)bucket * B.npairs;
-  for (int j = team; j < cnt; j += nteams) {
-    const int p = list[j];
-    int code = 0;
-    const bool ok = epa_item<L, K, false, D, kPosed>(t, B, B.cfg, p, M, true, &code, nullptr, slots);
-    const bool lead = t.lane() == 0;
-    const int q = warp_append(B.counts + kCntSpill, lead && !ok);
-    if (lead && !ok) B.spill[q] = code;
-    t.sync();  // the next pair reuses M
+  const WarpTeam<L, true> all;  // the expansions, by all teams of the warp together
+  const EpaResumeSink sink{B.resume, B.counts + kCntResume, B.resume_cap};
+  NextPair next;
+  next.load(B, list, team, cnt);
+#pragma unroll 1
+  for (int j = team; all.warp_any(j < cnt); j += nteams) {
+    typename PoseOf<kPosed, typename SrcOf<L, K, D>::type>::type src;
+    EpaRun<EpaMemSmall> r;
+    EpaOut o;
+    const int p = next.p;
+    bool run = false;
+    if (j < cnt) {
+      bind_src<L>(src, B.pool, next.ra, next.rb, t.lane(), slots, pose_of<kPosed>(B, next.pr.x),
+                  pose_of<kPosed>(B, next.pr.y));
+      GjkState g;
+      load_simplex(B.smp + p, B.dist[p], g);
+      run = epa_start(t, src, B.cfg, g, M, o, r);
+      if (!run) epa_store<false>(t, B, p, status_so_far(B, p), src, o, nullptr);  // touching
+    }
+    const bool loop = run;
+#pragma unroll 1
+    while (all.warp_any(run)) {
+      run = epa_step(all, src, B.cfg, M, o, r, true, run);
+      run = run && r.it < B.cfg.epa_max_iter;
+    }
+    // (on their way while this contact's face is worked out; not through the loop, whose
+    // registers they would take)
+    next.load(B, list, j + nteams, cnt);
+    if (loop) {
+      const int before = status_so_far(B, p);
+      epa_finish(t, src, B.cfg, M, o, r, true, sink);
+      int code = 0;
+      const bool ok = epa_store<false>(t, B, p, before, src, o, &code);
+      const bool lead = t.lane() == 0;
+      const int q = warp_append(B.counts + kCntSpill, lead && !ok);
+      if (lead && !ok) B.spill[q] = code;
+    }
+    all.sync();  // the next contact reuses M
   }
   if constexpr (D > 0) cp_async_wait<0>();  // no copy outlives the block
 }
