@@ -865,7 +865,7 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
     if (mode != kModeGjk) {
       // the contacts the refinement found (usually none), after it on the same stream
       ctx->mark("epa_late");
-      e = launch_epa_spill(B, fit_grid(g_grid_spill, std::max(1, npairs / 256), 32), rst, true);
+      e = launch_epa_spill(B, fit_grid(g_grid_spill, npairs, 32), rst, true);
       if (e != cudaSuccess) return ogx_cuda_fail(e, "k_epa_spill launch");
       stage("epa_late", rst);
       ++launches;
