@@ -248,7 +248,7 @@ ogx_status init_kernels(int device) {
   g_grid_refine = std::max(1, per_sm) * sms;
   e = continue_occupancy(kBlock, &per_sm);
   if (e != cudaSuccess) return ogx_cuda_fail(e, "occupancy(k_refine_cont)");
-  g_grid_cont = std::min(2, std::max(1, per_sm)) * sms;
+  g_grid_cont = std::max(1, per_sm) * sms;
   {
     std::vector<uint32_t> tab(kSubTabSize);
     fill_subtab(tab.data());

@@ -227,15 +227,21 @@ __device__ __forceinline__ void continue_list(const DevBatch& B, int cnt, const 
   }
 }
 
-// the first half of the blocks take the larger bodies' list (filled from the end of
-// refine_full), the others the small ones', each list over the whole grid when the other
-// is empty
+// Each list gets a share of the warps by its work: a larger body's continuation (refine_full
+// filled from its end, a whole warp scans) counts as kBigCost small ones (four scanned at a
+// time).  Both halves of the split at 1:1, 2 blocks per SM -> this split, 3 blocks per SM (what
+// 168 registers allow): 30k stress pairs (3,289 large and 13,814 small) 930 -> 852 us, 200k
+// scene pairs (14,680 and 3,128) 1,018 -> 1,010, 1M power-law pairs 5,225 -> 5,190; weighted 8,
+// 915 / 1,065 / 5,255.  More blocks at fewer registers spill and gain nothing more.
+constexpr int kBigCost = 2;
 template <bool kPosed>
 __global__ void __launch_bounds__(128, 3) k_refine_cont(DevBatch B) {
   const int big = B.counts[kCntRefineBig], small = B.counts[kCntRefineFull];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int split = small == 0 ? nwarps : (big == 0 ? 0 : nwarps / 2);
+  const int64_t cost = (int64_t)kBigCost * big;
+  int split = big == 0 ? 0 : (int)(nwarps * cost / (cost + small));
+  if (big > 0 && small > 0) split = min(max(split, 1), nwarps - 1);
   if (warp < split)
     continue_list<32, kPosed>(B, big, B.refine_full + (B.npairs - 1), -1, warp, split);
   else

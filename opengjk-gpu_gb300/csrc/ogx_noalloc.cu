@@ -120,7 +120,7 @@ ogx_status setup(int dev, Setup** out) {
   s.grid_refine = std::max(1, per) * sms;
   e = continue_occupancy(kNoAllocBlock, &per);
   if (e != cudaSuccess) return ogx_cuda_fail(e, "occupancy");
-  s.grid_cont = std::min(2, std::max(1, per)) * sms;
+  s.grid_cont = std::max(1, per) * sms;
   e = epa_spill_occupancy(kNoAllocBlock, &per);
   if (e != cudaSuccess) return ogx_cuda_fail(e, "occupancy");
   s.grid_spill = std::max(1, per) * sms;
