@@ -229,7 +229,7 @@ struct Compat {
   size_t nrm_cap = 0;
   double* d_c64 = nullptr;  // the *_f64 calls: the bodies' double coordinates, pool order
   size_t c64_cap = 0;
-  const float** d_src = nullptr;  // per body: the caller's coordinate pointer (k_pack_ptrs)
+  const void** d_src = nullptr;  // per body: the caller's coordinate pointer (k_pack_ptrs)
   size_t src_cap = 0;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   float last_ms = 0.0f;
@@ -440,20 +440,21 @@ ogx_status pool_from_device_desc(Compat& c, DescSrc src, int nb) {
 // over the pieces, every body's offsets.
 struct HostTables {
   std::vector<int32_t> counts;
-  std::vector<const float*> src;
+  std::vector<const void*> src;  // the caller's coordinates
   std::vector<int64_t> voff;
   std::vector<BodyRef> refs;
   int64_t pts = 0;
   uint64_t quad = 0;
 };
 
-ogx_status host_tables(const gkPolytope* a, const gkPolytope* b, int nb, HostTables& T) {
+template <class Poly>
+ogx_status host_tables(const Poly* a, const Poly* b, int nb, HostTables& T) {
   T.counts.resize(nb);
   T.src.resize(nb);
   T.voff.resize(nb);
   T.refs.resize(nb);
   std::vector<int32_t>& counts = T.counts;
-  std::vector<const float*>& src = T.src;
+  std::vector<const void*>& src = T.src;
   std::vector<int64_t>& voff = T.voff;
   std::vector<BodyRef>& refs = T.refs;
   const int nt = (int)std::min<int64_t>(16, std::max<int64_t>(1, nb >> 15));
@@ -462,7 +463,7 @@ ogx_status host_tables(const gkPolytope* a, const gkPolytope* b, int nb, HostTab
   parallel_for(nb, nt, [&](int lo, int hi, int k) {
     int64_t np = 0, nq = 0;
     for (int i = lo; i < hi; ++i) {
-      const gkPolytope& p = b ? ((i & 1) ? b[i >> 1] : a[i >> 1]) : a[i];
+      const Poly& p = b ? ((i & 1) ? b[i >> 1] : a[i >> 1]) : a[i];
       if (p.numpoints < 1 || !p.coord) {
         bad[k] = i;
         return;
@@ -477,7 +478,7 @@ ogx_status host_tables(const gkPolytope* a, const gkPolytope* b, int nb, HostTab
   });
   for (int k = 0; k < nt; ++k)
     if (bad[k] >= 0) {
-      const gkPolytope& p = b ? ((bad[k] & 1) ? b[bad[k] >> 1] : a[bad[k] >> 1]) : a[bad[k]];
+      const Poly& p = b ? ((bad[k] & 1) ? b[bad[k] >> 1] : a[bad[k] >> 1]) : a[bad[k]];
       return ogx_fail(OGX_ERR_INVALID, "polytope %d: numpoints %d, coord %p", bad[k], p.numpoints, (void*)p.coord);
     }
   for (int k = 0; k < nt; ++k) {
@@ -505,7 +506,7 @@ ogx_status host_tables(const gkPolytope* a, const gkPolytope* b, int nb, HostTab
 ogx_status upload_tables(Compat& c, const HostTables& T, int nb) {
   ogx_ctx* ctx = c.ctx;
   cudaStream_t st = ctx->stream;
-  const size_t tb = nb * sizeof(BodyRef), pb = nb * sizeof(const float*), ob = nb * sizeof(int64_t);
+  const size_t tb = nb * sizeof(BodyRef), pb = nb * sizeof(const void*), ob = nb * sizeof(int64_t);
   ogx_status s = ctx->ensure_stage(tb + pb + ob, 0);
   if (!s) s = grow(&c.d_bodies, &c.bodies_cap, (size_t)nb, "compat body table");
   if (!s) s = grow(&c.d_src, &c.src_cap, (size_t)nb, "compat coordinate pointers");
@@ -530,7 +531,7 @@ ogx_status pool_from_host_desc(Compat& c, const gkPolytope* a, const gkPolytope*
   ogx_status s0 = host_tables(a, b, nb, T);
   if (s0) return s0;
   const std::vector<int32_t>& counts = T.counts;
-  const std::vector<const float*>& src = T.src;
+  const std::vector<const void*>& src = T.src;
   const std::vector<int64_t>& voff = T.voff;
   const std::vector<BodyRef>& refs = T.refs;
   const int64_t pts = T.pts;
@@ -543,7 +544,8 @@ ogx_status pool_from_host_desc(Compat& c, const gkPolytope* a, const gkPolytope*
     // caller keeps them
     ogx_status s = upload_tables(c, T, nb);
     if (s) return s;
-    const cudaError_t e = launch_pack_ptrs(c.d_src, nb, c.d_bodies, c.d_points, 8 * ctx->sm_count, st);
+    const cudaError_t e = launch_pack_ptrs(reinterpret_cast<const float* const*>(c.d_src), nb, c.d_bodies, c.d_points,
+                                           8 * ctx->sm_count, st);
     if (e != cudaSuccess) return ogx_cuda_fail(e, "polytope pack from host memory");
     return OGX_OK;
   }
@@ -634,34 +636,97 @@ ogx_status finish(Compat& c) {
   return OGX_OK;
 }
 
+// FP32 copies of FP64 descriptor arrays: one float coordinate buffer, descriptors into it
+struct Narrowed {
+  std::vector<float> coords;
+  std::vector<gkPolytope> a, b;
+  std::vector<double> c64;  // the double coordinates in the pool's body order
+};
+
+ogx_status check_desc(const ogx_polytope_f64* src, int n) {
+  for (int i = 0; src && i < n; ++i)
+    if (src[i].numpoints < 1 || !src[i].coord)
+      return ogx_fail(OGX_ERR_INVALID, "polytope %d: numpoints %d, coord %p", i, src[i].numpoints,
+                      (void*)src[i].coord);
+  return OGX_OK;
+}
+
+void narrow_desc(const ogx_polytope_f64* src, int n, std::vector<gkPolytope>& out, std::vector<float>& coords,
+                 std::vector<int64_t>& first) {
+  out.resize(n);
+  for (int i = 0; i < n; ++i) {
+    first.push_back((int64_t)coords.size());
+    for (int k = 0; k < 3 * src[i].numpoints; ++k) coords.push_back((float)src[i].coord[k]);
+    out[i].numpoints = src[i].numpoints;
+    for (int k = 0; k < 3; ++k) out[i].s[k] = (float)src[i].s[k];
+    out[i].s_idx = src[i].s_idx;
+    out[i].coord = nullptr;  // set once the buffer stops growing
+  }
+}
+
+void narrow(int na, const ogx_polytope_f64* a, int nb, const ogx_polytope_f64* b, Narrowed& N) {
+  std::vector<int64_t> fa, fb;
+  narrow_desc(a, na, N.a, N.coords, fa);
+  if (b) narrow_desc(b, nb, N.b, N.coords, fb);
+  for (int i = 0; i < na; ++i) N.a[i].coord = N.coords.data() + fa[i];
+  for (int i = 0; b && i < nb; ++i) N.b[i].coord = N.coords.data() + fb[i];
+}
+
+// The pool and the double coordinates from FP64 descriptors in HOST memory (checked): read by
+// the device where the caller keeps them, as in pool_from_host_desc; else narrowed and
+// gathered on the host, into N (which has to outlive the call's device work).  The device
+// loads doubles, so an array that is not aligned to them is gathered too.  (1,000 pairs of 32
+// points, gathered on the host: 765 us a call; read by the device: 174.)
+ogx_status pool_from_host_f64(Compat& c, const ogx_polytope_f64* a, const ogx_polytope_f64* b, int nb, Narrowed& N) {
+  ogx_ctx* ctx = c.ctx;
+  cudaStream_t st = ctx->stream;
+  auto body = [=](int i) -> const ogx_polytope_f64& { return b ? ((i & 1) ? b[i >> 1] : a[i >> 1]) : a[i]; };
+  bool direct = pageable_reads(ctx->device);
+  int64_t pts = 0;
+  for (int i = 0; i < nb; ++i) {
+    direct = direct && reinterpret_cast<uintptr_t>(body(i).coord) % sizeof(double) == 0;
+    pts += body(i).numpoints;
+  }
+  ogx_status s = grow(&c.d_c64, &c.c64_cap, 3 * (size_t)pts, "compat double coordinates");
+  if (s) return s;
+  if (direct) {
+    HostTables T;
+    s = host_tables(a, b, nb, T);
+    if (!s) s = upload_tables(c, T, nb);
+    if (s) return s;
+    const cudaError_t e = launch_pack_ptrs64(reinterpret_cast<const double* const*>(c.d_src), nb, c.d_voff,
+                                             c.d_bodies, c.d_points, c.d_c64, 8 * ctx->sm_count, st);
+    return e == cudaSuccess ? OGX_OK : ogx_cuda_fail(e, "polytope pack from host memory");
+  }
+  if (b)
+    narrow(nb / 2, a, nb / 2, b, N);
+  else
+    narrow(nb, a, 0, nullptr, N);
+  s = pool_from_host_desc(c, N.a.data(), b ? N.b.data() : nullptr, nb);
+  if (s) return s;
+  N.c64.reserve(3 * (size_t)pts);
+  for (int i = 0; i < nb; ++i) N.c64.insert(N.c64.end(), body(i).coord, body(i).coord + 3 * (size_t)body(i).numpoints);
+  const cudaError_t e = cudaMemcpyAsync(c.d_c64, N.c64.data(), N.c64.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? OGX_OK : ogx_cuda_fail(e, "double coordinate upload");
+}
+
 // host-buffer query over pairs (2i, 2i+1) or explicit pairs; results to host arrays
 ogx_status host_query(const gkPolytope* a, const gkPolytope* b, int nbodies, int npairs,
                       const gkCollisionPair* host_pairs, gkSimplex* smp, float* dist, float* nrm,
                       float* w1, float* w2, int mode, bool upload_in, const ogx_polytope_f64* a64 = nullptr,
                       const ogx_polytope_f64* b64 = nullptr) {
   if (npairs <= 0) return OGX_OK;  // the reference returns early for n <= 0
-  if (!a || !smp || !dist) return ogx_fail(OGX_ERR_INVALID, "NULL argument");
+  if (!(a || a64) || !smp || !dist) return ogx_fail(OGX_ERR_INVALID, "NULL argument");
   Lease L;
   ogx_status s = lease(L);
   if (s) return s;
   Compat* c = L.c;
   cudaStream_t st = c->ctx->stream;
-  s = pool_from_host_desc(*c, a, b, nbodies);
+  Narrowed N;
+  s = a64 ? pool_from_host_f64(*c, a64, b64, nbodies, N) : pool_from_host_desc(*c, a, b, nbodies);
   if (!s) s = ensure_results(*c, npairs);
   if (s) return s;
-  std::vector<double> c64;
-  if (a64) {
-    // the double coordinates in the pool's body order (body i as pool_from_host_desc)
-    for (int i = 0; i < nbodies; ++i) {
-      const ogx_polytope_f64& p = b64 ? ((i & 1) ? b64[i >> 1] : a64[i >> 1]) : a64[i];
-      c64.insert(c64.end(), p.coord, p.coord + 3 * (size_t)p.numpoints);
-    }
-    s = grow(&c->d_c64, &c->c64_cap, std::max<size_t>(c64.size(), 1), "compat double coordinates");
-    if (s) return s;
-  }
   cudaError_t e = cudaSuccess;
-  if (a64) e = cudaMemcpyAsync(c->d_c64, c64.data(), c64.size() * sizeof(double), cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) return ogx_cuda_fail(e, "double coordinate upload");
   if (host_pairs) {
     const int nt = (int)std::min<int64_t>(16, std::max<int64_t>(1, npairs >> 16));
     std::vector<int> bad(nt, -1);
@@ -1023,39 +1088,6 @@ extern "C" float ogx_compat_last_gpu_ms(void) { return t_last_ms; }
 
 namespace {
 
-// FP32 copies of FP64 descriptor arrays: one float coordinate buffer, descriptors into it
-struct Narrowed {
-  std::vector<float> coords;
-  std::vector<gkPolytope> a, b;
-};
-
-ogx_status narrow_desc(const ogx_polytope_f64* src, int n, std::vector<gkPolytope>& out, std::vector<float>& coords,
-                       std::vector<int64_t>& first) {
-  out.resize(n);
-  for (int i = 0; i < n; ++i) {
-    if (src[i].numpoints < 1 || !src[i].coord)
-      return ogx_fail(OGX_ERR_INVALID, "polytope %d: numpoints %d, coord %p", i, src[i].numpoints,
-                      (void*)src[i].coord);
-    first.push_back((int64_t)coords.size());
-    for (int k = 0; k < 3 * src[i].numpoints; ++k) coords.push_back((float)src[i].coord[k]);
-    out[i].numpoints = src[i].numpoints;
-    for (int k = 0; k < 3; ++k) out[i].s[k] = (float)src[i].s[k];
-    out[i].s_idx = src[i].s_idx;
-    out[i].coord = nullptr;  // set once the buffer stops growing
-  }
-  return OGX_OK;
-}
-
-ogx_status narrow(int na, const ogx_polytope_f64* a, int nb, const ogx_polytope_f64* b, Narrowed& N) {
-  std::vector<int64_t> fa, fb;
-  ogx_status s = narrow_desc(a, na, N.a, N.coords, fa);
-  if (!s && b) s = narrow_desc(b, nb, N.b, N.coords, fb);
-  if (s) return s;
-  for (int i = 0; i < na; ++i) N.a[i].coord = N.coords.data() + fa[i];
-  for (int i = 0; b && i < nb; ++i) N.b[i].coord = N.coords.data() + fb[i];
-  return OGX_OK;
-}
-
 void narrow_simplex(const ogx_simplex_f64& d, gkSimplex& f) {
   f.nvrtx = d.nvrtx;
   for (int k = 0; k < 4; ++k)
@@ -1086,8 +1118,8 @@ ogx_status host_query_f64(const ogx_polytope_f64* a, const ogx_polytope_f64* b, 
                           double* w1, double* w2, int mode, bool upload_in) {
   if (npairs <= 0) return OGX_OK;
   if (!a || !smp || !dist) return ogx_fail(OGX_ERR_INVALID, "NULL argument");
-  Narrowed N;
-  ogx_status s = b ? narrow(npairs, a, npairs, b, N) : narrow(nbodies, a, 0, nullptr, N);
+  ogx_status s = check_desc(a, b ? npairs : nbodies);
+  if (!s) s = check_desc(b, npairs);
   if (s) return s;
   std::vector<gkSimplex> s32(npairs);
   std::vector<float> d32(npairs), n32(nrm ? 3 * (size_t)npairs : 0);
@@ -1097,7 +1129,7 @@ ogx_status host_query_f64(const ogx_polytope_f64* a, const ogx_polytope_f64* b, 
       narrow_simplex(smp[i], s32[i]);
       d32[i] = (float)dist[i];
     }
-  s = host_query(N.a.data(), b ? N.b.data() : nullptr, nbodies, npairs, pairs, s32.data(), d32.data(),
+  s = host_query(nullptr, nullptr, nbodies, npairs, pairs, s32.data(), d32.data(),
                  nrm ? n32.data() : nullptr, w1 ? w32a.data() : nullptr, w2 ? w32b.data() : nullptr, mode,
                  upload_in, a, b);
   if (s) return s;

@@ -301,21 +301,33 @@ __global__ void __launch_bounds__(128) k_polish(DevBatch B) {
 // the caller's host arrays: on a device that reads pageable host memory through the host's
 // page tables (cudaDevAttrPageableMemoryAccess, the GPU of a Grace system over NVLink-C2C)
 // the kernel loads the points where the caller keeps them, so the host gathers nothing.
-// Bodies with a NaN or infinite coordinate are marked as k_pack does.
-__global__ void k_pack_ptrs(const float* const* __restrict__ src, int nb, BodyRef* __restrict__ bodies,
-                            float* __restrict__ pool) {
+// Bodies with a NaN or infinite coordinate are marked as k_pack does.  From doubles, the pool
+// takes each rounded to float and c64 the doubles themselves (point i of body b at
+// 3 (voff[b] + i)).
+template <class T>
+__global__ void k_pack_ptrs(const T* const* __restrict__ src, int nb, BodyRef* __restrict__ bodies,
+                            float* __restrict__ pool, const int64_t* __restrict__ voff, double* __restrict__ c64) {
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int b = warp; b < nb; b += nwarps) {
     const BodyRef r = bodies[b];
-    const float* c = src[b];
+    const T* c = src[b];
     const int n4 = round4(r.n);
     float* dst = pool + 4 * (size_t)r.quad;
     bool finite = true;
     for (int i = lane; i < n4; i += 32) {
       const int s = i < r.n ? i : 0;
-      const float x = c[3 * s], y = c[3 * s + 1], z = c[3 * s + 2];
+      const T cx = c[3 * s], cy = c[3 * s + 1], cz = c[3 * s + 2];
+      if constexpr (sizeof(T) == sizeof(double)) {
+        if (i < r.n) {
+          double* d = c64 + 3 * (voff[b] + i);
+          d[0] = cx;
+          d[1] = cy;
+          d[2] = cz;
+        }
+      }
+      const float x = (float)cx, y = (float)cy, z = (float)cz;
       finite = finite && is_finite(x) && is_finite(y) && is_finite(z);
       dst[i] = x;
       dst[n4 + i] = y;
@@ -329,7 +341,14 @@ __global__ void k_pack_ptrs(const float* const* __restrict__ src, int nb, BodyRe
 cudaError_t launch_pack_ptrs(const float* const* src, int nbodies, BodyRef* bodies, float* pool, int grid,
                              cudaStream_t st) {
   if (nbodies <= 0) return cudaSuccess;
-  k_pack_ptrs<<<grid, 256, 0, st>>>(src, nbodies, bodies, pool);
+  k_pack_ptrs<float><<<grid, 256, 0, st>>>(src, nbodies, bodies, pool, nullptr, nullptr);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pack_ptrs64(const double* const* src, int nbodies, const int64_t* voff, BodyRef* bodies,
+                               float* pool, double* c64, int grid, cudaStream_t st) {
+  if (nbodies <= 0) return cudaSuccess;
+  k_pack_ptrs<double><<<grid, 256, 0, st>>>(src, nbodies, bodies, pool, voff, c64);
   return cudaGetLastError();
 }
 

@@ -521,6 +521,8 @@ cudaError_t launch_pack(const float* aos, const int64_t* voff, BodyRef* bodies, 
 // each body's count and pool offset
 cudaError_t launch_pack_ptrs(const float* const* src, int nbodies, BodyRef* bodies, float* pool, int grid,
                              cudaStream_t st);
+cudaError_t launch_pack_ptrs64(const double* const* src, int nbodies, const int64_t* voff, BodyRef* bodies,
+                               float* pool, double* c64, int grid, cudaStream_t st);
 cudaError_t launch_bin(const DevBatch& B, int grid, cudaStream_t st);
 // the whole pipeline with one warp per pair (ogx_k_warp.cu), any mode; not posed
 cudaError_t launch_warp_pairs(const DevBatch& B, cudaStream_t st);
