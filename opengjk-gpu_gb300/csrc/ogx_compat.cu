@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "ogx_engine.h"
+#include "ogx_continue.cuh"
 
 using namespace ogx;
 
@@ -166,35 +167,49 @@ __global__ void k_desc_pack(DescSrc src, int nb, BodyRef* __restrict__ bodies, f
 
 // Bodies given in double (the *_f64 calls): every separated pair continues GJK in FP64 on
 // the caller's double points from the FP32 pass's final simplex -- exact supports and
-// exact Minkowski points, one thread per pair -- so its distance carries no rounding of
-// the inputs; its simplex, witnesses and normal are replaced with the continuation's.
+// exact Minkowski points -- so its distance carries no rounding of the inputs; its simplex,
+// witnesses and normal are replaced with the continuation's.
 // Contacts keep the FP32 pass's result (their depth is within the inputs' rounding of
 // the FP64 one, far inside the 1e-4 depth tolerance); a pair the continuation finds
 // enclosed lies within rounding of touching and keeps it too.
-__global__ void __launch_bounds__(128) k_refine64(const float* __restrict__ pool, const BodyRef* __restrict__ bodies,
-                                                  const double* __restrict__ c64, const int64_t* __restrict__ voff,
-                                                  const int2* __restrict__ pairs, int npairs, gkSimplex* smp,
-                                                  float* dist, float* nrm) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npairs; p += gridDim.x * blockDim.x) {
+struct Work64 {
+  typedef D64Bodies Bodies;
+  const float* pool;
+  const BodyRef* bodies;
+  const double* c64;
+  const int64_t* voff;
+  const int2* pairs;
+  gkSimplex* smp;
+  float *dist, *nrm;
+  __device__ void idle(D64Bodies& B) const { B.bind64(pool, BodyRef{0u, 1}, BodyRef{0u, 1}, c64, c64); }
+  __device__ int load(int p, D64Bodies& B, GjkState& g) const {
     const float dp = dist[p];
-    if (!(dp > FLT_EPSILON)) continue;  // contacts, and bad input (NaN)
+    if (!(dp > FLT_EPSILON)) return -1;  // contacts, and bad input (NaN)
     const int2 pr = pairs[p];
     const BodyRef ra = bodies[pr.x], rb = bodies[pr.y];
-    if (ra.n < 1 || rb.n < 1) continue;
-    D64Bodies B;
+    if (ra.n < 1 || rb.n < 1 || smp[p].nvrtx < 1 || smp[p].nvrtx > 3) return -1;
     B.bind64(pool, ra, rb, c64 + 3 * voff[pr.x], c64 + 3 * voff[pr.y]);
-    GjkState g;
     load_simplex(smp + p, dp, g);
-    if (smp[p].nvrtx < 1 || smp[p].nvrtx > 3) continue;
-    g.certain = false;
     g.status = 0;
-    SerialTeam t;
-    gjk_refine(t, B, g, kRefineIters);
-    if (gjk_contact(g)) continue;
+    return p;
+  }
+  __device__ void store(int p, const GjkState& g) const {
+    if (gjk_contact(g)) return;
     store_simplex(smp + p, g);
     dist[p] = g.dist;
     if (nrm) store3(nrm + 3 * (size_t)p, sep_normal(g));
   }
+};
+
+// A warp per pair while three blocks per SM have one for each, or the bodies are large (as in
+// the refinement's lists); else a warp per SM quadrant, with the pairs spread over its lanes.
+// (One thread per pair ran 1,000 pairs of 32 points on 8 SMs: 47 us, now 25; the call 178 ->
+// 157 us, 100 pairs of 64 points 126 -> 90.  10,000 pairs of 8 points, 459 us a call, gain
+// nothing: with three blocks per SM they took 470.)
+template <int TL>
+__global__ void __launch_bounds__(128, 3) k_refine64(Work64 W, int npairs) {
+  continue_pairs<TL>(W, npairs, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
+                     nullptr);
 }
 
 __global__ void k_pairs_iota(gkCollisionPair* pairs, int n) {
@@ -229,6 +244,7 @@ struct Compat {
   size_t nrm_cap = 0;
   double* d_c64 = nullptr;  // the *_f64 calls: the bodies' double coordinates, pool order
   size_t c64_cap = 0;
+  int64_t points = 0;       // their number
   const void** d_src = nullptr;  // per body: the caller's coordinate pointer (k_pack_ptrs)
   size_t src_cap = 0;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
@@ -614,10 +630,13 @@ ogx_status run_timed(Compat& c, int nbodies, int npairs, const gkCollisionPair* 
   ogx_status s = ogx_run(c.ctx, c.d_points, c.d_bodies, nbodies, npairs, d_pairs, d_smp, d_dist, d_nrm,
                          nullptr, mode);
   if (!s && exact64 && mode != kModeEpa) {
-    const int grid = std::min(8 * c.ctx->sm_count, (npairs + 127) / 128);
-    k_refine64<<<std::max(grid, 1), 128, 0, c.ctx->stream>>>(c.d_points, c.d_bodies, c.d_c64, c.d_voff,
-                                                            reinterpret_cast<const int2*>(d_pairs), npairs,
-                                                            d_smp, d_dist, mode == kModeGjk ? nullptr : d_nrm);
+    const int grid = std::min(3 * c.ctx->sm_count, (npairs + 3) / 4);
+    const Work64 W{c.d_points, c.d_bodies, c.d_c64, c.d_voff, reinterpret_cast<const int2*>(d_pairs), d_smp, d_dist,
+                   mode == kModeGjk ? nullptr : d_nrm};
+    if (npairs <= 4 * grid || c.points > 128 * (int64_t)nbodies)
+      k_refine64<32><<<grid, 128, 0, c.ctx->stream>>>(W, npairs);
+    else
+      k_refine64<8><<<std::min(grid, c.ctx->sm_count), 128, 0, c.ctx->stream>>>(W, npairs);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) s = ogx_cuda_fail(e, "k_refine64 launch");
   }
@@ -689,6 +708,7 @@ ogx_status pool_from_host_f64(Compat& c, const ogx_polytope_f64* a, const ogx_po
   }
   ogx_status s = grow(&c.d_c64, &c.c64_cap, 3 * (size_t)pts, "compat double coordinates");
   if (s) return s;
+  c.points = pts;
   if (direct) {
     HostTables T;
     s = host_tables(a, b, nb, T);

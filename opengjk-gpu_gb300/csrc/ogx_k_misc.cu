@@ -1,5 +1,6 @@
 // ogx_k_misc.cu -- pool packing, pair binning and the FP64 polish pass.
 #include "ogx_kernels.cuh"
+#include "ogx_continue.cuh"
 
 namespace ogx {
 
@@ -87,7 +88,7 @@ __global__ void k_bin(DevBatch B) {
 
 // After FP64 refinement: contacts join their bucket's EPA list, separated pairs get their
 // normal from the refined witnesses.
-__device__ void refine_store(const DevBatch& B, int p, const BodyRef& ra, const BodyRef& rb, const GjkState& g) {
+__device__ void refine_store(const DevBatch& B, int p, const GjkState& g) {
   store_simplex(B.smp + p, g);
   B.dist[p] = g.dist;
   if (B.status) B.status[p] |= g.status;
@@ -113,24 +114,6 @@ __device__ __forceinline__ void bind_mem(Posed<MemBodies>& mb, const DevBatch& B
                                          BodyRef rb) {
   mb.bind_posed(B.pool, ra, rb, B.xf + 12 * (size_t)pr.x, B.xf + 12 * (size_t)pr.y);
 }
-// the bodies of lane j's pair (j may differ from lane to lane)
-__device__ __forceinline__ void shfl_bodies(MemBodies& to, const MemBodies& from, int j) {
-#pragma unroll
-  for (int w = 0; w < 2; ++w) {
-    to.base[w] = reinterpret_cast<const float*>(
-        __shfl_sync(0xffffffffu, reinterpret_cast<long long>(from.base[w]), j));
-    to.n[w] = __shfl_sync(0xffffffffu, from.n[w], j);
-    to.n4[w] = round4(to.n[w]);
-  }
-}
-__device__ __forceinline__ void shfl_bodies(Posed<MemBodies>& to, const Posed<MemBodies>& from, int j) {
-  shfl_bodies(static_cast<MemBodies&>(to), static_cast<const MemBodies&>(from), j);
-#pragma unroll
-  for (int w = 0; w < 2; ++w)
-    to.xf[w] = reinterpret_cast<const float*>(
-        __shfl_sync(0xffffffffu, reinterpret_cast<long long>(from.xf[w]), j));
-}
-
 // Re-solve of the separated pairs whose final support the GJK kernel proved exact (one
 // thread per pair): the exact closest point of their simplex in double-float arithmetic.
 template <bool kPosed>
@@ -145,87 +128,27 @@ __global__ void __launch_bounds__(128) k_refine(DevBatch B) {
     GjkState g;
     load_simplex(B.smp + p, B.dist[p], g);
     refine_certain(mb, g);
-    refine_store(B, p, ra, rb, g);
+    refine_store(B, p, g);
   }
 }
 
-// FP64 continuation of GJK for the pairs whose FP32 support was not certain.  An FP64
-// instruction holds its SM quadrant's FP64 unit for about 65 cycles however many lanes are
-// active (measured, GB300), and a pair's continuation is a chain of a few hundred of them,
-// so what counts is that every quadrant has a warp of its own and that a warp's
-// instructions serve several pairs only once there are more pairs than that: a warp takes
-// ceil(pairs / warps) pairs (1 to 32), one per lane.  Each FP64 iteration scans the warp's
-// unfinished pairs for their exact supports, 32 / TL at a time with teams of TL lanes, then
-// every lane takes its own pair's FP64 sub-distance step.  (32 pairs per warp always, and
-// one thread's serial scans for bodies of at most 128 points, left most SMs idle: 92 + 265
-// us for the 6,600 continuations of 200k power-law pairs.)
-template <int TL, bool kPosed>
-__device__ __forceinline__ void continue_list(const DevBatch& B, int cnt, const int* list, int dir, int warp,
-                                              int nwarps) {
-  const WarpTeam<TL> t;
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  constexpr int kTeams = 32 / TL;
-  const int per = min(32, max(1, (cnt + nwarps - 1) / nwarps));
-#pragma unroll 1
-  for (int base = per * warp; base < cnt; base += per * nwarps) {
-    const int k = base + lane;
-    const bool valid = lane < per && k < cnt;
-    int p = -1;
-    BodyRef ra{0u, 1}, rb{0u, 1};
-    typename PoseOf<kPosed, MemBodies>::type mb;
-    bind_mem(mb, B, make_int2(0, 0), ra, rb);  // never scanned: this lane's r.done stays set
-    GjkState g;
-    RefineState r;
-    r.done = true;
-    if (valid) {
-      p = list[dir * k];
-      const int2 pr = B.pairs[p];
-      ra = B.bodies[pr.x];
-      rb = B.bodies[pr.y];
-      bind_mem(mb, B, pr, ra, rb);
-      load_simplex(B.smp + p, B.dist[p], g);
-      g.certain = false;
-      refine_begin(mb, g, kRefineIters, r);
-    }
-#pragma unroll 1
-    for (;;) {
-      const unsigned m = __ballot_sync(full, !r.done);
-      if (m == 0u) break;
-      int my_xa = 0, my_xb = 0;
-#pragma unroll 1
-      for (int j0 = 0; j0 < per; j0 += kTeams) {
-        if (((m >> j0) & ((kTeams == 32 ? 0u : (1u << kTeams)) - 1u)) == 0u) continue;
-        const int j = j0 + lane / TL;  // this team's pair (lane j & 31's)
-        typename PoseOf<kPosed, MemBodies>::type bj;
-        shfl_bodies(bj, mb, j & 31);
-        const dv3 vj = v3<double>(__shfl_sync(full, r.v.x, j & 31), __shfl_sync(full, r.v.y, j & 31),
-                                  __shfl_sync(full, r.v.z, j & 31));
-        int xa = 0, xb = 0;
-        if (j < 32 && ((m >> j) & 1u)) {
-          float ma = -1.0f, mb2 = -1.0f;
-          xa = exact_support(t, bj, 0, -vj, ma);
-          xb = exact_support(t, bj, 1, vj, mb2);
-        }
-        __syncwarp();
-        const int src = ((lane - j0) * TL) & 31;  // the first lane of the team that scanned this lane's pair
-        xa = __shfl_sync(full, xa, src);
-        xb = __shfl_sync(full, xb, src);
-        if (lane >= j0 && lane < j0 + kTeams) {
-          my_xa = xa;
-          my_xb = xb;
-        }
-      }
-      if (!r.done) refine_step(mb, r, my_xa, my_xb, B.subtab);
-      __syncwarp();
-    }
-    if (valid) {
-      refine_end(mb, r, g);
-      refine_store(B, p, ra, rb, g);
-    }
-    __syncwarp();
+// A continuation list of the batch (dir = -1: filled from the end of its array)
+template <bool kPosed>
+struct ListWork {
+  typedef typename PoseOf<kPosed, MemBodies>::type Bodies;
+  const DevBatch& B;
+  const int* list;
+  int dir;
+  __device__ void idle(Bodies& mb) const { bind_mem(mb, B, make_int2(0, 0), BodyRef{0u, 1}, BodyRef{0u, 1}); }
+  __device__ int load(int k, Bodies& mb, GjkState& g) const {
+    const int p = list[dir * k];
+    const int2 pr = B.pairs[p];
+    bind_mem(mb, B, pr, B.bodies[pr.x], B.bodies[pr.y]);
+    load_simplex(B.smp + p, B.dist[p], g);
+    return p;
   }
-}
+  __device__ void store(int p, const GjkState& g) const { refine_store(B, p, g); }
+};
 
 // Each list gets a share of the warps by its work: a larger body's continuation (refine_full
 // filled from its end, a whole warp scans) counts as kBigCost small ones (four scanned at a
@@ -243,9 +166,9 @@ __global__ void __launch_bounds__(128, 3) k_refine_cont(DevBatch B) {
   int split = big == 0 ? 0 : (int)(nwarps * cost / (cost + small));
   if (big > 0 && small > 0) split = min(max(split, 1), nwarps - 1);
   if (warp < split)
-    continue_list<32, kPosed>(B, big, B.refine_full + (B.npairs - 1), -1, warp, split);
+    continue_pairs<32>(ListWork<kPosed>{B, B.refine_full + (B.npairs - 1), -1}, big, warp, split, B.subtab);
   else
-    continue_list<8, kPosed>(B, small, B.refine_full, 1, warp - split, nwarps - split);
+    continue_pairs<8>(ListWork<kPosed>{B, B.refine_full, 1}, small, warp - split, nwarps - split, B.subtab);
 }
 
 // The bucket kernels' contacts, list after list, each with the record at its pair's index
