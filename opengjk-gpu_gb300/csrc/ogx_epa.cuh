@@ -593,6 +593,58 @@ OGX_HD float4 set_plane(Mem& M, const Bodies& B, int s, int a, int b, int c, boo
   return pl;
 }
 
+#if defined(__CUDACC__)
+// The certified run's planes of n faces (face(k, s, a, b, c): slot and vertices), three lanes
+// per face, each with one component of every vector: plane64's operations, bit for bit, and
+// set_plane's stores.  An FP64 instruction takes its quadrant's unit for about 65 cycles
+// however many lanes are active, so the components side by side take 13 of them beside the
+// square root and the reciprocal (~600 cycles each) where one lane per face took 29.  The
+// full-capacity pass of 30k stress pairs 303 -> 289 us, of 5,003 ellipsoid pairs (3 contacts,
+// one chain each) 74 -> 68.
+template <class Mem, class Face>
+__device__ __forceinline__ void planes64_by_component(Mem& M, int n, Face face, float& cbd, int& cbest) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int c = lane % 3, first = lane - c;
+  const int li = first + (c + 1) % 3, lj = first + (c + 2) % 3;  // (lanes 30 and 31 take no face)
+  for (int k0 = 0; k0 < n; k0 += 10) {
+    const int k = k0 + lane / 3;
+    const bool mine = lane < 30 && k < n;
+    int s, va, vb, vc;
+    face(mine ? k : 0, s, va, vb, vc);
+    const double q0 = (&M.vp64[va].x)[c];
+    const double e1 = (&M.vp64[vb].x)[c] - q0, e2 = (&M.vp64[vc].x)[c] - q0;
+    const double e1i = __shfl_sync(full, e1, li), e1j = __shfl_sync(full, e1, lj);
+    const double e2i = __shfl_sync(full, e2, li), e2j = __shfl_sync(full, e2, lj);
+    const double m = e1i * e2j - e1j * e2i;
+    const double m2 = m * m, mq = m * q0;
+    auto sum = [&](double x) {
+      return __shfl_sync(full, x, first) + __shfl_sync(full, x, first + 1) + __shfl_sync(full, x, first + 2);
+    };
+    const double mm = sum(m2), mq3 = sum(mq);
+    double x = 0.0, w = (double)INFINITY;
+    if (mm > 0.0) {
+      const double inv = 1.0 / sqrt(mm);
+      x = m * inv;
+      w = mq3 * inv;
+    }
+    if (mine) {
+      const float fw = (float)w;
+      (&M.fn64[s].x)[c] = x;
+      (&M.fn[s].x)[c] = (float)x;
+      if (c == 0) {
+        M.fn64[s].w = w;
+        M.fn[s].w = fw;
+        if (fw < cbd || (fw == cbd && s < cbest)) {
+          cbd = fw;
+          cbest = s;
+        }
+      }
+    }
+  }
+}
+#endif
+
 // EPA for one pair whose GJK result is g.  `M` is this pair's shared working set.
 //
 // One expansion step, with the faces of the polytope split over the team's lanes
@@ -741,6 +793,11 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
   const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
   const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
   const bool cert = kCert && all64;
+#if defined(__CUDA_ARCH__)
+  const bool by_component = cert && L == 32;
+#else
+  const bool by_component = false;
+#endif
   // may the contact be run again with FP64 planes?
   const bool rerun = !Mem::kFull && can_spill && escalate;
   // closest live face
@@ -989,6 +1046,7 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
     M.fa[s0][0] = (uint16_t)((h0 >> 16 & 0xffu) | (h0 >> 24) << 8);
     M.fa[s0][1] = (uint16_t)(link1 | 2u << 8);
     M.fa[s0][2] = (uint16_t)(link2 | 1u << 8);
+    if (by_component) continue;
     const float4 pl = set_plane<kCert>(M, B, s0, (int)(h0 & 0xffu), (int)((h0 >> 8) & 0xffu), p, escalate, all64,
                                        cert, r.st);
     if (pl.w < cbd || (pl.w == cbd && s0 < cbest)) {
@@ -996,6 +1054,23 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
       cbest = s0;
     }
   }
+#if defined(__CUDA_ARCH__)
+  if constexpr (kCert && Team::L == 32) {
+    if (by_component) {
+      r.st |= OGX_S_EPA_ESCALATED;
+      planes64_by_component(
+          M, htot,
+          [&](int k, int& s, int& va, int& vb, int& vc) {
+            const uint32_t h = M.hz[k];
+            s = slot_of(k);
+            va = (int)(h & 0xffu);
+            vb = (int)((h >> 8) & 0xffu);
+            vc = p;
+          },
+          cbd, cbest);
+    }
+  }
+#endif
   if (live) {
 #pragma unroll 1
     for (int k = htot + lane; k < nvis; k += L) M.fn[vis.nth(k)] = make_float4_(0.0f, 0.0f, 0.0f, INFINITY);
