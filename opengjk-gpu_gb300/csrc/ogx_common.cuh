@@ -333,6 +333,31 @@ constexpr int kEpaFmax = 132;
 // ----------------------------------------------------------------------------------
 // teams
 
+// A double as a signed integer of the same order (-0 as +0, NaN below everything), and back:
+// compared and reduced without FP64 instructions.
+OGX_HD int64_t order_key64(double x) {
+  int64_t b;
+#if defined(__CUDA_ARCH__)
+  b = __double_as_longlong(x);
+#else
+  memcpy(&b, &x, sizeof b);
+#endif
+  const uint64_t mag = (uint64_t)b << 1;
+  if (mag == 0) b = 0;
+  if (mag > 0xffe0000000000000ull) return INT64_MIN;
+  return b ^ ((b >> 63) & INT64_MAX);
+}
+OGX_HD double order_value64(int64_t k) {
+  const int64_t b = k ^ ((k >> 63) & INT64_MAX);
+#if defined(__CUDA_ARCH__)
+  return __longlong_as_double(b);
+#else
+  double x;
+  memcpy(&x, &b, sizeof x);
+  return x;
+#endif
+}
+
 // Host team of one lane (test build).
 struct SerialTeam {
   static constexpr int L = 1;
@@ -340,10 +365,7 @@ struct SerialTeam {
   OGX_HD void argmax(float&, int&) const {}
   OGX_HD void argmax_pair(float&, int&, float&, int&) const {}
   OGX_HD void argmin(float&, int&) const {}
-  OGX_HD void argmax2(float&, int&, float&) const {}
-  OGX_HD void argmax_d(double&, int&) const {}
-  template <class T>
-  OGX_HD void argmax_t(T&, int&) const {}
+  OGX_HD void argmax_key(int64_t&, int&) const {}
   OGX_HD bool any(bool p) const { return p; }
   OGX_HD bool warp_any(bool p) const { return p; }
   OGX_HD int warp_max(int x) const { return x; }
@@ -447,53 +469,26 @@ struct WarpTeam {
     vb = odd ? v : v2;
     ib = odd ? i : i2;
   }
-  // FP64 max value, ties to the smaller index
-  __device__ void argmax_d(double& v, int& i) const {
+  // largest key (order_key64), ties to the smaller index: integer operations, where comparing
+  // doubles takes two FP64 instructions a round
+  __device__ void argmax_key(int64_t& v, int& i) const {
     if constexpr (L == 32) {
-      // usually one lane holds the only candidate (the others' value is -infinity)
-      const uint32_t c = __ballot_sync(0xffffffffu, v > -INFINITY);
-      if (__popc(c) == 1) {
-        const int src = __ffs(c) - 1;
-        v = __shfl_sync(0xffffffffu, v, src);
-        i = __shfl_sync(0xffffffffu, i, src);
-        return;
-      }
+      const int hi = (int)(v >> 32);
+      const int mh = __reduce_max_sync(0xffffffffu, hi);
+      const uint32_t lo = hi == mh ? (uint32_t)v : 0u;
+      const uint32_t ml = __reduce_max_sync(0xffffffffu, lo);
+      i = (int)__reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? (uint32_t)i : 0xffffffffu);
+      v = ((int64_t)mh << 32) | ml;
+      return;
     }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
-      const double v2 = __shfl_xor_sync(lanes(), v, o);
+      const int64_t v2 = __shfl_xor_sync(lanes(), v, o);
       const int i2 = __shfl_xor_sync(lanes(), i, o);
       if (v2 > v || (v2 == v && i2 < i)) {
         v = v2;
         i = i2;
       }
-    }
-  }
-  __device__ void argmax_t(double& v, int& i) const { argmax_d(v, i); }
-  __device__ void argmax_t(df& v, int& i) const {
-#pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) {
-      const df v2 = mk_df(__shfl_xor_sync(lanes(), v.hi, o), __shfl_xor_sync(lanes(), v.lo, o));
-      const int i2 = __shfl_xor_sync(lanes(), i, o);
-      if (v2 > v || (v2 == v && i2 < i)) {
-        v = v2;
-        i = i2;
-      }
-    }
-  }
-  // best value / index (ties to the smaller index) and the runner-up value over lanes
-  __device__ void argmax2(float& b1, int& i1, float& b2) const {
-#pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) {
-      const float c1 = __shfl_xor_sync(lanes(), b1, o);
-      const int j1 = __shfl_xor_sync(lanes(), i1, o);
-      const float c2 = __shfl_xor_sync(lanes(), b2, o);
-      const float lo = fminf(b1, c1);
-      if (c1 > b1 || (c1 == b1 && j1 < i1)) {
-        b1 = c1;
-        i1 = j1;
-      }
-      b2 = fmaxf(fmaxf(b2, c2), lo);
     }
   }
   // min value, ties to the smaller index (index -1 means "none" and loses)

@@ -83,8 +83,9 @@ __device__ __forceinline__ void continue_pairs(const Work& W, int cnt, int warp,
         int xa = 0, xb = 0;
         if (j < 32 && ((m >> j) & 1u)) {
           float ma = -1.0f, mb2 = -1.0f;
-          xa = exact_support(t, bj, 0, -vj, ma);
-          xb = exact_support(t, bj, 1, vj, mb2);
+          const fv3 fj = floats(vj);
+          xa = exact_support(t, bj, 0, -vj, -fj, ma);
+          xb = exact_support(t, bj, 1, vj, fj, mb2);
         }
         __syncwarp();
         const int src = ((lane - j0) * TL) & 31;  // the first lane of the team that scanned this lane's pair

@@ -254,8 +254,9 @@ OGX_HD bool thin_gain_exceeds(const Team& t, const Bodies& B, const Mem& M, int 
   const dv3 n64 = v3<double>(p.x, p.y, p.z);
   double ha, hb;
   float ma = -1.0f, mb = -1.0f;
-  exact_support(t, B, 0, n64, ma, &ha);
-  exact_support(t, B, 1, -n64, mb, &hb);
+  const fv3 n = floats(n64);
+  exact_support(t, B, 0, n64, n, ma, &ha);
+  exact_support(t, B, 1, -n64, -n, mb, &hb);
   return ha + hb - p.w > (double)tol;
 }
 
@@ -817,6 +818,7 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
   int qa = 0, qb = 0;
   fv3 q = v3<float>(0.0f, 0.0f, 0.0f);
   dv3 q64 = v3<double>(0.0, 0.0, 0.0);
+  float ac = 0.0f, bc = 0.0f;  // this lane's coordinate of q's points (by_component)
   float qq = 0.0f, scale = 0.0f;  // |q|^2, sqrt(max(scale2, |q|^2))
   bool conv = false;
   float gain = 0.0f, tol = 0.0f;
@@ -826,20 +828,28 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
         // exact supports along the closest face's FP64 normal
         const double4 pl = M.fn64[best];
         const dv3 n64 = v3<double>(pl.x, pl.y, pl.z);
+        const float4 nf = M.fn[best];  // rounded(pl)
+        const fv3 n = v3<float>(nf.x, nf.y, nf.z);
         float ea, eb;
-        qa = exact_support<Team, Bodies, double>(t, B, 0, n64, r.amax0, nullptr, &ea);
-        qb = exact_support<Team, Bodies, double>(t, B, 1, -n64, r.amax1, nullptr, &eb);
+        qa = exact_support<Team, Bodies, double>(t, B, 0, n64, n, r.amax0, nullptr, &ea);
+        qb = exact_support<Team, Bodies, double>(t, B, 1, -n64, -n, r.amax1, nullptr, &eb);
         const fv3 pa = B.point(0, qa), pb = B.point(1, qb);
         q = pa - pb;
-        q64 = B.dpoint(0, qa) - B.dpoint(1, qb);
+        if (by_component) {
+          static_assert(!kCert || !Bodies::kExact64, "the points are floats");
+          ac = lane == 0 ? pa.x : (lane == 1 ? pa.y : pa.z);
+          bc = lane == 0 ? pb.x : (lane == 1 ? pb.y : pb.z);
+        } else {
+          q64 = B.dpoint(0, qa) - B.dpoint(1, qb);
+        }
         qq = dot(q, q);
         scale = qq > r.scale2 ? sqrtf(qq) : r.root;
         // The support's gain over the face.  Its FP32 value is within ea + eb (the supports'
         // bounds) and a few roundings of the terms; only a gain nearer the tolerance than that
         // is evaluated in FP64.
-        const float fa = sdot(pa, v3<float>((float)pl.x, (float)pl.y, (float)pl.z));
-        const float fb = sdot(pb, v3<float>((float)-pl.x, (float)-pl.y, (float)-pl.z));
-        const float fw = (float)pl.w;
+        const float fa = sdot(pa, n);
+        const float fb = sdot(pb, -n);
+        const float fw = nf.w;
         const float slack = 2.0f * (ea + eb) + 4.0f * FLT_EPSILON * (fabsf(fa) + fabsf(fb) + fabsf(fw)) +
                             2e-10f * fmaxf(1.0f, scale);
         conv = !(fa + fb - fw > slack);
@@ -913,8 +923,18 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
       M.vp[p] = make_float4_(q.x, q.y, q.z, 0.0f);
       M.vid[p] = make_int2_(qa, qb);
       if constexpr (kCert)
-        if (cert) M.vp64[p] = q64;
+        if (cert && !by_component) M.vp64[p] = q64;
     }
+#if defined(__CUDA_ARCH__)
+    if constexpr (kCert) {
+      if (by_component) {
+        // a component per lane (planes64_by_component)
+        if (lane < 3) (&M.vp64[p].x)[lane] = (double)ac - (double)bc;
+        t.sync();
+        q64 = M.vp64[p];
+      }
+    }
+#endif
     ++r.nv;
     r.scale2 = fmaxf(r.scale2, qq);
     r.root = scale;
