@@ -154,6 +154,15 @@ int twin_pose_points(int nbodies, const int32_t* counts, const float* local, con
   return 0;
 }
 
+// order_key64 element by element, and the keys' values back
+int twin_order_key64(int64_t n, const double* x, int64_t* key, double* back) {
+  for (int64_t i = 0; i < n; ++i) {
+    key[i] = order_key64(x[i]);
+    back[i] = order_value64(key[i]);
+  }
+  return 0;
+}
+
 // world points of the transform kernel (world_point); settled[i]: all of point i's coordinates
 // came from the FP32 instructions
 int twin_world_points(int n, const float* xf, const float* local, float* out, uint8_t* settled) {
