@@ -18,7 +18,7 @@ SMP64 = np.dtype([("nvrtx", "<i4"), ("vrtx", "<f8", (4, 3)), ("vrtx_idx", "<i4",
 
 def _bodies(nb, seed):
     g = np.random.default_rng(seed)
-    counts = g.choice([1, 2, 3, 4, 5, 7, 8, 9, 31, 32, 33, 127, 130], nb)
+    counts = g.choice([1, 2, 3, 4, 5, 7, 8, 9, 31, 32, 33, 127, 130, 255, 257, 513], nb)
     off = np.concatenate([[0], np.cumsum(counts)[:-1]])
     pts = g.normal(size=(int(counts.sum()), 3))
     pts /= np.linalg.norm(pts, axis=1, keepdims=True)
