@@ -248,6 +248,26 @@ cudaError_t halloc(T** p, size_t n) {
   return cudaMallocHost(reinterpret_cast<void**>(p), std::max<size_t>(16, n * sizeof(T)));
 }
 
+// Index of the first NaN or infinity in x[0, n), n if there is none.  A block's entries are
+// or-ed together, so that the compiler can check several at a time: an exponent of all ones
+// carries into the sign's place.
+size_t first_not_finite(const float* x, size_t n) {
+  constexpr size_t kStep = 1024;
+  for (size_t i0 = 0; i0 < n; i0 += kStep) {
+    const size_t i1 = std::min(n, i0 + kStep);
+    uint32_t seen = 0;
+    for (size_t i = i0; i < i1; ++i) {
+      uint32_t u;
+      std::memcpy(&u, x + i, sizeof u);
+      seen |= (u & 0x7fffffffu) + 0x00800000u;
+    }
+    if ((seen >> 31) == 0u) continue;
+    for (size_t i = i0; i < i1; ++i)
+      if (!is_finite(x[i])) return i;
+  }
+  return n;
+}
+
 }  // namespace
 
 bool ogx_server::admit(Request* r, Slot& s, int w) {
@@ -657,10 +677,8 @@ extern "C" ogx_status ogx_server_set_transforms(ogx_server* S, const float* xf, 
   // a pose with a NaN or an infinity would put non-finite points into the world copy
   // that every request of the version reads: refuse the update
   {
-    const size_t nf = 12 * (size_t)S->local->nbodies;
-    for (size_t i = 0; i < nf; ++i)
-      if (!ogx::is_finite(xf[i]))
-        return ogx_fail(OGX_ERR_INVALID, "pose of body %zu has a NaN or infinite entry", i / 12);
+    const size_t nf = 12 * (size_t)S->local->nbodies, i = first_not_finite(xf, nf);
+    if (i < nf) return ogx_fail(OGX_ERR_INVALID, "pose of body %zu has a NaN or infinite entry", i / 12);
   }
   std::unique_lock<std::mutex> lk(S->mu);
   if (S->stop) return ogx_fail(OGX_ERR_INVALID, "server is being destroyed");
