@@ -99,8 +99,8 @@ OGX_LEAF bool exact_bit(const Vx<T>* s, int n, uint32_t m) {
 // Signed-volume step (openGJK.c:257-613) on exact points: reduces s (2 to 4 points, newest
 // last) to the vertices it needs and sets dir to its closest point to the origin.  The
 // decision is the FP32 step's, on exactly evaluated bits: `bits` are its predicates, those
-// in `known` already right (an FP32 value outside its rounding bound has the exact sign);
-// the others are evaluated when the decision comes to depend on them, each once.
+// in `known` already right (step_known); the others are evaluated when the decision comes to
+// depend on them, each once.
 template <class T>
 OGX_LEAF void subdistance(Sx<T>& s, vec3<T>& dir, const uint32_t* subtab, uint32_t bits, uint32_t known) {
   const int n = s.n;
@@ -445,7 +445,7 @@ OGX_HD void gjk_iterate(const Team& t, const Bodies& B, const Config& cfg, GjkRu
     }
     int order[4] = {0, 1, 2, 3};
     fv3 vd;
-    nn = escalate_step(B.mem_view(), n, ias, ibs, v, order, &vd, subtab, bits, ~unc);
+    nn = escalate_step(B.mem_view(), n, ias, ibs, v, order, &vd, subtab, bits, step_known(n, S, unc));
     v = vd;
     r.status |= OGX_S_GJK_ESCALATED;
 #pragma unroll
@@ -924,11 +924,11 @@ OGX_HD void refine_step(const Bodies& B, RefineStateT<T>& r, int xa, int xb, con
   r.ia[nw] = xa;
   r.ib[nw] = xb;
   s.n++;
-  // predicates outside their FP32 rounding bound on the rounded points are decided there
+  // predicates whose FP32 value on the rounded points has the exact sign are decided there
   StepIn S;
   uint32_t bits, unc;
   step_predicates(s.n, Pf, wf, S, bits, unc);
-  subdistance(s, r.v, subtab, bits, ~unc);
+  subdistance(s, r.v, subtab, bits, step_known(s.n, S, unc));
   T vnew = dot(r.v, r.v);
   r.lam_valid = false;
   if (s.n != 4 && !(vnew < vv * T(1.0 - 1e-12))) {

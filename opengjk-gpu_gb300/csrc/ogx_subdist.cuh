@@ -293,6 +293,29 @@ OGX_HD void step_predicates(int n, const fv3* P, fv3 q1, StepIn& S, uint32_t& bi
   }
 }
 
+// The predicate bits (of those that the n-point step has) that an evaluation on the exact
+// points may take over.  Its points differ from the ones in S: each coordinate there is the
+// exact one rounded once (u = FLT_EPSILON / 2), so edge k is off by up to 2 u (lq + le_k) in
+// 1-norm.  The bounds of K, D and F above hold that error: with the edges' errors and the
+// roundings of the evaluation, a_k is off by u lq (6 le_k + 2 lq), d(j,k) by
+// u lq le_j (30 le_j le_k + lq (8 le_k + 4 le_j)), q1.(e_j x e_k) by
+// u lq (10 le_j le_k + 2 lq (le_j + le_k)).  The sign of the volume is off by
+// u (11 le0 le1 le2 + 2 lq (le0 le1 + le0 le2 + le1 le2)), which bdet does not hold where the
+// edges are short against the points: bodies far apart for their size.  (The FP32 step goes
+// by bdet all the same: it takes the decision as a whole to be exact only if no bit is within
+// its bound, and there the F bits always are.)  The products of the edges' errors add less
+// than a hundredth: a value outside its bound has every edge in it longer than 16 u lq.
+OGX_HD uint32_t step_known(int n, const StepIn& S, uint32_t unc) {
+  uint32_t known = ~unc;
+  if (n == 4) {
+    const float det = dot(S.e[1], S.c02);
+    const float l01 = S.le[0] * S.le[1], l02 = S.le[0] * S.le[2], l12 = S.le[1] * S.le[2];
+    const float b = 16.0f * FLT_EPSILON * (l01 * S.le[2] + S.lq * (l01 + l02 + l12));
+    if (!(fabsf(det) > b)) known &= ~PB_NEG;
+  }
+  return known;
+}
+
 // decision of the n-point step from its predicate bits, walked through the tree
 OGX_LEAF SubOut step_decide_tree(int n, uint32_t bits) {
   Bits B{bits, 0u};

@@ -163,6 +163,37 @@ int twin_order_key64(int64_t n, const double* x, int64_t* key, double* back) {
   return 0;
 }
 
+// Predicates of n-point steps (count of them; p: 4 points each as 2 x 3 floats a, b, the point
+// being a - b, newest at n - 1): the FP32 bits on the rounded points, those that an exact
+// evaluation takes over, and the bits evaluated in FP64
+int twin_step_bits(int count, int n, const float* p, uint32_t* bits, uint32_t* known, uint32_t* exact) {
+  for (int i = 0; i < count; ++i) {
+    fv3 P[3], q = v3<float>(0.f, 0.f, 0.f);
+    Vx<double> s[4];
+    for (int j = 0; j < n; ++j) {
+      const float *a = p + 24 * (size_t)i + 6 * j, *b = a + 3;
+      const fv3 w = v3<float>(a[0], a[1], a[2]) - v3<float>(b[0], b[1], b[2]);
+      if (j == n - 1)
+        q = w;
+      else
+        P[j] = w;
+      s[j].p = v3<double>((double)a[0] - b[0], (double)a[1] - b[1], (double)a[2] - b[2]);
+    }
+    for (int j = n - 1; j < 3; ++j) P[j] = q;
+    StepIn S;
+    uint32_t unc;
+    step_predicates(n, P, q, S, bits[i], unc);
+    known[i] = step_known(n, S, unc);
+    exact[i] = 0u;
+    for (int k = 0; k < 13; ++k) {
+      const bool needs4 = k >= 3 && k < 7;
+      const int slot = k < 3 ? k : (k < (int)PB_D + 2 ? 1 : 2);
+      if (needs4 ? n == 4 : slot < n - 1) exact[i] |= exact_bit(s, n, 1u << k) ? 1u << k : 0u;
+    }
+  }
+  return 0;
+}
+
 // world points of the transform kernel (world_point); settled[i]: all of point i's coordinates
 // came from the FP32 instructions
 int twin_world_points(int n, const float* xf, const float* local, float* out, uint8_t* settled) {
