@@ -301,17 +301,25 @@ OGX_HD void step_predicates(int n, const fv3* P, fv3 q1, StepIn& S, uint32_t& bi
 // u lq le_j (30 le_j le_k + lq (8 le_k + 4 le_j)), q1.(e_j x e_k) by
 // u lq (10 le_j le_k + 2 lq (le_j + le_k)).  The sign of the volume is off by
 // u (11 le0 le1 le2 + 2 lq (le0 le1 + le0 le2 + le1 le2)), which bdet does not hold where the
-// edges are short against the points: bodies far apart for their size.  (The FP32 step goes
-// by bdet all the same: it takes the decision as a whole to be exact only if no bit is within
-// its bound, and there the F bits always are.)  The products of the edges' errors add less
-// than a hundredth: a value outside its bound has every edge in it longer than 16 u lq.
+// edges are short against the points: bodies far apart for their size, whose tetrahedra then
+// came out as enclosing the origin.  (bdet still says which FP32 steps are evaluated again.)
+// The products of the edges' errors add less than a hundredth: a value outside its bound has
+// every edge in it longer than 16 u lq.
+// All of this holds while no product overflows or underflows: lengths up to 2^30 leave the
+// products of four of them (and their bounds) finite, from 2^-24 they leave FLT_EPSILON times
+// those normal.  Outside, or where a length is not a number, nothing is known.
 OGX_HD uint32_t step_known(int n, const StepIn& S, uint32_t unc) {
+  const float lo = 5.9604645e-8f, hi = 1073741824.0f;  // 2^-24, 2^30
+  bool in_range = S.lq >= lo && S.lq <= hi;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) in_range = in_range && (k >= n - 1 || (S.le[k] >= lo && S.le[k] <= hi));
+  if (!in_range) return 0u;
   uint32_t known = ~unc;
   if (n == 4) {
     const float det = dot(S.e[1], S.c02);
     const float l01 = S.le[0] * S.le[1], l02 = S.le[0] * S.le[2], l12 = S.le[1] * S.le[2];
     const float b = 16.0f * FLT_EPSILON * (l01 * S.le[2] + S.lq * (l01 + l02 + l12));
-    if (!(fabsf(det) > b)) known &= ~PB_NEG;
+    if (fabsf(det) <= b) known &= ~PB_NEG;
   }
   return known;
 }

@@ -78,6 +78,34 @@ def test_known_bits_have_the_exact_sign(twin, n, apart):
         assert (((known & MASK[n]) == MASK[n]).mean()) > 0.5
 
 
+@pytest.mark.parametrize("n", [2, 3, 4])
+@pytest.mark.parametrize("scale", [-140, -60, -45, -38, -30, -25, -20, 20, 28, 31, 33, 40, 63, 100, 126])
+def test_known_bits_at_every_scale(twin, n, scale):
+    """Up to where products of four lengths overflow, and down to where they vanish."""
+    g = np.random.default_rng(abs(scale) + n)
+    for thickness in (1, 1e-3, 0):
+        p = tetrahedra(g, 4000, 1, thickness).astype(np.float64) * 2.0 ** scale
+        p *= 2.0 ** g.integers(-12, 1, (len(p), 4, 1))  # points of different sizes
+        p = np.clip(p, -3e38, 3e38).astype(np.float32)
+        bits, known, exact = step_bits(twin, n, p)
+        for i in np.nonzero((bits ^ exact) & known & MASK[n])[0]:
+            assert ((int(bits[i]) ^ rational_bits(n, p[i])) & int(known[i]) & MASK[n]) == 0, (thickness, p[i])
+    # (sizes 2^-12 to 1 times the scale: all of them out of range at the ends, some in it between)
+    any_known = ((known & MASK[n]) != 0).any()
+    assert any_known if -20 <= scale <= 28 else True
+    assert not any_known if scale <= -45 or scale >= 63 else True
+
+
+@pytest.mark.parametrize("exponent", [31, 50])
+@pytest.mark.parametrize("apart", [3, 30])
+def test_large_bodies_whose_products_overflow(orc, twin, apart, exponent):
+    b = far_bodies.batch(5 + apart, 3000, apart, 0.0, "line")
+    b.coords *= np.float32(2.0 ** exponent)
+    o = orc.run(b.coords, b.offsets, b.counts, b.pairs, mode=orc.MODE_GJK, precision="f64", threads=8)
+    r = twin.run(b, mode=1)
+    assert (np.abs(r["dist"] - o["dist"]) <= 1e-5 * o["dist"]).all()
+
+
 def test_fp64_bits_are_the_rational_ones(twin):
     g = np.random.default_rng(3)
     for n in (2, 3, 4):
