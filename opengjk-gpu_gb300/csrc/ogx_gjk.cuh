@@ -587,8 +587,9 @@ OGX_HD void gjk_pair(const Team& t, const Bodies& B, const Config& cfg, GjkState
 // instruction, a conversion or comparison too, costs 65 cycles on this part.  Otherwise the
 // band's points are evaluated in FP64, ties to the lowest index: each lane's best, at once, as
 // long as no lane holds two of them, else by a second pass over the body; the values are
-// compared as integers.  (Always the second pass, doubles compared in the reduction: 1,000
-// pairs of 1,000-point shells 75 us, now 65; 30k stress pairs 833 -> 771.)
+// compared as integers.  Where a product or a sum of the scan may overflow, the scan says
+// nothing and the second pass takes every point.  (Always the second pass, doubles compared in
+// the reduction: 1,000 pairs of 1,000-point shells 75 us, now 65; 30k stress pairs 833 -> 771.)
 // amax: the body's largest |coordinate|, or negative to have it found (and returned there).
 // fd: d rounded to FP32; val (may be null): the exact value; err (may be null): e.
 template <class Team, class Bodies, class T>
@@ -611,9 +612,10 @@ OGX_LEAF int exact_support_of(const Team t, const Bodies B, int w, vec3<T> d, fv
   // bodies given in double: the float points are the inputs rounded (half an ulp each),
   // one more FLT_EPSILON * amax * |d|_1 of difference to cover
   const float ef = Bodies::kExact64 ? 5.0f : 4.0f;
-  const float e = ef * FLT_EPSILON * am * (fabsf(fd.x) + fabsf(fd.y) + fabsf(fd.z)) + FLT_MIN;
+  const float l1d = fabsf(fd.x) + fabsf(fd.y) + fabsf(fd.z);
+  const float e = ef * FLT_EPSILON * am * l1d + FLT_MIN;
   if (err) *err = e;
-  const float lo = m - 2.0f * e;
+  const float lo = am * l1d < 1e38f ? m - 2.0f * e : -INFINITY;
   auto exact = [&](int i) -> T {
     if constexpr (Bodies::kExact64) {
       const dv3 p = B.dpoint(w, i);

@@ -194,6 +194,19 @@ int twin_step_bits(int count, int n, const float* p, uint32_t* bits, uint32_t* k
   return 0;
 }
 
+// exact support index and value of one body (SoA pool at quad 0, n points) along count directions
+int twin_exact_support(const float* pool, int n, int count, const double* d, int32_t* index, double* value) {
+  MemBodies B;
+  B.bind(pool, BodyRef{0u, n}, BodyRef{0u, n});
+  SerialTeam t;
+  float amax = -1.0f;
+  for (int i = 0; i < count; ++i) {
+    const dv3 v = v3<double>(d[3 * i], d[3 * i + 1], d[3 * i + 2]);
+    index[i] = exact_support(t, B, 0, v, floats(v), amax, value + i);
+  }
+  return 0;
+}
+
 // world points of the transform kernel (world_point); settled[i]: all of point i's coordinates
 // came from the FP32 instructions
 int twin_world_points(int n, const float* xf, const float* local, float* out, uint8_t* settled) {
