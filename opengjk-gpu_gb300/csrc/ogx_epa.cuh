@@ -669,8 +669,8 @@ __device__ __forceinline__ void planes64_by_component(Mem& M, int n, Face face, 
 //
 // EpaMemSmall: can_spill (always set in the pipelines) lets a contact that needs the full
 // capacity or the certified run leave with o.spill set; sink: where a capacity spill saves
-// itself.  EpaMemCert: no larger capacity; rs: a saved expansion to continue instead of
-// starting from the GJK simplex.  kCert (full capacity only): with FP64 face planes on, run
+// itself (FP32 planes only).  EpaMemCert: no larger capacity; rs: a saved expansion to continue
+// instead of starting from the GJK simplex.  kCert (full capacity only): with FP64 face planes on, run
 // the certified expansion described at kEpaCertGain.
 // The loop state of one expansion (registers that live through the loop: kept few).
 template <class Mem>
@@ -1107,14 +1107,16 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
 template <bool kCert = false, class Team, class Bodies, class Mem>
 OGX_HD void epa_finish(const Team& t, const Bodies& B, const Config& cfg, Mem& M, EpaOut& o, const EpaRun<Mem>& r,
                        bool can_spill, const EpaResumeSink& sink) {
+  const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
   if (o.spill) {
-    // the polytope as it was at the top of the last expansion
+    // The polytope as it was at the top of the last expansion.  With FP64 planes the full pass
+    // is a certified run, whose FP64 planes and points a record does not hold: that one starts
+    // again.
     if constexpr (!Mem::kFull)
-      epa_save(t, M, sink, o, r.flags & kRunLate ? r.nv - 1 : r.nv, r.fend, r.it - 1, r.st, r.scale2);
+      if (!all64) epa_save(t, M, sink, o, r.flags & kRunLate ? r.nv - 1 : r.nv, r.fend, r.it - 1, r.st, r.scale2);
     return;
   }
   const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
-  const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
   const bool cert = kCert && all64;
   const bool rerun = !Mem::kFull && can_spill && escalate;
   bool again = (r.flags & kRunAgain) != 0u;

@@ -34,6 +34,7 @@ struct Job {
 struct Work {
   EpaMemSmall small;
   EpaMemCert full;
+  EpaResume saved;
 };
 
 void bind(MemBodies& B, const Job& J, int b1, int b2, BodyRef A, BodyRef Bb) { B.bind(J.pool, A, Bb); }
@@ -72,21 +73,26 @@ void one(const Job& J, int i, Work& M) {
   float d = g.dist;
   fv3 w0 = g.w0, w1 = g.w1, n = v3<float>(0.f, 0.f, 0.f);
   int st = g.status, ei = 0;
-  if (J.mode == 2) {
+  if (J.mode >= 2) {
     if (contact) {
       // as on the device: the small working set first, full capacity when it runs out;
-      // contacts found by the refinement go straight to the certified full pass
+      // contacts found by the refinement go straight to the certified full pass.  Mode 3: a
+      // contact that outgrew the small capacity is saved and continued, as the bucket kernels do
       EpaOut o;
+      int nsaved = 0;
+      EpaResumeSink sink{J.mode == 3 ? &M.saved : nullptr, &nsaved, 1};
       if (late) {
         o.spill = true;
         o.spill64 = true;
       } else {
-        epa_pair(t, B, *J.cfg, g, M.small, o, true);
+        epa_pair(t, B, *J.cfg, g, M.small, o, true, sink);
       }
       if (o.spill) {
         ogx_config c = *J.cfg;
         if (o.spill64) c.flags |= OGX_F_EPA_FP64_PLANES;
-        epa_pair<true>(t, B, c, g, M.full, o, false);
+        const EpaResume* rs = !late && o.resume == 0 ? &M.saved : nullptr;
+        memset(&M.full, 0xff, sizeof M.full);  // (a pass that reads what it did not write shows)
+        epa_pair<true>(t, B, c, g, M.full, o, false, EpaResumeSink{nullptr, nullptr, 0}, rs);
       }
       if (o.polish) epa_polish(B, o);
       d = o.dist;
@@ -228,7 +234,7 @@ int twin_world_points(int n, const float* xf, const float* local, float* out, ui
 int twin_run_posed(int npairs, const float* pool, const uint32_t* quad, const int32_t* counts,
                    const int32_t* pairs, int mode, const ogx_config* cfg, float* dist, gkSimplex* smp,
                    float* nrm, int32_t* status, int32_t* iters, int nthreads, const float* xf) {
-  if (npairs < 0 || (mode != 1 && mode != 2)) return -1;
+  if (npairs < 0 || mode < 1 || mode > 3) return -1;
   Job base{0, npairs, mode, pool, quad, counts, pairs, cfg, dist, smp, nrm, status, iters, xf};
   if (nthreads <= 1 || npairs < 64) {
     worker(&base);
