@@ -1107,16 +1107,17 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
 template <bool kCert = false, class Team, class Bodies, class Mem>
 OGX_HD void epa_finish(const Team& t, const Bodies& B, const Config& cfg, Mem& M, EpaOut& o, const EpaRun<Mem>& r,
                        bool can_spill, const EpaResumeSink& sink) {
-  const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
   if (o.spill) {
     // The polytope as it was at the top of the last expansion.  With FP64 planes the full pass
     // is a certified run, whose FP64 planes and points a record does not hold: that one starts
     // again.
     if constexpr (!Mem::kFull)
-      if (!all64) epa_save(t, M, sink, o, r.flags & kRunLate ? r.nv - 1 : r.nv, r.fend, r.it - 1, r.st, r.scale2);
+      if (!(cfg.flags & OGX_F_EPA_FP64_PLANES))
+        epa_save(t, M, sink, o, r.flags & kRunLate ? r.nv - 1 : r.nv, r.fend, r.it - 1, r.st, r.scale2);
     return;
   }
   const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
+  const bool all64 = (cfg.flags & OGX_F_EPA_FP64_PLANES) != 0;
   const bool cert = kCert && all64;
   const bool rerun = !Mem::kFull && can_spill && escalate;
   bool again = (r.flags & kRunAgain) != 0u;
