@@ -217,6 +217,10 @@ OGX_HD fv3 simplex_sep_normal(const MemBodies& B, const gkSimplex& s) {
   return unit_or_x(w1 - w0);
 }
 
+// A scan whose values are all NaN or -infinity (coordinates whose products overflow) finds no
+// point: any one then, for the index is read with.
+OGX_HD int found(int i) { return i == 0x7fffffff ? 0 : i; }
+
 // support of the Minkowski difference along d (first maximum wins, EPA.c:307-344)
 template <class Team, class Bodies>
 OGX_HD fv3 msupport(const Team& t, const Bodies& B, fv3 d, int& ia, int& ib) {
@@ -224,6 +228,8 @@ OGX_HD fv3 msupport(const Team& t, const Bodies& B, fv3 d, int& ia, int& ib) {
   B.scan(t, 0, d, ba, ia);
   B.scan(t, 1, -d, bb, ib);
   t.argmax_pair(ba, ia, bb, ib);
+  ia = found(ia);
+  ib = found(ib);
   return B.point(0, ia) - B.point(1, ib);
 }
 
@@ -872,6 +878,8 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
     }
     t.argmax_pair(ba, qa, bb, qb);
     if (live) {
+      qa = found(qa);
+      qb = found(qb);
       q = B.point(0, qa) - B.point(1, qb);
       qq = dot(q, q);
       scale = qq > r.scale2 ? sqrtf(qq) : r.root;

@@ -650,7 +650,7 @@ OGX_LEAF int exact_support_of(const Team t, const Bodies B, int w, vec3<T> d, fv
   }
   t.argmax_key(k1, i1);
   if (val) *val = order_value64(k1);
-  return i1;
+  return i1 == 0x7fffffff ? 0 : i1;  // (every value NaN: d is)
 }
 // (on copies of the team and of the points-by-index view, so that the caller's body source
 // keeps its registers)
