@@ -98,17 +98,17 @@ struct Launch {
 
 std::vector<Launch> g_gjkv, g_epav;  // all compiled variants
 std::vector<Launch> g_gjkp, g_epap;  // the posed kernels, one per bucket
+std::vector<Launch> g_epaf;          // EPA of small and medium batches, one per bucket
 
 constexpr int kBlock = 128;
 // largest batches of the one-warp-per-pair pipeline (distances only / with EPA) and of EPA
-// with one warp per contact in the bucket kernels (ogx_run has the measurements)
-constexpr int kWarpPairsGjk = 4096, kWarpPairsEpa = 2048, kWideEpaPairs = 24576;
+// with a warp per contact while a bucket has few (ogx_run has the measurements)
+constexpr int kWarpPairsGjk = 4096, kWarpPairsEpa = 2048, kFewEpaPairs = 24576;
 constexpr int kBucketCap[kBuckets] = {16, 32, 64, 128, 256, 512, 0};
 
 std::mutex g_init_mu;
 int g_init_device = -1;
 int g_grid_bin = 0, g_grid_polish = 0, g_grid_pack = 0, g_grid_refine = 0, g_grid_cont = 0, g_grid_spill = 0;
-int g_epa_wide[kBuckets];  // EPA variant with one warp per contact, per bucket
 uint32_t* g_subtab = nullptr;  // sub-distance decision table on the initialised device
 // per-device autotuned choices (variant index per bucket), -1 = not tuned
 int g_tuned[16][2][kBuckets];
@@ -218,11 +218,14 @@ ogx_status init_kernels(int device) {
     if (s) return s;
   }
   {
-    const KernelInfo *pg, *pe;
+    const KernelInfo *pg, *pe, *fe;
     posed_variants(&pg, &pe);
+    few_variants(&fe);
     g_gjkp.clear();
     g_epap.clear();
+    g_epaf.clear();
     for (int b = 0; b < kBuckets; ++b) {
+      g_epaf.push_back(Launch{fe[b].fn, fe[b].L, fe[b].K, 0, 0});
       g_gjkp.push_back(Launch{pg[b].fn, pg[b].L, pg[b].K, 0, 0});
       g_epap.push_back(Launch{pe[b].fn, pe[b].L, pe[b].K, 0, 0});
     }
@@ -230,12 +233,12 @@ ogx_status init_kernels(int device) {
       ogx_status s = init_variant(&k, false, sms);
       if (s) return s;
     }
-    for (auto& k : g_epap) {
-      ogx_status s = init_variant(&k, true, sms);
-      if (s) return s;
-    }
+    for (auto* v : {&g_epap, &g_epaf})
+      for (auto& k : *v) {
+        ogx_status s = init_variant(&k, true, sms);
+        if (s) return s;
+      }
   }
-  for (int b = 0; b < kBuckets; ++b) g_epa_wide[b] = warp_choice(g_epav, b);
   g_grid_bin = 4 * sms;
   g_grid_pack = 8 * sms;
   int per_sm = 0;
@@ -777,10 +780,11 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
     ctx->last_launches = 1;
     return OGX_OK;
   }
-  // EPA with one warp per contact where the contacts of a batch cannot fill the GPU with
-  // narrower teams: a contact then ends sooner (10,000 pairs 253-286 us against 289-335;
-  // 20,000 318-342 against 349-353; 50,000 586-599 against 524-574).
-  const bool wide_epa = npairs <= kWideEpaPairs && !d_xf && !ctx->choice_set;
+  // EPA by the number of contacts (k_epa_few) in batches whose buckets may well have too few
+  // to fill the GPU with narrow teams: 5,000 power-law pairs 199 us, 10,000 281, 20,000 333,
+  // 24,000 412; with the tuned variants 5,000 259, 20,000 391, 24,000 490.  (A warp per contact
+  // always: 50,000 pairs 586-599 us against 524-574.)
+  const bool few_epa = npairs <= kFewEpaPairs && !d_xf && !ctx->choice_set;
   const int bin_grid = std::min(g_grid_bin, (npairs + 255) / 256);
   ctx->mark("bin");
   e = launch_bin(B, bin_grid, st);
@@ -844,9 +848,9 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   const bool refine = mode != kModeEpa && (ctx->cfg.flags & OGX_F_FP64_POLISH);
   if (mode != kModeGjk) {
     for (int b = kBuckets - 1; b >= 0 && e == cudaSuccess; --b) {
-      const Launch& k = d_xf ? g_epap[b] : g_epav[wide_epa ? g_epa_wide[b] : ctx->choice[1][b]];
+      const Launch& k = d_xf ? g_epap[b] : few_epa ? g_epaf[b] : g_epav[ctx->choice[1][b]];
       ctx->mark(kEpaName[b]);
-      k.fn<<<fit_grid(k.grid, npairs, k.L), kBlock, k.smem, bucket_stream(b)>>>(B, b);
+      k.fn<<<fit_grid(k.grid, npairs, few_epa ? 32 : k.L), kBlock, k.smem, bucket_stream(b)>>>(B, b);
       stage(kEpaName[b], bucket_stream(b));
       ++launches;
     }

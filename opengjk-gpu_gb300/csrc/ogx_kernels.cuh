@@ -419,15 +419,14 @@ OGX_HD constexpr size_t epa_team_stride(int L) {
 template <int L>
 OGX_HD constexpr size_t epa_mem_bytes() { return (kStageStride / L) * epa_team_stride(L); }
 
-template <int L, int K, int OCC = 1, int D = 0, bool kPosed = false>
-__global__ void __launch_bounds__(kStageStride, OCC) k_epa(DevBatch B, int bucket) {
+template <int L, int K, int D = 0, bool kPosed = false>
+__device__ __forceinline__ void epa_bucket(const DevBatch& B, int bucket, int cnt) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float4* slots = reinterpret_cast<float4*>(smem_raw + epa_mem_bytes<L>()) + threadIdx.x;
   const WarpTeam<L> t;
   EpaMemSmall& M = *reinterpret_cast<EpaMemSmall*>(smem_raw + (threadIdx.x / L) * epa_team_stride(L));
   const int team = (blockIdx.x * blockDim.x + threadIdx.x) / L;
   const int nteams = (gridDim.x * blockDim.x) / L;
-  const int cnt = B.counts[kCntEpa + bucket];
   const int* list = B.elists + (size_t)bucket * B.npairs;
   const WarpTeam<L, true> all;  // the expansions, by all teams of the warp together
   const EpaResumeSink sink{B.resume, B.counts + kCntResume, B.resume_cap};
@@ -471,6 +470,29 @@ __global__ void __launch_bounds__(kStageStride, OCC) k_epa(DevBatch B, int bucke
   if constexpr (D > 0) cp_async_wait<0>();  // no copy outlives the block
 }
 
+template <int L, int K, int OCC = 1, int D = 0, bool kPosed = false>
+__global__ void __launch_bounds__(kStageStride, OCC) k_epa(DevBatch B, int bucket) {
+  epa_bucket<L, K, D, kPosed>(B, bucket, B.counts[kCntEpa + bucket]);
+}
+
+// EPA over one bucket's contacts in a batch of at most 24,576 pairs.  A contact is bound by its
+// chain of expansions, which a whole warp ends soonest, as long as the contacts do not queue for
+// warps; a bucket with more of them than about half a wave (4 blocks of 4 warps on 152 SMs; the
+// other buckets run beside it) is done sooner by narrow teams.  How many there are only the
+// device knows, so both are in one kernel.  (A warp per contact whatever their number, by the
+// batch's pairs alone: 16,000 contacts of 16-point bodies 418 us, now 286, 16,000 of 64-point
+// ones 1,213 and 1,025, 20,000 power-law pairs 370 and 333.  Limits of 1,000, 1,500, 2,000 and
+// 2,432 contacts: 20,000 power-law pairs 333, 333, 342, 344, 5,000 all the same.)
+constexpr int kWideContacts = 1000;
+template <int LN>
+__global__ void __launch_bounds__(kStageStride, 4) k_epa_few(DevBatch B, int bucket) {
+  const int cnt = B.counts[kCntEpa + bucket];
+  if (cnt <= kWideContacts)
+    epa_bucket<32, 0>(B, bucket, cnt);
+  else
+    epa_bucket<LN, 0>(B, bucket, cnt);
+}
+
 // ---------------------------------------------------------------------------------
 // launch table (one translation unit per kernel family, see ogx_k_*.cu)
 
@@ -506,6 +528,8 @@ int epa_variants_c(const KernelInfo** out);
 int epa_variants_d(const KernelInfo** out);
 // the posed kernels (ogx_k_posed.cu): one GJK and one EPA variant per bucket
 void posed_variants(const KernelInfo** gjk, const KernelInfo** epa);
+// EPA of small and medium batches, one kernel per bucket (ogx_k_epa_few.cu)
+void few_variants(const KernelInfo** epa);
 
 // non-template kernels (ogx_k_misc.cu)
 cudaError_t launch_refine(const DevBatch& B, int grid, int grid_cont, cudaStream_t st, cudaStream_t st2,
