@@ -850,6 +850,7 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
     for (int b = kBuckets - 1; b >= 0 && e == cudaSuccess; --b) {
       const Launch& k = d_xf ? g_epap[b] : few_epa ? g_epaf[b] : g_epav[ctx->choice[1][b]];
       ctx->mark(kEpaName[b]);
+      B.wide_contacts = kWideContacts[b];
       k.fn<<<fit_grid(k.grid, npairs, few_epa ? 32 : k.L), kBlock, k.smem, bucket_stream(b)>>>(B, b);
       stage(kEpaName[b], bucket_stream(b));
       ++launches;

@@ -89,6 +89,7 @@ struct DevBatch {
                       // then holds the bodies in their own frame
   ogx_config cfg;
   int mode;
+  int wide_contacts = 0;  // k_epa_few: a warp per contact up to this many
 };
 
 // Append `want` lanes' items to a list guarded by counter *ctr; returns the slot of this
@@ -477,17 +478,19 @@ __global__ void __launch_bounds__(kStageStride, OCC) k_epa(DevBatch B, int bucke
 
 // EPA over one bucket's contacts in a batch of at most 24,576 pairs.  A contact is bound by its
 // chain of expansions, which a whole warp ends soonest, as long as the contacts do not queue for
-// warps; a bucket with more of them than about half a wave (4 blocks of 4 warps on 152 SMs; the
-// other buckets run beside it) is done sooner by narrow teams.  How many there are only the
-// device knows, so both are in one kernel.  (A warp per contact whatever their number, by the
-// batch's pairs alone: 16,000 contacts of 16-point bodies 418 us, now 286, 16,000 of 64-point
-// ones 1,213 and 1,025, 20,000 power-law pairs 370 and 333.  Limits of 1,000, 1,500, 2,000 and
-// 2,432 contacts: 20,000 power-law pairs 333, 333, 342, 344, 5,000 all the same.)
-constexpr int kWideContacts = 1000;
+// warps; a bucket with more of them than about a wave (4 blocks of 4 warps on 152 SMs are 2,432;
+// the buckets of small bodies run beside one another) is done sooner by narrow teams.  How many
+// there are only the device knows, so both are in one kernel.  (A warp per contact whatever their
+// number, by the batch's pairs alone: 16,000 contacts of 16-point bodies 418 us, now 286, 16,000
+// of 64-point ones 1,213 and 1,025, 20,000 power-law pairs 370 and 333.  Limits of 1,000, 1,500,
+// 2,000 and 2,432 contacts in every bucket: 20,000 power-law pairs 333, 333, 342, 344; but with
+// 1,000 for large bodies too 6,500 ellipsoid pairs took 279 us, now 244, 20,000 scene pairs 381
+// and 330.)
+constexpr int kWideContacts[kBuckets] = {1000, 1000, 1000, 1000, 2000, 3000, 2000};
 template <int LN>
 __global__ void __launch_bounds__(kStageStride, 4) k_epa_few(DevBatch B, int bucket) {
   const int cnt = B.counts[kCntEpa + bucket];
-  if (cnt <= kWideContacts)
+  if (cnt <= B.wide_contacts)
     epa_bucket<32, 0>(B, bucket, cnt);
   else
     epa_bucket<LN, 0>(B, bucket, cnt);

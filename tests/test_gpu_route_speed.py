@@ -55,3 +55,11 @@ def test_contacts_of_a_medium_batch(engine, n, points):
     choose(tuned)
     a, b = best_ms(engine, contacts(n, points), [rule, tuned])
     assert a < 1.2 * b, (a, b)
+
+
+@pytest.mark.parametrize("n,points", [(2500, 200), (2500, 400), (4000, 400)])
+def test_few_contacts_of_large_bodies(engine, n, points):
+    rule, narrow = engine.Context(0), engine.Context(0)
+    choose(narrow)
+    a, b = best_ms(engine, contacts(n, points, 1.0), [rule, narrow])
+    assert a < 1.1 * b, (a, b)
