@@ -104,10 +104,21 @@ constexpr int kBlock = 128;
 // largest batches of the one-warp-per-pair pipeline (distances only / with EPA) and of EPA
 // with a warp per contact while a bucket has few (ogx_run has the measurements)
 constexpr int kWarpPairsGjk = 4096, kWarpPairsEpa = 2048, kFewEpaPairs = 24576;
+// EPA of 257- to 512-point bodies takes 16 lanes a contact in place of 8 where more than 3/8 of
+// the batch are such contacts.  The teams of a warp run together, so the bodies that it scans in
+// turn are those of all its teams: where nearly every contact is between two large bodies, eight
+// lanes keep twice the bodies of sixteen in flight and miss L1 (60,000 contacts of 512-point
+// bodies 2,790 us, with sixteen lanes 1,401; of 300 points 1,327 and 1,063).  Among many others,
+// most of them against a small body, eight are better: 1M power-law pairs 5,167 us, with sixteen
+// lanes 5,258; 100,000 ellipsoid pairs of 64 to 512 points 1,415 and 1,485, of 128 to 512 1,710
+// and 1,720, of 256 to 512 2,380 and 2,037 (28, 37 and 50% of the pairs are such contacts).  The
+// count is known on the device: both kernels are launched and one of them finds nothing to do.
+constexpr int kShareBucket = 5;
 constexpr int kBucketCap[kBuckets] = {16, 32, 64, 128, 256, 512, 0};
 
 std::mutex g_init_mu;
 int g_init_device = -1;
+int g_epa_share = 0;  // EPA variant of kShareBucket where most of a batch are its contacts
 int g_grid_bin = 0, g_grid_polish = 0, g_grid_pack = 0, g_grid_refine = 0, g_grid_cont = 0, g_grid_spill = 0;
 uint32_t* g_subtab = nullptr;  // sub-distance decision table on the initialised device
 // per-device autotuned choices (variant index per bucket), -1 = not tuned
@@ -239,6 +250,8 @@ ogx_status init_kernels(int device) {
         if (s) return s;
       }
   }
+  for (int i = 0; i < (int)g_epav.size(); ++i)
+    if (g_epav[i].L == 16 && g_epav[i].K == (5 << kOccShift)) g_epa_share = i;
   g_grid_bin = 4 * sms;
   g_grid_pack = 8 * sms;
   int per_sm = 0;
@@ -269,6 +282,7 @@ ogx_status init_kernels(int device) {
 
 void set_defaults(ogx_ctx* ctx) {
   const bool tuned = ctx->device < 16 && g_tuned_valid[ctx->device];
+  ctx->tuned = tuned;
   for (int b = 0; b < kBuckets; ++b) {
     ctx->choice[0][b] = tuned ? g_tuned[ctx->device][0][b] : default_choice(g_gjkv, b, false);
     ctx->choice[1][b] = tuned ? g_tuned[ctx->device][1][b] : default_choice(g_epav, b, true);
@@ -848,12 +862,26 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   const bool refine = mode != kModeEpa && (ctx->cfg.flags & OGX_F_FP64_POLISH);
   if (mode != kModeGjk) {
     for (int b = kBuckets - 1; b >= 0 && e == cudaSuccess; --b) {
-      const Launch& k = d_xf ? g_epap[b] : few_epa ? g_epaf[b] : g_epav[ctx->choice[1][b]];
       ctx->mark(kEpaName[b]);
-      B.wide_contacts = kWideContacts[b];
-      k.fn<<<fit_grid(k.grid, npairs, few_epa ? 32 : k.L), kBlock, k.smem, bucket_stream(b)>>>(B, b);
+      DevBatch E = B;
+      auto run = [&](const Launch& k, int lanes) {
+        k.fn<<<fit_grid(k.grid, npairs, lanes), kBlock, k.smem, bucket_stream(b)>>>(E, b);
+        ++launches;
+      };
+      const bool by_share = b == kShareBucket && !few_epa && (d_xf || !(ctx->choice_set || ctx->tuned));
+      if (by_share) E.epa_max = (int)(3 * (int64_t)npairs / 8);
+      E.wide_contacts = kWideContacts[b];
+      const Launch& k = d_xf ? g_epap[b] : few_epa ? g_epaf[b] : g_epav[ctx->choice[1][b]];
+      run(k, few_epa ? 32 : k.L);
+      if (by_share) {
+        // (after the narrow one: ahead of it, its blocks would wait for room beside the other
+        // buckets' only to find nothing to do -- 200k scene pairs 1,038 us against 978)
+        const Launch& k16 = d_xf ? g_epap[b + 1] : g_epav[g_epa_share];
+        E.epa_min = E.epa_max + 1;
+        E.epa_max = 0x7fffffff;
+        run(k16, k16.L);
+      }
       stage(kEpaName[b], bucket_stream(b));
-      ++launches;
     }
     if (e != cudaSuccess) return ogx_cuda_fail(e, "EPA launches");
   }
@@ -1156,6 +1184,7 @@ extern "C" ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npair
     set_defaults(ctx);
     return s;
   }
+  ctx->tuned = true;
   for (int kind = 0; kind < 2; ++kind)
     for (int b = 0; b < kBuckets; ++b) ctx->choice[kind][b] = pick[kind][b];
   if (ctx->device < 16) {

@@ -33,6 +33,7 @@ struct ogx_ctx {
   size_t d_stage_bytes = 0;
   int last_launches = 0;
   int choice[2][ogx::kBuckets] = {};  // kernel variant per bucket: [0] GJK, [1] EPA
+  bool tuned = false;       // ... as the autotuner picked them (on this device)
   bool choice_set = false;  // the caller chose a variant: every call runs the bucket kernels
   // optional per-launch timing (CUDA events recorded between the launches of a call)
   bool timing = false;
@@ -40,6 +41,12 @@ struct ogx_ctx {
   cudaEvent_t ev[kMaxTimed + 1] = {};
   const char* ev_name[kMaxTimed] = {};
   int ev_count = 0;
+
+  void copy_choice(const ogx_ctx& from) {
+    for (int k = 0; k < 2; ++k)
+      for (int b = 0; b < ogx::kBuckets; ++b) choice[k][b] = from.choice[k][b];
+    tuned = from.tuned;
+  }
 
   void mark(const char* name);  // record an event before the next launch
   // concurrent bucket launches: one stream per size bucket, fork / join events

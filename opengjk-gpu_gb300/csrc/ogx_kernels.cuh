@@ -90,6 +90,7 @@ struct DevBatch {
   ogx_config cfg;
   int mode;
   int wide_contacts = 0;  // k_epa_few: a warp per contact up to this many
+  int epa_min = 0, epa_max = 0x7fffffff;  // k_epa: runs for this many contacts of the bucket only
 };
 
 // Append `want` lanes' items to a list guarded by counter *ctr; returns the slot of this
@@ -473,7 +474,8 @@ __device__ __forceinline__ void epa_bucket(const DevBatch& B, int bucket, int cn
 
 template <int L, int K, int OCC = 1, int D = 0, bool kPosed = false>
 __global__ void __launch_bounds__(kStageStride, OCC) k_epa(DevBatch B, int bucket) {
-  epa_bucket<L, K, D, kPosed>(B, bucket, B.counts[kCntEpa + bucket]);
+  const int cnt = B.counts[kCntEpa + bucket];
+  epa_bucket<L, K, D, kPosed>(B, bucket, cnt >= B.epa_min && cnt <= B.epa_max ? cnt : 0);
 }
 
 // EPA over one bucket's contacts in a batch of at most 24,576 pairs.  A contact is bound by its

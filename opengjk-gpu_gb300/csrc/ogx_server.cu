@@ -592,8 +592,7 @@ extern "C" ogx_status ogx_server_create(int device, const ogx_config* cfg, const
     if (st) break;
     st = s.ctx->ensure_aux();
     if (st) break;
-    for (int k = 0; k < 2; ++k)
-      for (int b = 0; b < kBuckets; ++b) s.ctx->choice[k][b] = S->pctx->choice[k][b];
+    s.ctx->copy_choice(*S->pctx);
     const size_t n = sc.slot_pairs;
     if ((e = dalloc(&s.d_pairs, n)) != cudaSuccess || (e = dalloc(&s.d_smp, n)) != cudaSuccess ||
         (e = dalloc(&s.d_dist, n)) != cudaSuccess || (e = dalloc(&s.d_nrm, 3 * n)) != cudaSuccess ||

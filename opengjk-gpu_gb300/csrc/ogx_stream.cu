@@ -109,8 +109,7 @@ ogx_status streamed(ogx_ctx* ctx, ogx_pool* pool, const float* xyz, int npairs, 
     c->cfg = ctx->cfg;
     c->timing = false;
     c->fork_ok = lane_fork;
-    for (int k = 0; k < 2; ++k)
-      for (int b = 0; b < kBuckets; ++b) c->choice[k][b] = ctx->choice[k][b];
+    c->copy_choice(*ctx);
     s = c->ensure_scratch(widest);
   }
   if (!s) s = ctx->ensure_stage(0, (size_t)pool->npoints * 3 * sizeof(float));

@@ -63,3 +63,14 @@ def test_few_contacts_of_large_bodies(engine, n, points):
     choose(narrow)
     a, b = best_ms(engine, contacts(n, points, 1.0), [rule, narrow])
     assert a < 1.1 * b, (a, b)
+
+
+@pytest.mark.parametrize("points", [300, 400, 512])
+def test_contacts_of_large_bodies(engine, points):
+    """257 to 512 points, more contacts than the rules for medium batches take."""
+    rule, narrow, wide = (engine.Context(0) for _ in range(3))
+    for ctx, lanes in ((narrow, 8), (wide, 16)):
+        choose(ctx)
+        ctx.set_kernel_choice("epa", 5, lanes, 5 << 8)
+    a, b, c = best_ms(engine, contacts(30000, points, 1.0), [rule, narrow, wide], reps=10)
+    assert a < 1.2 * min(b, c), (a, b, c)
