@@ -173,7 +173,10 @@ int ogx_ctx_work_counts(ogx_ctx* ctx, int32_t* counts, int cap);
 /* Kernel variant per size bucket (bucket b holds pairs whose larger body has at most
  * 16 * 2^b points, bucket 6 the rest): `lanes` lanes per pair, `blocks` float4 blocks of
  * x, y, z per lane and body kept in registers (0: points re-read from memory).
- * kind 0 = GJK, 1 = EPA. */
+ * kind 0 = GJK, 1 = EPA.  By default small batches take other kernels (up to 2,048 pairs, 4,096
+ * for GJK alone, one warp runs a pair's whole pipeline; up to 24,576 pairs, EPA takes a warp per
+ * contact while a bucket has few).  Setting a choice turns this off in the context, for good, in
+ * the calls that run its kind: they take the variants that are set at every batch size. */
 ogx_status ogx_ctx_get_kernel_choice(const ogx_ctx* ctx, int kind, int bucket, int* lanes,
                                      int* blocks);
 ogx_status ogx_ctx_set_kernel_choice(ogx_ctx* ctx, int kind, int bucket, int lanes, int blocks);

@@ -788,7 +788,8 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   // against 146, 2,000 160 against 250, 3,000 278 against 265; distances only, 3,000 pairs of
   // 32-point bodies 50 us against 93, 4,000 of 16-point ones 62 against 81, 10,000 117 against 81.
   const int warp_max = mode == kModeGjk ? kWarpPairsGjk : kWarpPairsEpa;
-  if (npairs <= warp_max && !d_xf && !ctx->choice_set && !ctx->timing && !ctx->stages) {
+  const bool chosen = (ctx->choice_set[0] && mode != kModeEpa) || (ctx->choice_set[1] && mode != kModeGjk);
+  if (npairs <= warp_max && !d_xf && !chosen && !ctx->timing && !ctx->stages) {
     e = launch_warp_pairs(B, st);
     if (e != cudaSuccess) return ogx_cuda_fail(e, "k_warp_pair launch");
     ctx->last_launches = 1;
@@ -798,7 +799,7 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   // to fill the GPU with narrow teams: 5,000 power-law pairs 199 us, 10,000 281, 20,000 333,
   // 24,000 412; with the tuned variants 5,000 259, 20,000 391, 24,000 490.  (A warp per contact
   // always: 50,000 pairs 586-599 us against 524-574.)
-  const bool few_epa = npairs <= kFewEpaPairs && !d_xf && !ctx->choice_set;
+  const bool few_epa = npairs <= kFewEpaPairs && !d_xf && !ctx->choice_set[1];
   const int bin_grid = std::min(g_grid_bin, (npairs + 255) / 256);
   ctx->mark("bin");
   e = launch_bin(B, bin_grid, st);
@@ -868,7 +869,7 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
         k.fn<<<fit_grid(k.grid, npairs, lanes), kBlock, k.smem, bucket_stream(b)>>>(E, b);
         ++launches;
       };
-      const bool by_share = b == kShareBucket && !few_epa && (d_xf || !(ctx->choice_set || ctx->tuned));
+      const bool by_share = b == kShareBucket && !few_epa && (d_xf || !(ctx->choice_set[1] || ctx->tuned));
       if (by_share) E.epa_max = (int)(3 * (int64_t)npairs / 8);
       E.wide_contacts = kWideContacts[b];
       const Launch& k = d_xf ? g_epap[b] : few_epa ? g_epaf[b] : g_epav[ctx->choice[1][b]];
@@ -992,7 +993,7 @@ extern "C" ogx_status ogx_ctx_set_kernel_choice(ogx_ctx* ctx, int kind, int buck
   for (int i = 0; i < (int)vs.size(); ++i)
     if (vs[i].L == lanes && vs[i].K == blocks && serves(vs[i], bucket)) {
       ctx->choice[kind][bucket] = i;
-      ctx->choice_set = true;
+      ctx->choice_set[kind] = true;
       return OGX_OK;
     }
   return ogx_fail(OGX_ERR_INVALID, "no variant (%d lanes, %d blocks) for bucket %d", lanes, blocks, bucket);
@@ -1105,8 +1106,9 @@ extern "C" ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npair
       best[kind][b] = INFINITY;
       pick[kind][b] = pick_prior[kind][b] = ctx->choice[kind][b];
     }
-  const bool was_timing = ctx->timing, was_set = ctx->choice_set;
-  ctx->choice_set = true;  // the bucket kernels are what is timed, at every batch size
+  const bool was_timing = ctx->timing, was_set[2] = {ctx->choice_set[0], ctx->choice_set[1]};
+  // the bucket kernels are what is timed, at every batch size
+  for (bool& set : ctx->choice_set) set = true;
   ogx_status s = ogx_ctx_set_timing(ctx, 1);
   for (int r = 0; r < rounds && !s; ++r) {
     for (int kind = 0; kind < 2; ++kind)
@@ -1176,7 +1178,7 @@ extern "C" ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npair
         for (int b = 0; b < kBuckets; ++b) pick[kind][b] = prior[kind][b];
   }
   ogx_ctx_set_timing(ctx, was_timing);
-  ctx->choice_set = was_set;
+  for (int kind = 0; kind < 2; ++kind) ctx->choice_set[kind] = was_set[kind];
   cudaFree(smp);
   cudaFree(dist);
   cudaFree(nrm);

@@ -34,7 +34,8 @@ struct ogx_ctx {
   int last_launches = 0;
   int choice[2][ogx::kBuckets] = {};  // kernel variant per bucket: [0] GJK, [1] EPA
   bool tuned = false;       // ... as the autotuner picked them (on this device)
-  bool choice_set = false;  // the caller chose a variant: every call runs the bucket kernels
+  bool choice_set[2] = {};  // the caller chose a variant for a bucket of this kind: calls that run
+                            // the kind take the chosen variants at every batch size
   // optional per-launch timing (CUDA events recorded between the launches of a call)
   bool timing = false;
   static constexpr int kMaxTimed = 32;
