@@ -46,6 +46,7 @@ struct ogx_ctx {
   void copy_choice(const ogx_ctx& from) {
     for (int k = 0; k < 2; ++k)
       for (int b = 0; b < ogx::kBuckets; ++b) choice[k][b] = from.choice[k][b];
+    for (int k = 0; k < 2; ++k) choice_set[k] = from.choice_set[k];
     tuned = from.tuned;
   }
 

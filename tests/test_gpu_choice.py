@@ -1,5 +1,6 @@
-"""A caller's choice of kernel variants holds in the calls that run its kind
-and leaves the others their own routes."""
+"""A caller's choice of kernel variants holds in the calls that run its kind, in streamed calls
+too, and leaves the others their own routes."""
+import numpy as np
 import pytest
 
 from ogx import workloads as W
@@ -32,3 +33,20 @@ def test_a_choice_concerns_its_own_kind(engine, kind):
     assert (_launches(engine, ctx, b, engine.MODE_GJK) == 1) == (kind == "epa")
     assert (_launches(engine, ctx, b, engine.MODE_EPA) == 1) == (kind == "gjk")
     assert _launches(engine, ctx, b, engine.MODE_GJK_EPA) > 1
+
+
+def test_streamed_calls_take_the_choice(engine):
+    b = W.powerlaw(seed=9, n_pairs=2000)
+    launches, out = [], []
+    for chosen in (False, True):
+        ctx = engine.Context(0)
+        if chosen:
+            _set(ctx, "gjk")
+            _set(ctx, "epa")
+        pool = engine.Pool(ctx, b.counts)
+        out.append(engine.streamed(ctx, pool, np.ascontiguousarray(b.coords), b.pairs, chunks=4))
+        launches.append(ctx.last_launches)
+    # (a chunk is one launch by default, and at least a kernel per bucket and kind otherwise)
+    assert launches[0] <= 8 and launches[1] >= 4 * 14, launches
+    for k in ("dist", "normal", "status", "simplex"):
+        assert out[0][k].tobytes() == out[1][k].tobytes(), k
