@@ -183,8 +183,11 @@ ogx_status ogx_ctx_set_kernel_choice(ogx_ctx* ctx, int kind, int bucket, int lan
 /* Autotuner: times every compiled variant that can serve each bucket on this batch
  * (device buffers; `reps` runs per candidate, kernels one after another, best time
  * kept) and takes the fastest per bucket; since a call runs the buckets concurrently, it
- * then times whole calls with that set and with the context's previous one and keeps
- * the faster, for this context and for contexts created later on the same device.
+ * then times whole calls with that set and as the context ran them before (its previous
+ * set, or the other kernels that a batch of this size takes) and keeps the faster, for
+ * this context and for contexts created later on the same device.  A set kept from a batch
+ * of at most 24,576 pairs serves batches of that size and larger; smaller ones, and those
+ * where the set comes from a larger batch, go on taking the kernels of their size.
  * Synchronous. */
 ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npairs,
                         const gkCollisionPair* d_pairs, int reps);

@@ -124,6 +124,7 @@ uint32_t* g_subtab = nullptr;  // sub-distance decision table on the initialised
 // per-device autotuned choices (variant index per bucket), -1 = not tuned
 int g_tuned[16][2][kBuckets];
 bool g_tuned_valid[16];
+int g_tuned_below[16];  // ogx_ctx::rules_below that goes with them
 
 // Persistent grid of a launch over at most `units` work items of `lanes` lanes each: the
 // full resident grid, or fewer blocks when the batch cannot fill it (small batches then
@@ -283,6 +284,7 @@ ogx_status init_kernels(int device) {
 void set_defaults(ogx_ctx* ctx) {
   const bool tuned = ctx->device < 16 && g_tuned_valid[ctx->device];
   ctx->tuned = tuned;
+  ctx->rules_below = tuned ? g_tuned_below[ctx->device] : 0x7fffffff;
   for (int b = 0; b < kBuckets; ++b) {
     ctx->choice[0][b] = tuned ? g_tuned[ctx->device][0][b] : default_choice(g_gjkv, b, false);
     ctx->choice[1][b] = tuned ? g_tuned[ctx->device][1][b] : default_choice(g_epav, b, true);
@@ -789,7 +791,7 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   // 32-point bodies 50 us against 93, 4,000 of 16-point ones 62 against 81, 10,000 117 against 81.
   const int warp_max = mode == kModeGjk ? kWarpPairsGjk : kWarpPairsEpa;
   const bool chosen = (ctx->choice_set[0] && mode != kModeEpa) || (ctx->choice_set[1] && mode != kModeGjk);
-  if (npairs <= warp_max && !d_xf && !chosen && !ctx->timing && !ctx->stages) {
+  if (npairs <= warp_max && npairs < ctx->rules_below && !d_xf && !chosen && !ctx->timing && !ctx->stages) {
     e = launch_warp_pairs(B, st);
     if (e != cudaSuccess) return ogx_cuda_fail(e, "k_warp_pair launch");
     ctx->last_launches = 1;
@@ -799,7 +801,8 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   // to fill the GPU with narrow teams: 5,000 power-law pairs 199 us, 10,000 281, 20,000 333,
   // 24,000 412; with the tuned variants 5,000 259, 20,000 391, 24,000 490.  (A warp per contact
   // always: 50,000 pairs 586-599 us against 524-574.)
-  const bool few_epa = npairs <= kFewEpaPairs && !d_xf && !ctx->choice_set[1];
+  const bool few_epa =
+      npairs <= kFewEpaPairs && npairs < ctx->rules_below && !d_xf && !ctx->choice_set[1];
   const int bin_grid = std::min(g_grid_bin, (npairs + 255) / 256);
   ctx->mark("bin");
   e = launch_bin(B, bin_grid, st);
@@ -1075,7 +1078,9 @@ extern "C" ogx_status ogx_graph_destroy(ogx_graph* G) {
 
 // Times every compiled variant that can serve each bucket on the caller's batch (round r
 // runs candidate r of every bucket at once, `reps` times, keeping the best time) and keeps
-// the fastest per bucket for this context and for contexts created later on the device.
+// the fastest per bucket for this context and for contexts created later on the device.  A set
+// that wins at a size with a route of its own (one warp per pair, k_epa_few) wins from that size
+// on: the routes stay below it.
 extern "C" ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npairs, const gkCollisionPair* d_pairs,
                                    int reps) {
   if (!ctx || !pool || !d_pairs || npairs <= 0) return ogx_fail(OGX_ERR_INVALID, "bad autotune arguments");
@@ -1142,7 +1147,8 @@ extern "C" ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npair
   }
   // The candidates were timed one after another, but a call runs the buckets
   // concurrently: keep the picked set only if a whole concurrent call with it is not
-  // slower than with the set the context started from (best of three each).
+  // slower than the call as the context ran it before -- its set, or the route that this
+  // size takes (best of three each).
   ogx_ctx_set_timing(ctx, 0);
   auto whole_call = [&](int (*ch)[kBuckets], float* best_ms) -> ogx_status {
     for (int kind = 0; kind < 2; ++kind)
@@ -1166,16 +1172,16 @@ extern "C" ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npair
     if (e1) cudaEventDestroy(e1);
     return r;
   };
+  bool keep_prior = false;
   if (!s) {
     int prior[2][kBuckets];
     for (int kind = 0; kind < 2; ++kind)
       for (int b = 0; b < kBuckets; ++b) prior[kind][b] = pick_prior[kind][b];
     float t_pick = INFINITY, t_prior = INFINITY;
     s = whole_call(pick, &t_pick);
+    for (int kind = 0; kind < 2; ++kind) ctx->choice_set[kind] = was_set[kind];
     if (!s) s = whole_call(prior, &t_prior);
-    if (!s && t_prior < t_pick)
-      for (int kind = 0; kind < 2; ++kind)
-        for (int b = 0; b < kBuckets; ++b) pick[kind][b] = prior[kind][b];
+    keep_prior = !s && t_prior < t_pick;
   }
   ogx_ctx_set_timing(ctx, was_timing);
   for (int kind = 0; kind < 2; ++kind) ctx->choice_set[kind] = was_set[kind];
@@ -1186,13 +1192,19 @@ extern "C" ogx_status ogx_autotune(ogx_ctx* ctx, const ogx_pool* pool, int npair
     set_defaults(ctx);
     return s;
   }
-  ctx->tuned = true;
-  for (int kind = 0; kind < 2; ++kind)
-    for (int b = 0; b < kBuckets; ++b) ctx->choice[kind][b] = pick[kind][b];
+  if (keep_prior) {  // (whole_call left it set)
+    if (!ctx->tuned && !was_set[0] && !was_set[1]) return OGX_OK;  // what every context starts with
+  } else {
+    ctx->tuned = true;
+    ctx->rules_below = npairs <= kFewEpaPairs ? npairs : 0x7fffffff;
+    for (int kind = 0; kind < 2; ++kind)
+      for (int b = 0; b < kBuckets; ++b) ctx->choice[kind][b] = pick[kind][b];
+  }
   if (ctx->device < 16) {
     std::lock_guard<std::mutex> lk(g_init_mu);
     for (int kind = 0; kind < 2; ++kind)
-      for (int b = 0; b < kBuckets; ++b) g_tuned[ctx->device][kind][b] = pick[kind][b];
+      for (int b = 0; b < kBuckets; ++b) g_tuned[ctx->device][kind][b] = ctx->choice[kind][b];
+    g_tuned_below[ctx->device] = ctx->rules_below;
     g_tuned_valid[ctx->device] = true;
   }
   return OGX_OK;

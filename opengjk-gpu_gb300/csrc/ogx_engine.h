@@ -34,6 +34,8 @@ struct ogx_ctx {
   int last_launches = 0;
   int choice[2][ogx::kBuckets] = {};  // kernel variant per bucket: [0] GJK, [1] EPA
   bool tuned = false;       // ... as the autotuner picked them (on this device)
+  int rules_below = 0x7fffffff;  // smallest batch that the picked set has been found faster on than
+                                 // the routes of small and medium batches: those stay below it
   bool choice_set[2] = {};  // the caller chose a variant for a bucket of this kind: calls that run
                             // the kind take the chosen variants at every batch size
   // optional per-launch timing (CUDA events recorded between the launches of a call)
@@ -48,6 +50,7 @@ struct ogx_ctx {
       for (int b = 0; b < ogx::kBuckets; ++b) choice[k][b] = from.choice[k][b];
     for (int k = 0; k < 2; ++k) choice_set[k] = from.choice_set[k];
     tuned = from.tuned;
+    rules_below = from.rules_below;
   }
 
   void mark(const char* name);  // record an event before the next launch

@@ -1,5 +1,9 @@
 """A caller's choice of kernel variants holds in the calls that run its kind, in streamed calls
 too, and leaves the others their own routes."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -50,3 +54,38 @@ def test_streamed_calls_take_the_choice(engine):
     assert launches[0] <= 8 and launches[1] >= 4 * 14, launches
     for k in ("dist", "normal", "status", "simplex"):
         assert out[0][k].tobytes() == out[1][k].tobytes(), k
+
+
+AUTOTUNE = """
+import sys
+sys.path[:0] = {path!r}
+import torch
+import test_gpu_route_speed as R
+from ogx import engine
+b = R.contacts(12000, 32)
+tuned, chosen = engine.Context(0), engine.Context(0)
+pool = engine.Pool(tuned, b.counts)
+pool.upload(b.coords)
+picked = tuned.autotune(pool, torch.from_numpy(b.pairs).cuda(), reps=3)
+for kind in ("gjk", "epa"):
+    for k, (lanes, blocks) in enumerate(picked[kind]):
+        chosen.set_kernel_choice(kind, k, lanes, blocks)
+later = engine.Context(0)
+times = R.best_ms(engine, b, [tuned, later, chosen])
+small = R.contacts(500, 32)
+pool = engine.Pool(later, small.counts)
+pool.upload(small.coords)
+engine.run(later, pool, torch.from_numpy(small.pairs).cuda())
+print(*times, later.last_launches)
+"""
+
+
+def test_calls_take_what_the_autotuner_kept(engine):
+    """At the size that it was given, in the context and in later ones; smaller calls keep their
+    route.  In a process of its own: the picks stay for the process."""
+    code = AUTOTUNE.format(path=[os.path.dirname(os.path.abspath(__file__))] + sys.path)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-1000:]
+    tuned, later, chosen, launches = (float(x) for x in r.stdout.split())
+    assert tuned < 1.08 * chosen and later < 1.08 * chosen, (tuned, later, chosen)
+    assert launches == 1
