@@ -147,14 +147,16 @@ ogx_status ogx_epa(ogx_ctx* ctx, const ogx_pool* pool, int npairs, const gkColli
 /* Kernels launched by the last engine call on this context (for accounting). */
 int ogx_ctx_last_launches(const ogx_ctx* ctx);
 /* Per-launch timing: when on, each batched call records CUDA events on the context's
- * stream between its launches.  ogx_ctx_kernel_times waits for the last call and
+ * stream between its launches, which then run one after another.  A small batch is one
+ * launch ("warp_pairs").  ogx_ctx_kernel_times waits for the last call and
  * fills up to cap (name, milliseconds) entries; returns the number filled. */
 ogx_status ogx_ctx_set_timing(ogx_ctx* ctx, int on);
 int ogx_ctx_kernel_times(ogx_ctx* ctx, const char** names, float* ms, int cap);
 /* Stage timeline of the concurrent (forked) launches, for finding the chain that sets a
  * call's duration: with it on, each call records an event after every bucket's GJK and
  * EPA kernel on that bucket's stream and after the refinement, the late pass, the spill
- * pass, the polish pass and the final join.  ogx_ctx_stage_timeline waits for the last
+ * pass, the polish pass and the final join (of a small batch, one launch: its end).
+ * ogx_ctx_stage_timeline waits for the last
  * call and fills up to cap (name, ms from the call's start) entries; returns the number
  * filled.  Not recorded while a graph is being captured or with per-kernel timing on. */
 ogx_status ogx_ctx_set_stage_timeline(ogx_ctx* ctx, int on);

@@ -451,6 +451,19 @@ void ogx_ctx::mark(const char* name) {
   ++ev_count;
 }
 
+bool ogx_ctx::start_stages(cudaStream_t st) {
+  if (!stage_ev[0]) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(st, &cs);
+  stage_count = 0;
+  return cs == cudaStreamCaptureStatusNone && cudaEventRecord(stage_ev[0], st) == cudaSuccess;
+}
+
+void ogx_ctx::stage(const char* name, cudaStream_t st) {
+  if (stage_count >= kMaxStages) return;
+  if (cudaEventRecord(stage_ev[1 + stage_count], st) == cudaSuccess) stage_name[stage_count++] = name;
+}
+
 extern "C" ogx_status ogx_ctx_set_timing(ogx_ctx* ctx, int on) {
   if (!ctx) return ogx_fail(OGX_ERR_INVALID, "ctx is NULL");
   cudaSetDevice(ctx->device);
@@ -791,9 +804,13 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   // 32-point bodies 50 us against 93, 4,000 of 16-point ones 62 against 81, 10,000 117 against 81.
   const int warp_max = mode == kModeGjk ? kWarpPairsGjk : kWarpPairsEpa;
   const bool chosen = (ctx->choice_set[0] && mode != kModeEpa) || (ctx->choice_set[1] && mode != kModeGjk);
-  if (npairs <= warp_max && npairs < ctx->rules_below && !d_xf && !chosen && !ctx->timing && !ctx->stages) {
+  if (npairs <= warp_max && npairs < ctx->rules_below && !d_xf && !chosen) {
+    const bool staged = ctx->stages && !ctx->timing && ctx->start_stages(st);
+    ctx->mark("warp_pairs");
     e = launch_warp_pairs(B, st);
     if (e != cudaSuccess) return ogx_cuda_fail(e, "k_warp_pair launch");
+    if (ctx->timing) cudaEventRecord(ctx->ev[ctx->ev_count], st);
+    if (staged) ctx->stage("end", st);
     ctx->last_launches = 1;
     return OGX_OK;
   }
@@ -814,17 +831,9 @@ ogx_status ogx_run(ogx_ctx* ctx, const float* d_pool, const BodyRef* d_bodies, i
   const bool fork = !ctx->timing && ctx->fork_ok && ctx->ensure_aux() == OGX_OK;
   const int W = ctx->fork_width;  // bucket b runs on aux[b mod W]
   // optional stage timeline of a forked call (not while a graph is being captured)
-  bool staged = false;
-  if (fork && ctx->stages && ctx->stage_ev[0]) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(st, &cs);
-    staged = cs == cudaStreamCaptureStatusNone && cudaEventRecord(ctx->stage_ev[0], st) == cudaSuccess;
-    ctx->stage_count = 0;
-  }
+  const bool staged = fork && ctx->stages && ctx->start_stages(st);
   auto stage = [&](const char* name, cudaStream_t s2) {
-    if (!staged || ctx->stage_count >= ogx_ctx::kMaxStages) return;
-    if (cudaEventRecord(ctx->stage_ev[1 + ctx->stage_count], s2) == cudaSuccess)
-      ctx->stage_name[ctx->stage_count++] = name;
+    if (staged) ctx->stage(name, s2);
   };
   auto bucket_stream = [&](int b) -> cudaStream_t { return fork ? ctx->aux[b % W] : st; };
   auto fork_out = [&]() -> cudaError_t {

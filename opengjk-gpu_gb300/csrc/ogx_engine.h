@@ -79,6 +79,8 @@ struct ogx_ctx {
   cudaEvent_t stage_ev[kMaxStages + 1] = {};  // [0] the call's start
   const char* stage_name[kMaxStages] = {};
   int stage_count = 0;
+  bool start_stages(cudaStream_t st);             // the call's start; false: not recorded
+  void stage(const char* name, cudaStream_t st);  // a stage's end
   std::vector<ogx_ctx*> sub;           // streamed calls: contexts running chunks side by side
 
   ogx_status ensure_scratch(int npairs);

@@ -89,3 +89,26 @@ def test_calls_take_what_the_autotuner_kept(engine):
     tuned, later, chosen, launches = (float(x) for x in r.stdout.split())
     assert tuned < 1.08 * chosen and later < 1.08 * chosen, (tuned, later, chosen)
     assert launches == 1
+
+
+@pytest.mark.parametrize("n", [500, 3000])
+def test_timing_leaves_the_route_alone(engine, n):
+    import torch
+    b = W.powerlaw(seed=10, n_pairs=n)
+    ctx = engine.Context(0)
+    pool = engine.Pool(ctx, b.counts)
+    pool.upload(b.coords)
+    pairs = torch.from_numpy(b.pairs).cuda()
+    want = engine.run(ctx, pool, pairs).to_host()
+    launches = ctx.last_launches
+    ctx.set_timing(True)
+    got = engine.run(ctx, pool, pairs).to_host()
+    times = ctx.kernel_times()
+    assert ctx.last_launches == launches
+    assert (len(times) == 1) == (launches == 1) and all(t > 0 for _, t in times), times
+    ctx.set_timing(False)
+    ctx.set_stage_timeline(True)
+    engine.run(ctx, pool, pairs)
+    stages = ctx.stage_timeline()
+    assert ctx.last_launches == launches and stages[-1][0] == "end" and stages[-1][1] > 0
+    assert got["dist"].tobytes() == want["dist"].tobytes()
