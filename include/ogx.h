@@ -165,8 +165,8 @@ int ogx_ctx_stage_timeline(ogx_ctx* ctx, const char** names, float* ms, int cap)
  * per EPA bucket [7, 14), EPA faces re-solved in FP64 [14], pairs whose GJK result was
  * refined in FP64 [15], of which continued in FP64 (uncertain FP32 support) [16],
  * contacts whose EPA outgrew the bucket kernels' working set and ran again at full
- * capacity [17], FP64 continuations of pairs with a body above 128 points (one warp
- * each; the others in [16] - [18] run one thread each) [18], contacts that only the
+ * capacity [17], FP64 continuations of pairs with a body above 128 points, which whole
+ * warps scan (those of [16] are scanned by 8 lanes each) [18], contacts that only the
  * FP64 refinement found (certified full-capacity EPA) [19], capacity spills whose
  * expansion the full-capacity pass continued instead of restarting [20] (at most 4096 per
  * call).  cap must be >= 21. */
@@ -325,7 +325,7 @@ ogx_status ogx_graph_destroy(ogx_graph* graph);
  * latency, plugins whose host forbids them to allocate.  The pool is given by
  * its device arrays in the engine layout (ogx_pool_device_layout, or written by the
  * caller); the caller passes the pairs and all outputs.  The pipeline's work lists live
- * in one static device array of 1,835,264 bytes that every GPU loading this library
+ * in one static device array of 1,638,656 bytes that every GPU loading this library
  * holds until exit.  At most 16384 pairs per call (OGX_ERR_CAPACITY beyond).  Each call
  * clears the array's counters itself; nothing has to be zeroed by the caller.  All calls
  * share the array, so calls that overlap on the GPU race: serialise them.  The first call on

@@ -290,9 +290,8 @@ OGX_HD fv3 world_point(const float* m, fv3 p) {
 }
 
 // Rigid pose of a body: m[0..9) the rotation R row-major, m[9..12) the translation t.
-// A posed point is R p + t in FP32, one fused multiply-add chain per coordinate: the
-// serving loop's world copies and the fused-pose sources below evaluate exactly this, so
-// both give the same world points bit for bit.
+// A posed point is R p + t in FP32, one fused multiply-add chain per coordinate, wherever the
+// pose is applied as the points are read; the serving loop's world copies are world_point's.
 OGX_HD fv3 pose_point(const float* m, fv3 p) {
   return v3<float>(fmaf(m[2], p.z, fmaf(m[1], p.y, fmaf(m[0], p.x, m[9]))),
                    fmaf(m[5], p.z, fmaf(m[4], p.y, fmaf(m[3], p.x, m[10]))),

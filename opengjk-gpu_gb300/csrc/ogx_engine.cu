@@ -543,7 +543,7 @@ bool ogx_pageable_reads(int dev) {
 }
 
 size_t ogx_scratch_bytes_per_pair() {
-  return 2 * kBuckets * sizeof(int) + sizeof(PolishRec) + sizeof(RefineRec) + 2 * sizeof(int);
+  return 2 * kBuckets * sizeof(int) + sizeof(PolishRec) + 3 * sizeof(int);
 }
 
 ogx_status ogx_ctx::ensure_scratch(int npairs) {
@@ -555,7 +555,7 @@ ogx_status ogx_ctx::ensure_scratch(int npairs) {
   if ((e = cudaMalloc(&d_lists, kBuckets * cap * sizeof(int))) != cudaSuccess ||
       (e = cudaMalloc(&d_elists, kBuckets * cap * sizeof(int))) != cudaSuccess ||
       (e = cudaMalloc(&d_polish, cap * sizeof(PolishRec))) != cudaSuccess ||
-      (e = cudaMalloc(&d_refine, cap * sizeof(RefineRec))) != cudaSuccess ||
+      (e = cudaMalloc(&d_refine, cap * sizeof(int))) != cudaSuccess ||
       (e = cudaMalloc(&d_refine_full, cap * sizeof(int))) != cudaSuccess ||
       (e = cudaMalloc(&d_spill, cap * sizeof(int))) != cudaSuccess ||
       (e = cudaMalloc(&d_resume, kResumeCap * sizeof(EpaResume))) != cudaSuccess ||

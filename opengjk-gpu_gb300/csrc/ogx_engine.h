@@ -20,7 +20,7 @@ struct ogx_ctx {
   int* d_elists = nullptr;
   int* d_counts = nullptr;
   ogx::PolishRec* d_polish = nullptr;
-  ogx::RefineRec* d_refine = nullptr;
+  int* d_refine = nullptr;
   int* d_refine_full = nullptr;
   int* d_spill = nullptr;
   ogx::EpaResume* d_resume = nullptr;  // kResumeCap saved expansions of capacity spills

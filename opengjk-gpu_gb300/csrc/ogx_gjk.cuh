@@ -209,7 +209,6 @@ OGX_LEAF void closest_on_simplex_t(int n, const vec3<T>* P, T* lam, vec3<T>& v) 
   lam[2] = s2;
   v = a + ab * s1 + ac * s2;
 }
-OGX_HD void closest_on_simplex(int n, const dv3* P, double* lam, dv3& v) { closest_on_simplex_t<double>(n, P, lam, v); }
 
 // --------------------------------------------------------------------------------
 // per-pair GJK
@@ -226,8 +225,7 @@ struct GjkState {
   int status;
   int exit;     // why the loop ended (GJK_EXIT_*)
   bool polish;  // separated: certify and re-solve (or continue) in FP64
-  int wa, wb;   // support pair along the final direction
-  bool certain; // that support is the exact (FP64) support along the exact direction
+  bool certain; // the final support is the exact (FP64) one along the exact direction
 };
 
 // loop exit reasons (reported in status bits 16..18)
@@ -497,7 +495,6 @@ OGX_HD void gjk_end(const Team& t, const Bodies& B, const Config& cfg, const Gjk
   const int* IB = r.IB;
   const int n = r.n;
   const float wmax2 = r.wmax2;
-  const int ia = r.ia, ib = r.ib;
   const int k = r.k;
   g.status = r.status;
   g.exit = r.exit;
@@ -531,8 +528,6 @@ OGX_HD void gjk_end(const Team& t, const Bodies& B, const Config& cfg, const Gjk
   // that is not small against the distance.
   g.polish = false;
   g.certain = false;
-  g.wa = ia;
-  g.wb = ib;
   if ((cfg.flags & OGX_F_FP64_POLISH) && g.n >= 1 && g.n <= 3 && !gjk_contact(g)) {
     // Every separated pair is certified or continued in FP64: a stop on the FP32 gap
     // bounds the distance (about 1e-7 relative) but not its direction, which on flat
@@ -1097,26 +1092,6 @@ OGX_HD void gjk_refine(const Team& t, const Bodies& B, GjkState& g, int max_iter
     refine_step(B, r, xa, xb, subtab);
   }
   refine_end(B, r, g);
-}
-
-// FP64 re-solve of the final simplex: exact Minkowski points, exact closest point.
-template <class Bodies>
-OGX_HD void gjk_polish(const Bodies& B, GjkState& g) {
-  dv3 P[3];
-  for (int j = 0; j < g.n && j < 3; ++j) P[j] = B.dpoint(0, g.ia[j]) - B.dpoint(1, g.ib[j]);
-  double lam[4];
-  dv3 v;
-  closest_on_simplex(g.n, P, lam, v);
-  dv3 w0 = v3<double>(0.0, 0.0, 0.0), w1 = w0;
-  for (int j = 0; j < g.n; ++j) {
-    w0 = w0 + B.dpoint(0, g.ia[j]) * lam[j];
-    w1 = w1 + B.dpoint(1, g.ib[j]) * lam[j];
-  }
-  g.v = cvt<float>(v);
-  g.dist = (float)sqrt(dot(v, v));
-  g.w0 = cvt<float>(w0);
-  g.w1 = cvt<float>(w1);
-  g.status |= OGX_S_POLISHED;
 }
 
 }  // namespace ogx

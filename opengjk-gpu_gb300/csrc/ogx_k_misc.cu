@@ -120,7 +120,7 @@ template <bool kPosed>
 __global__ void __launch_bounds__(128) k_refine(DevBatch B) {
   const int cnt = B.counts[kCntRefine];
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
-    const int p = B.refine[k].pair;
+    const int p = B.refine[k];
     const int2 pr = B.pairs[p];
     const BodyRef ra = B.bodies[pr.x], rb = B.bodies[pr.y];
     typename PoseOf<kPosed, MemBodies>::type mb;

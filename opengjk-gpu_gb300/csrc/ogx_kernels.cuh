@@ -5,13 +5,19 @@
 //             (bucket = larger point count: <=16, 32, 64, 128, 256, 512, more)
 //   k_gjk     persistent GJK over one bucket: a team of L lanes per pair, both bodies
 //             in registers (K float4 blocks of x, y, z per lane and body); contacts are
-//             appended to the bucket's EPA list, pairs whose FP32 distance is not
-//             certain to polish_rel to the FP64 polish list
-//   k_epa     persistent EPA over one bucket's contacts, polytope in shared memory
-//   k_polish  FP64 re-solve of the listed pairs, one thread per pair (full warps of
-//             FP64 work instead of one lane per team)
-// All work lists are filled with warp-aggregated atomics; kernels stride over them, so
-// the grid size is independent of the batch (persistent launch, graph-capturable).
+//             appended to the bucket's EPA list, separated pairs to the refinement's: those
+//             whose support is proved exact, and those to be continued in FP64
+//   k_refine, k_refine_cont
+//             exact closest points of the former, FP64 continuations of the latter
+//   k_epa     persistent EPA over one bucket's contacts, polytope in shared memory (k_epa_few:
+//             the same for small and medium batches)
+//   k_epa_spill
+//             EPA at full capacity, and the certified runs, one warp per contact
+//   k_polish  FP64 re-solve of the bucket kernels' final faces, one thread per contact
+//   k_warp_pair
+//             all of it with one warp per pair, for small batches
+// All work lists are filled with warp-aggregated atomics (a contact's face is kept at its
+// pair's index); kernels stride over them, so the grid size is independent of the batch (persistent launch, graph-capturable).
 #pragma once
 
 #include "ogx_bodies.cuh"
@@ -28,14 +34,6 @@ OGX_HD int bucket_of(int m) {
 }
 
 OGX_HD int bucket_max(int b) { return b == kBuckets - 1 ? 0x7fffffff : 16 << b; }
-
-// FP64 refinement request of a separated pair whose support pair (wa, wb) along the final
-// direction the FP32 pass proved exact
-struct RefineRec {
-  int pair;
-  int wa, wb;
-  int certain;
-};
 
 // re-solve request of a contact, at its pair's index: none (kind 0), or the final EPA face
 // (kind 1)
@@ -77,9 +75,9 @@ struct DevBatch {
   int* elists;      // kBuckets regions of npairs entries
   int* counts;      // kCntSlots
   PolishRec* polish;
-  RefineRec* refine;  // npairs entries
-  int* refine_full;   // npairs entries: pair ids whose FP32 support was not certain
-                      // (small bodies from the front, large ones from the back)
+  int* refine;        // npairs entries: separated pairs whose FP32 support was proved exact
+  int* refine_full;   // npairs entries: the others (small bodies from the front, large ones
+                      // from the back)
   int* spill;         // npairs entries: contacts to re-run at full EPA capacity
   EpaResume* resume;  // resume_cap saved small-capacity expansions (null: none)
   int resume_cap;
@@ -269,14 +267,7 @@ __device__ __forceinline__ void gjk_store(const DevBatch& B, int bucket, int p, 
   }
   if (mc) {
     bc = __shfl_sync(act, bc, __ffs(mc) - 1);
-    if (certain) {
-      RefineRec r;
-      r.pair = p;
-      r.wa = g.wa;
-      r.wb = g.wb;
-      r.certain = 1;
-      B.refine[bc + __popc(mc & below)] = r;
-    }
+    if (certain) B.refine[bc + __popc(mc & below)] = p;
   }
   if (mu) {
     bu = __shfl_sync(act, bu, __ffs(mu) - 1);

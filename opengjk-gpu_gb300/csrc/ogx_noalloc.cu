@@ -11,7 +11,7 @@
 // Limits and behaviour (also in include/ogx.h):
 //  * at most kNoAllocMaxPairs pairs per call; larger batches are rejected with
 //    OGX_ERR_CAPACITY;
-//  * the array (kNoAllocScratchBytes, 1,835,264 bytes) exists on every GPU that loads the
+//  * the array (kNoAllocScratchBytes, 1,638,656 bytes) exists on every GPU that loads the
 //    library, from load until the process exits;
 //  * every call uses the same array and the array keeps the last call's contents; the
 //    work-list counters must start at zero and each call clears them itself (a memset on
@@ -40,12 +40,12 @@ constexpr size_t kOffCounts = 0;
 constexpr size_t kOffLists = 256;
 constexpr size_t kOffElists = kOffLists + (size_t)kBuckets * kNoAllocMaxPairs * sizeof(int);
 constexpr size_t kOffRefine = kOffElists + (size_t)kBuckets * kNoAllocMaxPairs * sizeof(int);
-constexpr size_t kOffRefineFull = kOffRefine + (size_t)kNoAllocMaxPairs * sizeof(RefineRec);
+constexpr size_t kOffRefineFull = kOffRefine + (size_t)kNoAllocMaxPairs * sizeof(int);
 constexpr size_t kOffPolish = kOffRefineFull + (size_t)kNoAllocMaxPairs * sizeof(int);
 constexpr size_t kOffSpill = kOffPolish + (size_t)kNoAllocMaxPairs * sizeof(PolishRec);
 constexpr size_t kNoAllocScratchBytes = kOffSpill + (size_t)kNoAllocMaxPairs * sizeof(int);
 
-static_assert(kNoAllocScratchBytes == 1835264, "the size is documented in include/ogx.h");
+static_assert(kNoAllocScratchBytes == 1638656, "the size is documented in include/ogx.h");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -174,7 +174,7 @@ extern "C" ogx_status ogx_gjk_epa_noalloc(const float* d_points, const void* d_b
   B.counts = reinterpret_cast<int*>(S->scratch + kOffCounts);
   B.lists = reinterpret_cast<int*>(S->scratch + kOffLists);
   B.elists = reinterpret_cast<int*>(S->scratch + kOffElists);
-  B.refine = reinterpret_cast<RefineRec*>(S->scratch + kOffRefine);
+  B.refine = reinterpret_cast<int*>(S->scratch + kOffRefine);
   B.refine_full = reinterpret_cast<int*>(S->scratch + kOffRefineFull);
   B.polish = reinterpret_cast<PolishRec*>(S->scratch + kOffPolish);
   B.spill = reinterpret_cast<int*>(S->scratch + kOffSpill);
