@@ -730,6 +730,15 @@ ogx_status pool_from_host_f64(Compat& c, const ogx_polytope_f64* a, const ogx_po
   return e == cudaSuccess ? OGX_OK : ogx_cuda_fail(e, "double coordinate upload");
 }
 
+// Waits for the stream where a call ends early: the device may still be reading the caller's
+// arrays, or the narrowed ones, which are gone once the call has returned.
+struct Drain {
+  cudaStream_t st;
+  ~Drain() {
+    if (st) cudaStreamSynchronize(st);
+  }
+};
+
 // host-buffer query over pairs (2i, 2i+1) or explicit pairs; results to host arrays
 ogx_status host_query(const gkPolytope* a, const gkPolytope* b, int nbodies, int npairs,
                       const gkCollisionPair* host_pairs, gkSimplex* smp, float* dist, float* nrm,
@@ -743,6 +752,7 @@ ogx_status host_query(const gkPolytope* a, const gkPolytope* b, int nbodies, int
   Compat* c = L.c;
   cudaStream_t st = c->ctx->stream;
   Narrowed N;
+  Drain early{st};
   s = a64 ? pool_from_host_f64(*c, a64, b64, nbodies, N) : pool_from_host_desc(*c, a, b, nbodies);
   if (!s) s = ensure_results(*c, npairs);
   if (s) return s;
@@ -798,6 +808,7 @@ ogx_status host_query(const gkPolytope* a, const gkPolytope* b, int nbodies, int
   if (e != cudaSuccess) return ogx_cuda_fail(e, "result copy");
   s = finish(*c);
   if (s) return s;
+  early.st = nullptr;
   if (!direct) {
     parallel_copy(smp, hs, sb);
     parallel_copy(dist, hs + sb, db);
