@@ -79,13 +79,13 @@ OGX_HD SubOut tri_tree(Bits& B, int t0, int t1, int q) {
   if (k12) {
     if (!B.D(t1, t0)) {
       if (k13 && B.D(t0, t1)) return so_line(t0, q, t0);
-      return so_plane(t0, t1, q, t0, t1);
+      return so_plane(t0, t1, q, t1, t0);
     }
     return so_line(q, t1, t1);
   }
   if (k13) {
     if (B.D(t0, t1)) return so_line(t0, q, t0);
-    return so_plane(t0, t1, q, t0, t1);
+    return so_plane(t0, t1, q, t1, t0);
   }
   return so_vertex(q);
 }

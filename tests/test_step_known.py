@@ -127,3 +127,25 @@ def test_bodies_far_apart_for_their_size(orc, twin, apart, kind, thickness, mode
             r["normal"] = None
         bad = far_bodies.errors(b, r, o)
         assert len(bad) == 0, (size2, bad[:5], r["dist"][bad[:5]], o["dist"][bad[:5]])
+
+
+def test_projection_on_a_triangle_keeps_its_signs(twin):
+    """The normal of the plane is that of (newest, second, first): where it has a zero component, the
+    zero's sign is part of the result."""
+    fn = twin._lib_twin.twin_triangle_step
+    fn.argtypes = [ctypes.c_int] + [ctypes.c_void_p] * 3
+    g = np.random.default_rng(9)
+    p = g.integers(-4, 5, (4000, 3, 3)).astype(np.float64)
+    p[:, :, 2] = g.integers(1, 3, (4000, 1))  # in a plane z = const: the origin projects on (0, 0, z)
+    left, v = np.zeros(len(p), np.int32), np.zeros((len(p), 3))
+    fn(len(p), p.ctypes.data, left.ctypes.data, v.ctypes.data)
+    on = left == 3
+    assert on.sum() > 100
+    q1, q2, q3 = p[on, 2], p[on, 1], p[on, 0]
+    a, b = q1 - q2, q1 - q3
+    n = np.stack([a[:, 1] * b[:, 2] - a[:, 2] * b[:, 1], a[:, 2] * b[:, 0] - a[:, 0] * b[:, 2],
+                  a[:, 0] * b[:, 1] - a[:, 1] * b[:, 0]], 1)
+    d = (n[:, 0] * q1[:, 0] + n[:, 1] * q1[:, 1]) + n[:, 2] * q1[:, 2]
+    with np.errstate(invalid="ignore"):
+        want = n * (d / ((n[:, 0] * n[:, 0] + n[:, 1] * n[:, 1]) + n[:, 2] * n[:, 2]))[:, None]
+    assert v[on].tobytes() == want.tobytes()

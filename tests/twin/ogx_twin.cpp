@@ -200,6 +200,27 @@ int twin_step_bits(int count, int n, const float* p, uint32_t* bits, uint32_t* k
   return 0;
 }
 
+// The sub-distance step on exact 3-point simplices (newest last): the points that stay, and the
+// closest point to the origin
+int twin_triangle_step(int count, const double* p, int32_t* left, double* dir) {
+  for (int i = 0; i < count; ++i) {
+    Sx<double> s;
+    s.n = 3;
+    for (int j = 0; j < 3; ++j) {
+      const double* q = p + 9 * (size_t)i + 3 * j;
+      s.v[j].p = v3<double>(q[0], q[1], q[2]);
+      s.v[j].k = j;
+    }
+    dv3 v = v3<double>(0.0, 0.0, 0.0);
+    subdistance(s, v, nullptr, 0u, 0u);
+    left[i] = s.n;
+    dir[3 * i] = v.x;
+    dir[3 * i + 1] = v.y;
+    dir[3 * i + 2] = v.z;
+  }
+  return 0;
+}
+
 // exact support index and value of one body (SoA pool at quad 0, n points) along count directions
 int twin_exact_support(const float* pool, int n, int count, const double* d, int32_t* index, double* value) {
   MemBodies B;
