@@ -1110,18 +1110,23 @@ OGX_HD bool epa_step(const Team& t, const Bodies& B, const Config& cfg, Mem& M, 
   return live;
 }
 
+// Keeps an expansion that outgrew the small capacity: the polytope as it was at the top of the
+// last step.  With FP64 planes the full pass is a certified run, whose FP64 planes and points a
+// record does not hold: that one starts again.
+template <class Team, class Mem>
+OGX_HD void epa_save_run(const Team& t, const Config& cfg, const Mem& M, const EpaResumeSink& sink, EpaOut& o,
+                         const EpaRun<Mem>& r) {
+  if (!(cfg.flags & OGX_F_EPA_FP64_PLANES))
+    epa_save(t, M, sink, o, r.flags & kRunLate ? r.nv - 1 : r.nv, r.fend, r.it - 1, r.st, r.scale2);
+}
+
 // The result once the loop has ended; a capacity spill (o.spill, at the top of its last
 // expansion) saves itself.
 template <bool kCert = false, class Team, class Bodies, class Mem>
 OGX_HD void epa_finish(const Team& t, const Bodies& B, const Config& cfg, Mem& M, EpaOut& o, const EpaRun<Mem>& r,
                        bool can_spill, const EpaResumeSink& sink) {
   if (o.spill) {
-    // The polytope as it was at the top of the last expansion.  With FP64 planes the full pass
-    // is a certified run, whose FP64 planes and points a record does not hold: that one starts
-    // again.
-    if constexpr (!Mem::kFull)
-      if (!(cfg.flags & OGX_F_EPA_FP64_PLANES))
-        epa_save(t, M, sink, o, r.flags & kRunLate ? r.nv - 1 : r.nv, r.fend, r.it - 1, r.st, r.scale2);
+    if constexpr (!Mem::kFull) epa_save_run(t, cfg, M, sink, o, r);
     return;
   }
   const bool escalate = (cfg.flags & OGX_F_FP64_ESCALATE) != 0;
@@ -1154,11 +1159,10 @@ OGX_HD void epa_finish(const Team& t, const Bodies& B, const Config& cfg, Mem& M
   o.spill = o.spill64 = again;
 }
 
+// r: the loop's state when it ended
 template <bool kCert = false, class Team, class Bodies, class Mem>
 OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const GjkState& g, Mem& M, EpaOut& o,
-                     bool can_spill, EpaResumeSink sink = EpaResumeSink{nullptr, nullptr, 0},
-                     const EpaResume* rs = nullptr) {
-  EpaRun<Mem> r;
+                     bool can_spill, EpaResumeSink sink, const EpaResume* rs, EpaRun<Mem>& r) {
   if (epa_start<kCert>(t, B, cfg, g, M, o, r, rs)) {
 #pragma unroll 1
     while (r.it < cfg.epa_max_iter && epa_step<kCert>(t, B, cfg, M, o, r, can_spill)) {
@@ -1171,6 +1175,14 @@ OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const Gj
     o.w1 = g.w1;
     o.nrm = unit_or_x(g.w1 - g.w0);
   }
+}
+
+template <bool kCert = false, class Team, class Bodies, class Mem>
+OGX_HD void epa_pair(const Team& t, const Bodies& B, const Config& cfg, const GjkState& g, Mem& M, EpaOut& o,
+                     bool can_spill, EpaResumeSink sink = EpaResumeSink{nullptr, nullptr, 0},
+                     const EpaResume* rs = nullptr) {
+  EpaRun<Mem> r;
+  epa_pair<kCert>(t, B, cfg, g, M, o, can_spill, sink, rs, r);
 }
 
 }  // namespace ogx

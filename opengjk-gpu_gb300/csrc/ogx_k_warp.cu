@@ -83,14 +83,23 @@ __device__ __noinline__ void warp_refine(const WarpTeam<32> t, const MemBodies B
   *g = s;
 }
 
-// full capacity from the start: certified, or (a contact that only outgrew the small
-// capacity) with FP32 planes
+// full capacity: certified, from the start, or (a contact that only outgrew the small
+// capacity) with FP32 planes, on from the polytope that the small pass left in smem, which is
+// kept in a record of the batch's meanwhile
 __device__ __noinline__ void warp_epa_full(const WarpTeam<32> t, const MemBodies B, const Config* cfg, bool certified,
-                                           const GjkState* g, EpaMemCert& M, EpaOut* out) {
+                                           const GjkState* g, unsigned char* smem, const EpaResumeSink sink,
+                                           const EpaRun<EpaMemSmall>* run, int status, EpaOut* out) {
   Config c = *cfg;
-  if (certified) c.flags |= OGX_F_EPA_FP64_PLANES;
   EpaOut o;
-  epa_pair<true>(t, B, c, *g, M, o, false);
+  o.status = status;
+  o.resume = -1;
+  if (certified)
+    c.flags |= OGX_F_EPA_FP64_PLANES;
+  else
+    epa_save_run(t, c, *reinterpret_cast<EpaMemSmall*>(smem), sink, o, *run);
+  t.sync();
+  const EpaResume* rs = o.resume >= 0 ? sink.buf + o.resume : nullptr;
+  epa_pair<true>(t, B, c, *g, *reinterpret_cast<EpaMemCert*>(smem), o, false, EpaResumeSink{nullptr, nullptr, 0}, rs);
   *out = o;
 }
 
@@ -166,9 +175,11 @@ __global__ void __launch_bounds__(32, kMode == kModeGjk ? 20 : 16) k_warp_pair(D
   }
   if constexpr (kMode != kModeGjk) {
     EpaOut o;
+    EpaRun<EpaMemSmall> run;
     if (!late) {
       count(B, kCntEpa + bucket, lead);
-      epa_pair(t, src, B.cfg, g, *reinterpret_cast<EpaMemSmall*>(smem_raw), o, true);
+      epa_pair(t, src, B.cfg, g, *reinterpret_cast<EpaMemSmall*>(smem_raw), o, true,
+               EpaResumeSink{nullptr, nullptr, 0}, nullptr, run);
       if (!o.spill && o.polish) count(B, kCntPolish, lead);
     } else {
       o.spill = o.spill64 = true;
@@ -178,7 +189,9 @@ __global__ void __launch_bounds__(32, kMode == kModeGjk ? 20 : 16) k_warp_pair(D
       t.sync();
       const GjkState g2 = g;
       EpaOut o2;
-      warp_epa_full(t, src.mem, &B.cfg, o.spill64, &g2, *reinterpret_cast<EpaMemCert*>(smem_raw), &o2);
+      const EpaRun<EpaMemSmall> run2 = run;
+      const EpaResumeSink sink{B.resume, B.counts + kCntResume, B.resume_cap};
+      warp_epa_full(t, src.mem, &B.cfg, o.spill64, &g2, smem_raw, sink, &run2, o.status, &o2);
       o = o2;
     }
     if (o.polish) epa_polish(src, o);

@@ -50,3 +50,20 @@ def test_routes_agree_on_large_expansions(engine, flags):
         out.append(r.to_host())
     for k in ("dist", "normal", "status", "simplex"):
         assert out[0][k].tobytes() == out[1][k].tobytes(), k
+
+
+@pytest.mark.gpu
+def test_both_routes_continue_large_expansions(engine):
+    import torch
+    b = _batch()
+    for bucket_kernels in (False, True):
+        ctx = engine.Context(0)
+        if bucket_kernels:
+            for k, (lanes, blocks) in enumerate(ctx.kernel_choice()["epa"]):
+                ctx.set_kernel_choice("epa", k, lanes, blocks)
+        pool = engine.Pool(ctx, b.counts)
+        pool.upload(b.coords)
+        engine.run(ctx, pool, torch.from_numpy(b.pairs).cuda(), engine.MODE_GJK_EPA)
+        ctx.synchronize()
+        assert (ctx.last_launches > 1) == bucket_kernels
+        assert ctx.work_counts()["epa_resumed"] > 20
