@@ -28,7 +28,11 @@
 // long arithmetic used from many places (double-float division, FP64 predicates), kept out
 // of line: inlined, the kernels grew to 110-230 KB of code each and a warp spent more time
 // on instruction fetches than on anything else where few warps share a code path
+#if defined(OGX_INLINE_LEAVES)
+#define OGX_LEAF OGX_HD
+#else
 #define OGX_LEAF inline __host__ __device__ __noinline__
+#endif
 #else
 #define OGX_HD inline
 #define OGX_COLD inline

@@ -1,4 +1,4 @@
-// ogx_k_misc.cu -- pool packing, pair binning and the FP64 polish pass.
+// ogx_k_misc.cu -- pool packing, the FP64 refinement and polish passes, EPA at full capacity.
 #include "ogx_kernels.cuh"
 #include "ogx_continue.cuh"
 
@@ -30,59 +30,6 @@ __global__ void k_pack(const float* __restrict__ aos, const int64_t* __restrict_
     }
     finite = __all_sync(0xffffffffu, finite);
     if (lane == 0) bodies[b].n = finite ? n : -n;
-  }
-}
-
-// ---------------------------------------------------------------------------------
-__device__ __forceinline__ bool pair_ok(const DevBatch& B, int2 pr) {
-  return pr.x >= 0 && pr.x < B.nbodies && pr.y >= 0 && pr.y < B.nbodies;
-}
-
-__global__ void k_bin(DevBatch B) {
-  const int stride = gridDim.x * blockDim.x;
-  const int n32 = (B.npairs + 31) & ~31;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n32; p += stride) {
-    const bool in = p < B.npairs;
-    int b = -1;
-    bool bad = false;
-    bool work = false;
-    if (in) {
-      const int2 pr = B.pairs[p];
-      bad = !pair_ok(B, pr);
-      if (!bad) {
-        const int na = B.bodies[pr.x].n, nb = B.bodies[pr.y].n;
-        bad = na < 1 || nb < 1;
-        b = bucket_of(na > nb ? na : nb);
-      }
-      if (bad) {
-        mark_bad(B, p);
-      } else if (B.mode == kModeEpa) {
-        // EPA only: contacts go to the EPA lists, separated pairs only get a normal
-        const gkSimplex& s = B.smp[p];
-        work = s.nvrtx == 4 || !(B.dist[p] > FLT_EPSILON);
-        if (!work) {
-          MemBodies mb;
-          mb.bind(B.pool, B.bodies[pr.x], B.bodies[pr.y]);
-          store3(B.nrm + 3 * (size_t)p, simplex_sep_normal(mb, s));
-          if (B.status) B.status[p] = 0;
-        }
-      } else {
-        work = true;
-      }
-    }
-    // warp-aggregated append per bucket
-    const int key = work ? b : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, key);
-    const int wl = threadIdx.x & 31;
-    const int leader = __ffs(peers) - 1;
-    if (key >= 0) {
-      int* ctr = B.counts + (B.mode == kModeEpa ? kCntEpa : kCntGjk) + key;
-      int* list = (B.mode == kModeEpa ? B.elists : B.lists) + (size_t)key * B.npairs;
-      int base = 0;
-      if (wl == leader) base = atomicAdd(ctr, __popc(peers));
-      base = __shfl_sync(peers, base, leader);
-      list[base + __popc(peers & ((1u << wl) - 1u))] = p;
-    }
   }
 }
 
@@ -295,11 +242,6 @@ cudaError_t launch_pack_ptrs64(const double* const* src, int nbodies, const int6
 cudaError_t launch_pack(const float* aos, const int64_t* voff, BodyRef* bodies, int nbodies,
                         float* pool, int grid, cudaStream_t st) {
   k_pack<<<grid, 256, 0, st>>>(aos, voff, bodies, nbodies, pool);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_bin(const DevBatch& B, int grid, cudaStream_t st) {
-  k_bin<<<grid, 256, 0, st>>>(B);
   return cudaGetLastError();
 }
 
