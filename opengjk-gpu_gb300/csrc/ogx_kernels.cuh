@@ -527,7 +527,7 @@ void posed_variants(const KernelInfo** gjk, const KernelInfo** epa);
 // EPA of small and medium batches, one kernel per bucket (ogx_k_epa_few.cu)
 void few_variants(const KernelInfo** epa);
 
-// non-template kernels (ogx_k_misc.cu, ogx_k_bin.cu)
+// non-template kernels (ogx_k_misc.cu, ogx_k_bin.cu, ogx_k_spill.cu)
 cudaError_t launch_refine(const DevBatch& B, int grid, int grid_cont, cudaStream_t st, cudaStream_t st2,
                           cudaEvent_t ready);
 cudaError_t continue_occupancy(int block, int* per_sm);
